@@ -21,7 +21,7 @@ LIB_PATH = os.path.join(LIB_DIR, "libnatten_b200.so")
 # (tests/test_gpu_robustness.py) to make a wait expire; the package never loads it.
 HOOK_LIB_PATH = os.path.join(LIB_DIR, "libnatten_b200_testhooks.so")
 SOURCES = ["capi.cu", "tokperm.cu", "merge.cu", "na_simt.cu", "na_bwd_simt.cu", "fna_sm100.cu", "fna_bwd_sm100.cu", "na_fused.cu"]
-HEADERS = ["common.cuh", "ptx.cuh", "fna_host.cuh", "fna_device.cuh", "fna_instrument.cuh", os.path.join("..", "..", "include", "natten_b200.h")]
+HEADERS = ["common.cuh", "ptx.cuh", "fna_host.cuh", "fna_device.cuh", "fna_instrument.cuh", "simt_tile.cuh", os.path.join("..", "..", "include", "natten_b200.h")]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-std=c++17", "-lineinfo",
               "-Xcompiler", "-fPIC", "-Xcompiler", "-fvisibility=hidden"]
 

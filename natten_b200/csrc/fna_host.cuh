@@ -23,7 +23,7 @@ int fna_device_info(int* sms, int** status_ptr);
 // under stream capture gets a pair of its own from a pool of 3072 that is handed out in turn.
 int fna_work_counters(unsigned long long** pair, cudaStream_t stream);
 
-// delta[row] = sum_d o[row, d] * d_out[row, d] (fp32), rows of D elements of `dtype`.
+// delta[row] = sum_d o[row, d] * d_out[row, d] (fp32), rows of 64 or 128 16-bit elements.
 int launch_delta(const void* o, const void* d_out, float* delta, int64_t rows, int D, int dtype,
                  cudaStream_t stream);
 

@@ -5,186 +5,177 @@
 // Semantics follow the reference's naive kernel and mask
 // (csrc/include/natten/cuda/reference/fna_reference_forward.hpp:63-211, mask.hpp:47-89, 220-225,
 // 306-343): scaled logits, running max, exp, O = sum(p v) / sum(p), LSE = log(sum) + max, extra KV
-// tokens attended by every query. Instead of scanning all keys and masking, each query walks only
-// the keys inside its window box.
+// tokens attended by every query.
 //
-// One warp owns one (batch, token, head) query. Keys are processed 32 at a time: lane l computes
-// the full q.k dot product of key l, the warp reduces max and sum with shuffles, and for P.V every
-// lane owns head-dim columns l, l+32, ... so value rows are read coalesced.
-#include <cuda_bf16.h>
-#include <cuda_fp16.h>
+// A block owns 32 queries of one head and streams the keys of their windows' union past them (see
+// simt_tile.cuh for the split and its reasons): S = Q K^T in 4 x 4 register tiles, online softmax
+// per 64 keys with the 16 lanes that share a row, P through shared memory (read back by the same
+// warp only), O accumulated in registers.
+//
+// Bound: the fp32 pipe on the union boxes, 2-3 times the attended pairs for small windows; for one
+// small map (32 x 32, 128 blocks) the latency of a few dependent steps.
 #include <math.h>
 
+#include <mutex>
+#include <unordered_set>
+
 #include "common.cuh"
+#include "simt_tile.cuh"
 
 namespace b200na {
 namespace {
 
-constexpr int kMaxD = 256;
-constexpr int kWarpsPerBlock = 4;
+using namespace simt;
 
-template <class T> __device__ __forceinline__ float ld_f(const T* p);
-template <> __device__ __forceinline__ float ld_f<float>(const float* p) { return *p; }
-template <> __device__ __forceinline__ float ld_f<__half>(const __half* p) { return __half2float(*p); }
-template <> __device__ __forceinline__ float ld_f<__nv_bfloat16>(const __nv_bfloat16* p) {
-  return __bfloat162float(*p);
-}
-template <class T> __device__ __forceinline__ void st_f(T* p, float v);
-template <> __device__ __forceinline__ void st_f<float>(float* p, float v) { *p = v; }
-template <> __device__ __forceinline__ void st_f<__half>(__half* p, float v) { *p = __float2half_rn(v); }
-template <> __device__ __forceinline__ void st_f<__nv_bfloat16>(__nv_bfloat16* p, float v) {
-  *p = __float2bfloat16_rn(v);
-}
-
-struct SimtParams {
-  NaAxes ax;
-  int64_t N;   // key/value tokens per batch
-  int64_t Nq;  // query tokens per batch (== N except for dense cross attention)
-  int dense;   // dense attention: every query sees keys [0, N) (causal: [0, i + 1))
-  int B, Hq, Hkv, D;
-  int n_extra;
-  float scale;
+template <int DM>
+struct FwdSmem {
+  float q[kRows * (DM + 4)];
+  float k[kCols * (DM + 4)];
+  float v[kCols * (DM + 4)];
+  float w[kRows * kPStride];
+  Cols cols[2];
+  Rows rows;
 };
 
-__device__ __forceinline__ float warp_max(float v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
-  return v;
-}
-__device__ __forceinline__ float warp_sum(float v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
-}
-
-template <class T>
-__global__ void __launch_bounds__(kWarpsPerBlock * 32) na_simt_kernel(
+template <class T, int DM, bool kVec>
+__global__ void __launch_bounds__(kThreads) na_simt_kernel(
     const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v, T* __restrict__ o,
     float* __restrict__ lse, const T* __restrict__ add_k, const T* __restrict__ add_v,
-    const SimtParams p) {
-  __shared__ float q_sm[kWarpsPerBlock][kMaxD];
-  const int lane = threadIdx.x & 31;
-  const int wib = threadIdx.x >> 5;
-  const int64_t total = (int64_t)p.B * p.Nq * p.Hq;
-  const int64_t n_warps = (int64_t)gridDim.x * kWarpsPerBlock;
-  const int rep = p.Hq / p.Hkv;
-  const int D = p.D;
+    const Params p) {
+  extern __shared__ __align__(16) uint8_t smem_raw[];
+  FwdSmem<DM>& sm = *reinterpret_cast<FwdSmem<DM>*>(smem_raw);
+  const int tid = threadIdx.x;
+  const int rg = tid >> 4, cl = tid & 15;
   const int nd = p.ax.ndim;
+  const int dp = (p.D + 3) & ~3;
 
-  for (int64_t w = (int64_t)blockIdx.x * kWarpsPerBlock + wib; w < total; w += n_warps) {
-    const int h = (int)(w % p.Hq);
-    const int64_t bt = w / p.Hq;
-    const int64_t tok = bt % p.Nq;
-    const int64_t b = bt / p.Nq;
-    const int hk = h / rep;
+  for (int64_t item = blockIdx.x; item < p.n_items; item += gridDim.x) {
+    __syncthreads();                 // the previous item's readers are done
+    if (tid < kRows) decode_rows<false>(p, item, sm.rows);
+    __syncthreads();
+    const int64_t n_tok = (int64_t)sm.rows.box_len[0] * sm.rows.box_len[1] * sm.rows.box_len[2];
+    const int64_t n_all = n_tok > 0 ? n_tok + p.n_extra : 0;   // no columns: padding rows only
+    if (tid < kCols) decode_col<false>(p, sm.rows, n_tok, n_all, tid, sm.cols[0], tid);
+    load_rows<T, DM, kVec, kRows>(sm.q, q, sm.rows.row, p.D);
 
-    // window box of this query, in dilation-group coordinates
-    int g[B200NA_MAX_DIM] = {0, 0, 0}, st[B200NA_MAX_DIM] = {0, 0, 0}, len[B200NA_MAX_DIM] = {1, 1, 1};
-    if (p.dense) {
-      len[0] = p.ax.causal[0] ? (int)min((int64_t)tok + 1, p.N) : (int)p.N;
-    } else {
-      int64_t r = tok;
+    float m[4], sum[4], acc[4][OutCols<DM>::kPer];
 #pragma unroll
-      for (int a = B200NA_MAX_DIM - 1; a >= 0; --a) {
-        if (a < nd) {
-          const int c = (int)(r % p.ax.shape[a]);
-          r /= p.ax.shape[a];
-          const int d = p.ax.dilation[a];
-          g[a] = c % d;
-          const int i = c / d;
-          const int L = group_extent(p.ax.shape[a], d, g[a]);
-          st[a] = win_start(i, p.ax.kernel[a], p.ax.stride[a], L, p.ax.causal[a]);
-          len[a] = win_end(i, st[a], p.ax.kernel[a], L, p.ax.causal[a]) - st[a];
+    for (int r = 0; r < 4; ++r) {
+      m[r] = -INFINITY;
+      sum[r] = 0.f;
+#pragma unroll
+      for (int t = 0; t < OutCols<DM>::kPer; ++t) acc[r][t] = 0.f;
+    }
+    int buf = 0;
+    for (int64_t j0 = 0; j0 < n_all; j0 += kCols, buf ^= 1) {
+      __syncthreads();               // this step's column table is written, the last tiles are read
+      const Cols& cols = sm.cols[buf];
+      load_key_values<T, DM, kVec>(p, sm.rows, cols, j0, n_tok, n_all, sm.k, sm.v, k, v, add_k,
+                                   add_v);
+      if (tid < kCols && j0 + kCols < n_all)
+        decode_col<false>(p, sm.rows, n_tok, n_all, j0 + kCols + tid, sm.cols[buf ^ 1], tid);
+      __syncthreads();
+
+      float s[4][4];
+#pragma unroll
+      for (int r = 0; r < 4; ++r)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) s[r][i] = 0.f;
+      dot_tile<DM>(sm.q, sm.k, rg, cl, dp, s);
+      int4 cc[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) cc[i] = cols.c[cl + 16 * i];
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        float mx = -INFINITY;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          s[r][i] = pair_on(sm.rows, rg * 4 + r, cc[i], nd) ? s[r][i] * p.scale : -INFINITY;
+          mx = fmaxf(mx, s[r][i]);
         }
-      }
-    }
-    const int nk = len[0] * len[1] * len[2];
-    const int n_all = nk + p.n_extra;
-
-    __syncwarp();
-    const T* qr = q + ((b * p.Nq + tok) * p.Hq + h) * D;
-    for (int c = lane; c < D; c += 32) q_sm[wib][c] = ld_f(qr + c);
-    __syncwarp();
-
-    float m = -INFINITY, sum = 0.f;
-    float acc[kMaxD / 32];
+        const float m_new = fmaxf(m[r], row_max(mx));
+        // a row without a key so far keeps -inf; its exponents must not become NaN
+        const float ref = m_new == -INFINITY ? 0.f : m_new;
+        const float corr = expf(m[r] - ref);      // exp(-inf) = 0 on the first keys
+        float part = 0.f;
 #pragma unroll
-    for (int t = 0; t < kMaxD / 32; ++t) acc[t] = 0.f;
-
-    for (int j0 = 0; j0 < n_all; j0 += 32) {
-      const int j = j0 + lane;
-      const T* krow = nullptr;
-      const T* vrow = nullptr;
-      if (j < nk) {
-        int r = j;
-        const int c2 = r % len[2]; r /= len[2];
-        const int c1 = r % len[1]; r /= len[1];
-        const int c0 = r;
-        const int cc[B200NA_MAX_DIM] = {c0, c1, c2};
-        int64_t lin = 0;
-#pragma unroll
-        for (int a = 0; a < B200NA_MAX_DIM; ++a)
-          if (a < nd) lin = lin * p.ax.shape[a] + ((int64_t)(st[a] + cc[a]) * p.ax.dilation[a] + g[a]);
-        krow = k + ((b * p.N + lin) * p.Hkv + hk) * D;
-        vrow = v + ((b * p.N + lin) * p.Hkv + hk) * D;
-      } else if (j < n_all) {
-        const int64_t e = j - nk;
-        krow = add_k + ((b * p.n_extra + e) * p.Hkv + hk) * D;
-        vrow = add_v + ((b * p.n_extra + e) * p.Hkv + hk) * D;
-      }
-      float s = -INFINITY;
-      if (krow) {
-        float d = 0.f;
-        for (int c = 0; c < D; ++c) d = fmaf(q_sm[wib][c], ld_f(krow + c), d);
-        s = d * p.scale;
-      }
-      const float m_new = fmaxf(m, warp_max(s));  // finite: every chunk holds at least one key
-      const float corr = expf(m - m_new);         // exp(-inf) = 0 on the first chunk
-      const float pj = krow ? expf(s - m_new) : 0.f;
-      sum = sum * corr + warp_sum(pj);
-#pragma unroll
-      for (int t = 0; t < kMaxD / 32; ++t) acc[t] *= corr;
-      m = m_new;
-      const int n_here = min(32, n_all - j0);
-      for (int jj = 0; jj < n_here; ++jj) {
-        const float pb = __shfl_sync(0xffffffffu, pj, jj);
-        const T* vr = reinterpret_cast<const T*>(
-            __shfl_sync(0xffffffffu, (unsigned long long)vrow, jj));
-#pragma unroll
-        for (int t = 0; t < kMaxD / 32; ++t) {
-          const int c = lane + 32 * t;
-          if (c < D) acc[t] = fmaf(pb, ld_f(vr + c), acc[t]);
+        for (int i = 0; i < 4; ++i) {
+          const float pj = expf(s[r][i] - ref);
+          part += pj;
+          sm.w[(rg * 4 + r) * kPStride + cl + 16 * i] = pj;
         }
-      }
-    }
-    const float inv = 1.f / sum;
-    T* orow = o + ((b * p.Nq + tok) * p.Hq + h) * D;
+        sum[r] = sum[r] * corr + row_sum(part);
+        m[r] = m_new;
 #pragma unroll
-    for (int t = 0; t < kMaxD / 32; ++t) {
-      const int c = lane + 32 * t;
-      if (c < D) st_f(orow + c, acc[t] * inv);
+        for (int t = 0; t < OutCols<DM>::kPer; ++t) acc[r][t] *= corr;
+      }
+      __syncwarp();                  // P rows are read by the warp that wrote them
+      const int n4 = (int)min((int64_t)kCols, (n_all - j0 + 3) & ~(int64_t)3);
+      accumulate_tile<DM>(sm.w, sm.v, rg, cl, n4, acc);
     }
-    if (lse && lane == 0) lse[(b * p.Nq + tok) * p.Hq + h] = logf(sum) + m;
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      const int64_t row = sm.rows.row[rg * 4 + r];
+      if (row < 0) continue;
+      store_row<T, DM>(o + row * p.D, acc[r], 1.f / sum[r], cl, p.D);
+      if (lse && cl == 0) lse[row] = logf(sum[r]) + m[r];
+    }
   }
 }
 
+template <class T, int DM>
+int launch_dm(const void* q, const void* k, const void* v, void* o, float* lse, const void* ak,
+              const void* av, Params& p, cudaStream_t stream) {
+  const bool vec = vectorised(p.D, sizeof(T), reinterpret_cast<uintptr_t>(q) |
+                              reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v));
+  const void* fn = vec ? (const void*)na_simt_kernel<T, DM, true>
+                       : (const void*)na_simt_kernel<T, DM, false>;
+  void* args[] = {(void*)&q, (void*)&k, (void*)&v, (void*)&o, (void*)&lse, (void*)&ak, (void*)&av,
+                  (void*)&p};
+  return simt::launch(fn, p.n_items, (int)sizeof(FwdSmem<DM>), args, stream);
+}
 template <class T>
-int launch_simt(const void* q, const void* k, const void* v, void* o, float* lse, const void* ak,
-                const void* av, const SimtParams& p, cudaStream_t stream) {
-  int sms = 0;
-  int rc = sm_count_of_current_device(&sms);
-  if (rc != B200NA_OK) return rc;
-  const int64_t total = (int64_t)p.B * p.Nq * p.Hq;
-  int64_t blocks = (total + kWarpsPerBlock - 1) / kWarpsPerBlock;
-  const int64_t cap = (int64_t)sms * 32;
-  if (blocks > cap) blocks = cap;
-  na_simt_kernel<T><<<(int)blocks, kWarpsPerBlock * 32, 0, stream>>>(
-      (const T*)q, (const T*)k, (const T*)v, (T*)o, lse, (const T*)ak, (const T*)av, p);
-  B200NA_CUDA_TRY(cudaGetLastError());
-  return B200NA_OK;
+int launch_fwd(const void* q, const void* k, const void* v, void* o, float* lse, const void* ak,
+               const void* av, Params& p, cudaStream_t stream) {
+  plan_rows(p);
+  if (p.D <= 32) return launch_dm<T, 32>(q, k, v, o, lse, ak, av, p, stream);
+  if (p.D <= 64) return launch_dm<T, 64>(q, k, v, o, lse, ak, av, p, stream);
+  if (p.D <= 128) return launch_dm<T, 128>(q, k, v, o, lse, ak, av, p, stream);
+  return launch_dm<T, 256>(q, k, v, o, lse, ak, av, p, stream);
+}
+int launch_typed(const void* q, const void* k, const void* v, void* o, float* lse, const void* ak,
+                 const void* av, Params& p, int dtype, cudaStream_t s) {
+  switch (dtype) {
+    case B200NA_F32: return launch_fwd<float>(q, k, v, o, lse, ak, av, p, s);
+    case B200NA_F16: return launch_fwd<__half>(q, k, v, o, lse, ak, av, p, s);
+    case B200NA_BF16: return launch_fwd<__nv_bfloat16>(q, k, v, o, lse, ak, av, p, s);
+    default: return B200NA_ERR_INVALID_ARGUMENT;
+  }
 }
 
 }  // namespace
+
+namespace simt {
+int launch(const void* fn, int64_t items, int smem_bytes, void** args, cudaStream_t stream) {
+  if (smem_bytes > 48 * 1024) {
+    static std::mutex mu;
+    static std::unordered_set<const void*> done[64];
+    int dev = 0;
+    B200NA_CUDA_TRY(cudaGetDevice(&dev));
+    if (dev < 0 || dev >= 64) return B200NA_ERR_DEVICE;
+    std::lock_guard<std::mutex> lk(mu);
+    if (done[dev].count(fn) == 0) {
+      B200NA_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           smem_bytes));
+      done[dev].insert(fn);
+    }
+  }
+  if (items == 0) return B200NA_OK;
+  const int64_t grid = items < 0x7fffffff ? items : 0x7fffffff;
+  B200NA_CUDA_TRY(cudaLaunchKernel(fn, dim3((unsigned)grid), dim3(kThreads), args, smem_bytes, stream));
+  return B200NA_OK;
+}
+}  // namespace simt
 
 // Dense attention on CUDA cores (fp32 operands, or head dims the tensor-core kernel does not
 // take); called by b200na_fmha_forward.
@@ -192,7 +183,7 @@ int simt_dense_forward(const void* q, const void* k, const void* v, void* o, flo
                        int Nq, int Nk, int Hq, int Hkv, int D, int dtype, float scale, int causal,
                        cudaStream_t stream) {
   if (D > kMaxD) return B200NA_ERR_UNSUPPORTED;
-  SimtParams p;
+  Params p;
   memset(&p, 0, sizeof(p));
   p.ax.ndim = 1;
   for (int a = 0; a < B200NA_MAX_DIM; ++a) {
@@ -200,14 +191,9 @@ int simt_dense_forward(const void* q, const void* k, const void* v, void* o, flo
   }
   p.ax.shape[0] = Nk;
   p.ax.causal[0] = causal ? 1 : 0;
-  p.N = Nk; p.Nq = Nq; p.dense = 1;
-  p.B = B; p.Hq = Hq; p.Hkv = Hkv; p.D = D; p.n_extra = 0; p.scale = scale;
-  switch (dtype) {
-    case B200NA_F32: return launch_simt<float>(q, k, v, o, lse, nullptr, nullptr, p, stream);
-    case B200NA_F16: return launch_simt<__half>(q, k, v, o, lse, nullptr, nullptr, p, stream);
-    case B200NA_BF16: return launch_simt<__nv_bfloat16>(q, k, v, o, lse, nullptr, nullptr, p, stream);
-    default: return B200NA_ERR_INVALID_ARGUMENT;
-  }
+  p.N = Nk; p.Nq = Nq; p.dense = 1; p.G = 1;
+  p.B = B; p.Hq = Hq; p.Hkv = Hkv; p.row_heads = Hq; p.D = D; p.scale = scale;
+  return launch_typed(q, k, v, o, lse, nullptr, nullptr, p, dtype, stream);
 }
 
 }  // namespace b200na
@@ -221,21 +207,21 @@ extern "C" B200NA_API int b200na_na_forward_simt(const void* q, const void* k, c
   using namespace b200na;
   if (!q || !k || !v || !o) return B200NA_ERR_INVALID_ARGUMENT;
   if (B < 1 || Hq < 1 || Hkv < 1 || Hq % Hkv != 0 || D < 1) return B200NA_ERR_INVALID_ARGUMENT;
-  if (D > kMaxD) return B200NA_ERR_UNSUPPORTED;
+  if (D > simt::kMaxD) return B200NA_ERR_UNSUPPORTED;
   if (n_extra < 0 || (n_extra > 0 && (!add_k || !add_v))) return B200NA_ERR_INVALID_ARGUMENT;
-  SimtParams p;
+  simt::Params p;
+  memset(&p, 0, sizeof(p));
   int rc = fill_axes(p.ax, ndim, shape, kernel, stride, dilation, causal);
   if (rc != B200NA_OK) return rc;
   p.N = 1;
-  for (int a = 0; a < ndim; ++a) p.N *= shape[a];
-  p.Nq = p.N;
-  p.dense = 0;
-  p.B = B; p.Hq = Hq; p.Hkv = Hkv; p.D = D; p.n_extra = n_extra; p.scale = scale;
-  cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-  switch (dtype) {
-    case B200NA_F32: return launch_simt<float>(q, k, v, o, lse, add_k, add_v, p, s);
-    case B200NA_F16: return launch_simt<__half>(q, k, v, o, lse, add_k, add_v, p, s);
-    case B200NA_BF16: return launch_simt<__nv_bfloat16>(q, k, v, o, lse, add_k, add_v, p, s);
-    default: return B200NA_ERR_INVALID_ARGUMENT;
+  int64_t groups = 1;
+  for (int a = 0; a < ndim; ++a) {
+    p.N *= shape[a];
+    groups *= p.ax.dilation[a];
   }
+  if (groups > 0x7fffffffLL) return B200NA_ERR_UNSUPPORTED;
+  p.G = (int)groups;
+  p.Nq = p.N;
+  p.B = B; p.Hq = Hq; p.Hkv = Hkv; p.row_heads = Hq; p.D = D; p.n_extra = n_extra; p.scale = scale;
+  return launch_typed(q, k, v, o, lse, add_k, add_v, p, dtype, reinterpret_cast<cudaStream_t>(stream));
 }

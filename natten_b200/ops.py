@@ -283,7 +283,7 @@ def na_backward_simt(query: Tensor, key: Tensor, value: Tensor, out: Tensor, d_o
             _lib.ints(query.shape[1:1 + na_dim]), _lib.ints(kernel_size), _lib.ints(stride),
             _lib.ints(dilation), _lib.ints(_flags(is_causal)), query.shape[0], query.shape[-2],
             key.shape[-2], query.shape[-1], DTYPE_CODE[query.dtype], float(scale),
-            _stream(query)), "b200na_na_backward_simt", kernel_launches=4 if n_extra else 3)
+            _stream(query)), "b200na_na_backward_simt", kernel_launches=3 if n_extra else 2)
     return dq, dk, dv, dak, dav
 
 

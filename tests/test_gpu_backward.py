@@ -146,6 +146,34 @@ def test_dense_attention_gradients(n, causal, hq, hkv, D):
         assert np.abs(t.grad.float().cpu().numpy() - w).max() <= 2e-2 * max(1.0, np.abs(w).max())
 
 
+@pytest.mark.parametrize("shape,ks,st,di,ca,hq,hkv,D,n_extra", [
+    ((7,), (3,), (2,), (2,), (True,), 1, 1, 3, 0),            # one row tile, scalar loads
+    ((33,), (32,), (1,), (1,), (False,), 2, 1, 32, 65),       # extras across the 64-column steps
+    ((64,), (64,), (1,), (1,), (True,), 2, 2, 36, 0),         # dense, exact tiles
+    ((9, 65), (3, 33), (1, 5), (3, 1), (False, True), 4, 2, 64, 1),
+    ((5, 6, 7), (2, 3, 7), (1, 2, 1), (2, 1, 1), (False, False, True), 2, 2, 130, 63),
+    ((17, 16), (8, 8), (1, 1), (1, 2), (False, False), 1, 1, 256, 0)])
+def test_cuda_core_tiles_forward_and_backward(shape, ks, st, di, ca, hq, hkv, D, n_extra):
+    """fp32 at the edges of the 32-row / 64-column tiles and of the head-dim variants; tolerances
+    of this file (1e-4 forward, 2e-4 of the largest entry for gradients)."""
+    torch.manual_seed(31)
+    fn = {1: nb.na1d, 2: nb.na2d, 3: nb.na3d}[len(shape)]
+    q, d_out = (torch.randn(2, *shape, hq, D) for _ in range(2))
+    k, v = (torch.randn(2, *shape, hkv, D) for _ in range(2))
+    extras = [torch.randn(2, n_extra, hkv, D) for _ in range(2)] if n_extra else []
+    leaves = [t.cuda().requires_grad_() for t in [q, k, v] + extras]
+    add = dict(additional_keys=leaves[3], additional_values=leaves[4]) if n_extra else {}
+    out, lse = fn(*leaves[:3], ks, st, di, ca, return_lse=True, **add)
+    out.backward(d_out.cuda())
+    ex = dict(add_k=extras[0].numpy(), add_v=extras[1].numpy()) if n_extra else {}
+    want_o, want_l = oracle.na_forward(q.numpy(), k.numpy(), v.numpy(), ks, st, di, ca, **ex)
+    assert np.abs(out.detach().cpu().numpy() - want_o).max() <= 1e-4
+    assert np.abs(lse.detach().cpu().numpy() - want_l).max() <= 1e-4
+    want = oracle.na_backward(q.numpy(), k.numpy(), v.numpy(), d_out.numpy(), ks, st, di, ca, **ex)
+    for t, w in zip(leaves, want):
+        assert np.abs(t.grad.cpu().numpy() - w).max() <= 2e-4 * max(1.0, np.abs(w).max())
+
+
 def test_compiled_training_step_matches_eager():
     """torch.compile (AOT autograd) traces the registered backward too: gradients of a compiled
     layer equal the eager ones."""
