@@ -180,6 +180,20 @@ B200NA_API int b200na_na_forward_direct_strided(
     b200na_stream_t stream);
 
 /*
+ * b200na_na_forward_direct_strided without its limit on 1-D dilation: a dilated 1-D layout is read
+ * as (position in group, group), two axes of the tensor map, so that a tile is 128 positions of one
+ * group whatever the dilation. Two launches instead of one when the dilation (> 1) does not divide
+ * the length: the groups then have two different lengths.
+ */
+B200NA_API int b200na_na_forward_view(
+    const void* q, const void* k, const void* v, const void* add_k, const void* add_v,
+    int n_extra, void* o, float* lse, int ndim, const int* shape, const int* kernel,
+    const int* stride, const int* dilation, const int* causal, const int* q_tile,
+    const int* kv_tile, int B, int Hq, int Hkv, int D, int dtype, float scale,
+    long long q_token_stride, long long k_token_stride, long long v_token_stride,
+    b200na_stream_t stream);
+
+/*
  * The same kernel on one rank's SLAB of a spatially sharded, undilated token layout. The
  * reference has no counterpart (it has no multi-GPU code); window arithmetic follows
  * csrc/include/natten/cuda/reference/mask.hpp:59-89 in layout ("global") coordinates.
@@ -317,7 +331,7 @@ B200NA_API int b200na_na_forward_simt(const void* q, const void* k, const void* 
  *   q, dq, o, d_out: [B, *shape, Hq, D]; k, v, dk, dv: [B, *shape, Hkv, D]; lse: [B, *shape, Hq]
  *   fp32 as returned by the forward; add_k, add_v, d_add_k, d_add_v: [B, n_extra, Hkv, D] or NULL;
  *   delta_scratch: B * prod(shape) * Hq floats of caller-owned scratch (overwritten).
- * Three to four launches (delta, dQ, dK/dV, extra tokens), no atomics: results are deterministic.
+ * Two to three launches (delta and dQ, dK/dV, extra tokens), no atomics: results are deterministic.
  */
 B200NA_API int b200na_na_backward_simt(
     const void* q, const void* k, const void* v, const void* o, const void* d_out, const float* lse,
@@ -348,6 +362,35 @@ B200NA_API int b200na_na_backward_direct(
     const int* stride, const int* dilation, const int* causal, const int* q_tile,
     const int* kv_tile, int B, int Hq, int Hkv, int D, int dtype, float scale,
     b200na_stream_t stream);
+
+/*
+ * b200na_na_backward_direct for tensors as the forward's views take them:
+ *   - q, k, v and dq, dk, dv with token strides of their own (elements between consecutive tokens,
+ *     0 = contiguous), e.g. the three slices of a fused projection and of its gradient; o, d_out,
+ *     lse and the extra tokens are contiguous;
+ *   - D any multiple of 8 up to 128 (below 64 / 128 the tensor maps return zeros for the missing
+ *     channels; a 3-D layout then needs B == 1, otherwise B200NA_ERR_UNSUPPORTED);
+ *   - any 1-D dilation (see b200na_na_forward_view; two launches per pass when it does not divide
+ *     the length).
+ */
+B200NA_API int b200na_na_backward_view(
+    const void* q, const void* k, const void* v, const void* o, const void* d_out, const float* lse,
+    const void* add_k, const void* add_v, int n_extra, void* dq, void* dk, void* dv, void* d_add_k,
+    void* d_add_v, float* delta_scratch, int ndim, const int* shape, const int* kernel,
+    const int* stride, const int* dilation, const int* causal, const int* q_tile,
+    const int* kv_tile, int B, int Hq, int Hkv, int D, int dtype, float scale,
+    long long q_token_stride, long long k_token_stride, long long v_token_stride,
+    long long dq_token_stride, long long dk_token_stride, long long dv_token_stride,
+    b200na_stream_t stream);
+
+/*
+ * Column sums of a [rows, cols] matrix of 16-bit floats (row-major, contiguous), fp32 accumulation in
+ * a fixed order, result in the matrix's type: the bias gradient of a linear layer. cols a multiple of
+ * 8, pointers 16-byte aligned. scratch: b200na_column_sum_scratch(rows, cols) bytes of device memory.
+ */
+B200NA_API int64_t b200na_column_sum_scratch(int64_t rows, int cols);
+B200NA_API int b200na_column_sum(const void* in, void* out, int64_t rows, int cols, int dtype,
+                                 void* scratch, b200na_stream_t stream);
 
 /*
  * Two-way LSE merge: replaces the elementwise chain of natten.merge_attentions

@@ -92,6 +92,11 @@ struct BwdTcParams {
   int n_rtiles;             // row tiles per (batch, group, head)
   int row_heads;            // heads the row tiles carry: Hq (pass dQ) or Hkv (pass dKdV)
   long long total_work;     // n_rtiles * row_heads * B * G
+  int d_real;               // head dim of the tensors (<= the kernel's D; the rest reads as zeros)
+  int sep_heads;            // tensor maps list the head as an axis of its own (d_real < D)
+  int fold_d, fold_g0, fold_len;   // > 0: dilated 1-D layout as (position in group, group), X[0] =
+                            // extent of this launch's G groups, token = position fold_d + fold_g0 + group
+  long long out0_stride, out1_stride;   // elements between consecutive tokens of the outputs
   float scale;              // applied to dQ / dK in the epilogue
   float scale_log2;         // scale * log2(e)
   const float* lse;         // [B, *X, Hq]
@@ -241,6 +246,7 @@ __device__ __forceinline__ void decode_item(const BwdTcParams& p, const WorkCurs
       it.int_lo[a] = 0; it.int_hi[a] = 1;
     }
   }
+  if (NDIM == 1 && p.fold_d) it.g[1] = gl;   // the group is a tensor axis of its own
   it.n_na = it.n_per_head * (kKeyRows ? p.rep : 1);
   it.n_tiles = it.n_na + (kKeyRows ? 0 : p.extra_tiles);
 }
@@ -477,6 +483,9 @@ fna_bwd_kernel(const __grid_constant__ CUtensorMap tm_r1, const __grid_constant_
           lo_a[a] = 0; hi_a[a] = 1;
         }
       }
+      if (NDIM == 1 && p.fold_d)
+        row_tok = (long long)it.b * p.fold_len + (long long)(it.r_lo[0] + tr[0]) * p.fold_d +
+                  p.fold_g0 + it.g[1];
       // pass dQ: the statistics belong to this thread's row
       float row_l = INFINITY, row_d = 0.f;
       if (!kKeyRows && row_valid) {
@@ -516,6 +525,9 @@ fna_bwd_kernel(const __grid_constant__ CUtensorMap tm_r1, const __grid_constant_
                 tok = tok * p.X[a] + (i * p.dil[a] + it.g[a]);
               }
             }
+            if (NDIM == 1 && p.fold_d)
+              tok = (long long)it.b * p.fold_len + (long long)(base3[0] + tcol[0]) * p.fold_d +
+                    p.fold_g0 + it.g[1];
             // a column past the extent gets -LSE = -inf, i.e. P = 0
             // stored negated, so that the packed additions below take them as they are
             stat[row] = ok ? -p.lse[tok * p.Hq + hq] * kLog2e : -INFINITY;
@@ -666,11 +678,11 @@ fna_bwd_kernel(const __grid_constant__ CUtensorMap tm_r1, const __grid_constant_
         break;
       ph_acc ^= 1;
       ptx::tc_fence_after_sync();
-      const long long out_row = row_tok * p.row_heads + it.h;
 #pragma unroll
       for (int acc = 0; acc < (kKeyRows ? 2 : 1); ++acc) {
         constexpr int kCols = D / kParts;  // output columns per thread: 32 or 16
-        T* orow = reinterpret_cast<T*>(acc ? p.out1 : p.out0) + out_row * D + part * kCols;
+        T* orow = reinterpret_cast<T*>(acc ? p.out1 : p.out0) +
+                  row_tok * (acc ? p.out1_stride : p.out0_stride) + it.h * p.d_real + part * kCols;
         const float mul = acc ? 1.f : p.scale;
         const uint32_t src = lane_addr + (acc ? kAcc1Col : kAcc0Col) + part * kCols;
         uint32_t orr[kCols];
@@ -680,6 +692,7 @@ fna_bwd_kernel(const __grid_constant__ CUtensorMap tm_r1, const __grid_constant_
         if (row_valid) {
 #pragma unroll
           for (int v4 = 0; v4 < kCols / 8; ++v4) {
+            if (part * kCols + v4 * 8 >= p.d_real) break;   // rows are d_real elements wide
             uint4 o;
             o.x = pack2<kType>(__uint_as_float(orr[v4 * 8 + 0]) * mul, __uint_as_float(orr[v4 * 8 + 1]) * mul);
             o.y = pack2<kType>(__uint_as_float(orr[v4 * 8 + 2]) * mul, __uint_as_float(orr[v4 * 8 + 3]) * mul);
@@ -925,6 +938,17 @@ fna_bwd_kernel(const __grid_constant__ CUtensorMap tm_r1, const __grid_constant_
       uint32_t ph_re = 1, slot = 0, ph_ce = 1, slot2 = 0, ph_ve = 1, published = 0, tseq = 0;
       BTRACE_DECL(2 * 40)
       bool alive = true;
+      // One 64-channel block of a tile. Narrow heads: (channel, head, `n_axes` layout axes, batch
+      // entry), channels past the head come back as zeros.
+      const int axes = (NDIM == 1 && p.fold_d) ? 2 : NDIM;
+      auto load_tile = [&](uint8_t* dst, const CUtensorMap* tm, uint64_t* bar, int head, int db,
+                           int x0, int x1, int x2, int b, int n_axes) {
+        if (p.sep_heads)
+          ptx::tma_load_5d(dst, tm, bar, db * 64, head, x0, n_axes == 1 ? b : x1,
+                           n_axes == 2 ? b : x2);
+        else
+          ptx::tma_load_5d(dst, tm, bar, head * D + db * 64, x0, x1, x2, b);
+      };
       // items are drawn in order from an atomic counter (row tiles differ a lot in how many
       // column tiles they need: borders, the first rows of a causal axis)
       WorkCursor cur;
@@ -962,10 +986,9 @@ fna_bwd_kernel(const __grid_constant__ CUtensorMap tm_r1, const __grid_constant_
           const int x0 = it.r_lo[0] * p.dil[0] + g0, x1 = it.r_lo[1] * p.dil[1] + g1,
                     x2 = it.r_lo[2] * p.dil[2] + g2;
           for (int db = 0; db < kDBlocks; ++db) {
-            ptx::tma_load_5d(row_sm + db * kBlockBytes, &tm_r1, bars.r_full, it.h * D + db * 64,
-                             x0, x1, x2, b);
-            ptx::tma_load_5d(row_sm + kTileBytes + db * kBlockBytes, &tm_r2, bars.r_full,
-                             it.h * D + db * 64, x0, x1, x2, b);
+            load_tile(row_sm + db * kBlockBytes, &tm_r1, bars.r_full, it.h, db, x0, x1, x2, b, axes);
+            load_tile(row_sm + kTileBytes + db * kBlockBytes, &tm_r2, bars.r_full, it.h, db, x0, x1,
+                      x2, b, axes);
           }
         }
         TileWalk tw;
@@ -1009,9 +1032,9 @@ fna_bwd_kernel(const __grid_constant__ CUtensorMap tm_r1, const __grid_constant_
             BTRACE(1, 6);
             ptx::mbar_arrive_expect_tx(bars.v_full + slot2, kTileBytes);
             for (int db = 0; db < kDBlocks; ++db)
-              ptx::tma_load_5d(col2_sm + slot2 * kTileBytes + db * kBlockBytes,
-                               is_extra ? &tm_e2 : &tm_c2, bars.v_full + slot2,
-                               col_head * D + db * 64, x0, x1, x2, b);
+              load_tile(col2_sm + slot2 * kTileBytes + db * kBlockBytes,
+                        is_extra ? &tm_e2 : &tm_c2, bars.v_full + slot2, col_head, db, x0, x1, x2, b,
+                        is_extra ? 1 : axes);
             if (++slot2 == kStages) {
               slot2 = 0;
               ph_ve ^= 1;
@@ -1023,9 +1046,9 @@ fna_bwd_kernel(const __grid_constant__ CUtensorMap tm_r1, const __grid_constant_
             BTRACE(1, 7);
             ptx::mbar_arrive_expect_tx(bars.c_full + slot, kTileBytes);
             for (int db = 0; db < kDBlocks; ++db)
-              ptx::tma_load_5d(col_sm + slot * kTileBytes + db * kBlockBytes,
-                               is_extra ? &tm_e1 : &tm_c1, bars.c_full + slot,
-                               col_head * D + db * 64, x0, x1, x2, b);
+              load_tile(col_sm + slot * kTileBytes + db * kBlockBytes,
+                        is_extra ? &tm_e1 : &tm_c1, bars.c_full + slot, col_head, db, x0, x1, x2, b,
+                        is_extra ? 1 : axes);
           } else {
             if (!wait_bar(bars.c_empty + slot, ph_ce, abort_flag, p.status,
                           (7 << 8) | kStCEmpty)) {
@@ -1034,10 +1057,10 @@ fna_bwd_kernel(const __grid_constant__ CUtensorMap tm_r1, const __grid_constant_
             ptx::mbar_arrive_expect_tx(bars.c_full + slot, 2 * kTileBytes);
             uint8_t* dst = col_sm + slot * 2 * kTileBytes;
             for (int db = 0; db < kDBlocks; ++db) {
-              ptx::tma_load_5d(dst + db * kBlockBytes, is_extra ? &tm_e1 : &tm_c1,
-                               bars.c_full + slot, col_head * D + db * 64, x0, x1, x2, b);
-              ptx::tma_load_5d(dst + kTileBytes + db * kBlockBytes, is_extra ? &tm_e2 : &tm_c2,
-                               bars.c_full + slot, col_head * D + db * 64, x0, x1, x2, b);
+              load_tile(dst + db * kBlockBytes, &tm_c1, bars.c_full + slot, col_head, db, x0, x1, x2,
+                        b, axes);
+              load_tile(dst + kTileBytes + db * kBlockBytes, &tm_c2, bars.c_full + slot, col_head, db,
+                        x0, x1, x2, b, axes);
             }
           }
           if (++slot == kRing1) {
@@ -1128,35 +1151,66 @@ int ensure_smem_attribute(const void* fn, int smem_bytes) {
 }  // namespace
 }  // namespace b200na
 
-extern "C" B200NA_API int b200na_na_backward_direct(
-    const void* q, const void* k, const void* v, const void* o, const void* d_out, const float* lse,
-    const void* add_k, const void* add_v, int n_extra, void* dq, void* dk, void* dv, void* d_add_k,
-    void* d_add_v, float* delta_scratch, int ndim, const int* shape, const int* kernel,
-    const int* stride, const int* dilation, const int* causal, const int* q_tile,
-    const int* kv_tile, int B, int Hq, int Hkv, int D, int dtype, float scale,
-    b200na_stream_t stream_) {
-  using namespace b200na;
-  if (!q || !k || !v || !o || !d_out || !lse || !dq || !dk || !dv || !delta_scratch || !shape ||
-      !kernel || !q_tile || !kv_tile)
+namespace b200na {
+namespace {
+struct BwdCall {
+  const void *q, *k, *v, *o, *d_out;
+  const float* lse;
+  const void *add_k, *add_v;
+  int n_extra;
+  void *dq, *dk, *dv, *d_add_k, *d_add_v;
+  float* delta;
+  // elements between consecutive tokens, 0 = contiguous
+  long long q_ts, k_ts, v_ts, dq_ts, dk_ts, dv_ts;
+  bool views;   // narrow head dims and folded 1-D dilation allowed
+};
+
+// One pass over one part of the layout (all of it, or the dilation groups of a folded 1-D part).
+int launch_pass(const BwdTcParams& p, int D, int dtype, int kernel_ndim, bool key_rows, void** args,
+                int sms, cudaStream_t stream) {
+  const void* fn = bwd_kernel_variant(D, dtype == B200NA_BF16, kernel_ndim, key_rows);
+  const int smem_bytes = key_rows ? (D == 128 ? Smem<128, false>::kBytes : Smem<64, false>::kBytes)
+                                  : (D == 128 ? Smem<128, true>::kBytes : Smem<64, true>::kBytes);
+  const int rc = ensure_smem_attribute(fn, smem_bytes);
+  if (rc != B200NA_OK) return rc;
+  const int grid = (int)(p.total_work < sms ? p.total_work : sms);
+  B200NA_CUDA_TRY(cudaLaunchKernel(fn, dim3(grid), dim3(kThreads), args, smem_bytes, stream));
+  return B200NA_OK;
+}
+
+int backward_impl(const BwdCall& c, int ndim, const int* shape, const int* kernel, const int* stride,
+                  const int* dilation, const int* causal, const int* q_tile, const int* kv_tile,
+                  int B, int Hq, int Hkv, int D, int dtype, float scale, cudaStream_t stream) {
+  if (!c.q || !c.k || !c.v || !c.o || !c.d_out || !c.lse || !c.dq || !c.dk || !c.dv || !c.delta ||
+      !shape || !kernel || !q_tile || !kv_tile)
     return B200NA_ERR_INVALID_ARGUMENT;
-  if (n_extra < 0 || (n_extra > 0 && (!add_k || !add_v || !d_add_k || !d_add_v)))
+  const int n_extra = c.n_extra;
+  if (n_extra < 0 || (n_extra > 0 && (!c.add_k || !c.add_v || !c.d_add_k || !c.d_add_v)))
     return B200NA_ERR_INVALID_ARGUMENT;
   if (B < 1 || Hq < 1 || Hkv < 1 || Hq % Hkv != 0) return B200NA_ERR_INVALID_ARGUMENT;
   if (dtype != B200NA_F16 && dtype != B200NA_BF16) return B200NA_ERR_UNSUPPORTED;
-  if (D != 64 && D != 128) return B200NA_ERR_UNSUPPORTED;
+  const bool narrow = D != 64 && D != 128;
+  if (D < 8 || D > 128 || D % 8 != 0 || (narrow && !c.views)) return B200NA_ERR_UNSUPPORTED;
+  const int Dk = D <= 64 ? 64 : 128;   // head dim of the kernel
   if (!(scale > 0.f)) return B200NA_ERR_INVALID_ARGUMENT;
-  uintptr_t al = reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) |
-                 reinterpret_cast<uintptr_t>(v) | reinterpret_cast<uintptr_t>(d_out) |
-                 reinterpret_cast<uintptr_t>(dq) | reinterpret_cast<uintptr_t>(dk) |
-                 reinterpret_cast<uintptr_t>(dv);
+  const long long wq = (long long)Hq * D, wkv = (long long)Hkv * D;
+  const long long q_ts = c.q_ts ? c.q_ts : wq, k_ts = c.k_ts ? c.k_ts : wkv,
+                  v_ts = c.v_ts ? c.v_ts : wkv, dq_ts = c.dq_ts ? c.dq_ts : wq,
+                  dk_ts = c.dk_ts ? c.dk_ts : wkv, dv_ts = c.dv_ts ? c.dv_ts : wkv;
+  if (q_ts < wq || k_ts < wkv || v_ts < wkv || dq_ts < wq || dk_ts < wkv || dv_ts < wkv)
+    return B200NA_ERR_INVALID_ARGUMENT;
+  uintptr_t al = reinterpret_cast<uintptr_t>(c.q) | reinterpret_cast<uintptr_t>(c.k) |
+                 reinterpret_cast<uintptr_t>(c.v) | reinterpret_cast<uintptr_t>(c.d_out) |
+                 reinterpret_cast<uintptr_t>(c.dq) | reinterpret_cast<uintptr_t>(c.dk) |
+                 reinterpret_cast<uintptr_t>(c.dv) |
+                 (uintptr_t)((q_ts | k_ts | v_ts | dq_ts | dk_ts | dv_ts) * 2);
   if (n_extra > 0)
-    al |= reinterpret_cast<uintptr_t>(add_k) | reinterpret_cast<uintptr_t>(add_v) |
-          reinterpret_cast<uintptr_t>(d_add_k) | reinterpret_cast<uintptr_t>(d_add_v);
+    al |= reinterpret_cast<uintptr_t>(c.add_k) | reinterpret_cast<uintptr_t>(c.add_v) |
+          reinterpret_cast<uintptr_t>(c.d_add_k) | reinterpret_cast<uintptr_t>(c.d_add_v);
   if (al % 16 != 0) return B200NA_ERR_ALIGNMENT;
   NaAxes ax;
   int rc = fill_axes(ax, ndim, shape, kernel, stride, dilation, causal);
   if (rc != B200NA_OK) return rc;
-  cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
   int sms = 0;
   int* status_ptr = nullptr;
   if ((rc = fna_device_info(&sms, &status_ptr)) != B200NA_OK) return rc;
@@ -1182,86 +1236,143 @@ extern "C" B200NA_API int b200na_na_backward_direct(
   if (nq != kTile || nkv != kTile) return B200NA_ERR_INVALID_ARGUMENT;
   if (tokens * B > 0x7fffffffLL || (long long)Hq * D > 0x7fffffffLL) return B200NA_ERR_UNSUPPORTED;
   base.B = B; base.Hq = Hq; base.Hkv = Hkv; base.rep = Hq / Hkv;
+  base.d_real = D;
+  base.sep_heads = narrow ? 1 : 0;
   base.scale = scale;
   base.scale_log2 = scale * 1.4426950408889634f;
-  base.lse = lse;
-  base.delta = delta_scratch;
+  base.lse = c.lse;
+  base.delta = c.delta;
   base.status = status_ptr;
 
-  CUtensorMap mq, mdo, mk, mv;
-  if ((rc = fna_make_tensor_map_direct(&mq, q, dtype, B, base.X, Hq, D, tq, base.dil)) != B200NA_OK) return rc;
-  if ((rc = fna_make_tensor_map_direct(&mdo, d_out, dtype, B, base.X, Hq, D, tq, base.dil)) != B200NA_OK) return rc;
-  if ((rc = fna_make_tensor_map_direct(&mk, k, dtype, B, base.X, Hkv, D, tkv, base.dil)) != B200NA_OK) return rc;
-  if ((rc = fna_make_tensor_map_direct(&mv, v, dtype, B, base.X, Hkv, D, tkv, base.dil)) != B200NA_OK) return rc;
   // extra tokens [B, n_extra, Hkv, D] are a one-axis layout of their own; flat views of Q / dO
   // ([B, N, Hq, D]) serve the pass that computes their gradients
   const int flat_tile[B200NA_MAX_DIM] = {kTile, 1, 1}, ones[B200NA_MAX_DIM] = {1, 1, 1};
   const int x_extra[B200NA_MAX_DIM] = {n_extra > 0 ? n_extra : 1, 1, 1};
   const int x_flat[B200NA_MAX_DIM] = {(int)tokens, 1, 1};
-  CUtensorMap mek = mk, mev = mv, mqf = mq, mdof = mdo;
+  const int sep1 = narrow ? 1 : 0, sep = narrow ? ndim : 0;
+  CUtensorMap mek, mev, mqf, mdof;
   if (n_extra > 0) {
-    if ((rc = fna_make_tensor_map_direct(&mek, add_k, dtype, B, x_extra, Hkv, D, flat_tile, ones)) != B200NA_OK) return rc;
-    if ((rc = fna_make_tensor_map_direct(&mev, add_v, dtype, B, x_extra, Hkv, D, flat_tile, ones)) != B200NA_OK) return rc;
-    if ((rc = fna_make_tensor_map_direct(&mqf, q, dtype, B, x_flat, Hq, D, flat_tile, ones)) != B200NA_OK) return rc;
-    if ((rc = fna_make_tensor_map_direct(&mdof, d_out, dtype, B, x_flat, Hq, D, flat_tile, ones)) != B200NA_OK) return rc;
+    if ((rc = fna_make_tensor_map_direct(&mek, c.add_k, dtype, B, x_extra, Hkv, D, flat_tile, ones, 0, sep1)) != B200NA_OK) return rc;
+    if ((rc = fna_make_tensor_map_direct(&mev, c.add_v, dtype, B, x_extra, Hkv, D, flat_tile, ones, 0, sep1)) != B200NA_OK) return rc;
+    if ((rc = fna_make_tensor_map_direct(&mqf, c.q, dtype, B, x_flat, Hq, D, flat_tile, ones, q_ts, sep1)) != B200NA_OK) return rc;
+    if ((rc = fna_make_tensor_map_direct(&mdof, c.d_out, dtype, B, x_flat, Hq, D, flat_tile, ones, 0, sep1)) != B200NA_OK) return rc;
   }
 
-  if ((rc = launch_delta(o, d_out, delta_scratch, tokens * B * Hq, D, dtype, stream)) != B200NA_OK)
-    return rc;
-
-  // pass 0: dQ (rows Q, dO; columns K, V, then the extra tokens); pass 1: dK, dV (rows K, V;
-  // columns Q, dO); pass 2, with extra tokens only: their gradients (rows = the extra tokens,
-  // columns = all queries of the batch entry, flat)
-  for (int pass = 0; pass < (n_extra > 0 ? 3 : 2); ++pass) {
-    const bool key_rows = pass >= 1;
-    const bool dense = pass == 2;
-    BwdTcParams p = base;
-    int kernel_ndim = ndim;
-    if (dense) {
-      kernel_ndim = 1;
-      p.ndim = 1;
-      p.G = 1;
-      p.dense_rows = 1;
-      p.row_extent = n_extra;
-      for (int a = 0; a < B200NA_MAX_DIM; ++a) {
-        p.X[a] = a == 0 ? (int)tokens : 1;
-        p.kernel[a] = 1; p.stride[a] = 1; p.dil[a] = 1; p.causal[a] = 0;
+  FoldedPart parts[2] = {{0, 0, 0}, {0, 0, 0}};
+  const int n_fold = c.views ? fna_fold_parts(ndim, base.X[0], base.dil[0], parts) : 0;
+  bool delta_done = false;
+  for (int part = 0; part < (n_fold ? n_fold : 1); ++part) {
+    BwdTcParams view = base;
+    FoldedAxis folded = {base.dil[0], parts[part].g0, parts[part].groups, base.X[0]};
+    const FoldedAxis* fold = n_fold ? &folded : nullptr;
+    if (n_fold) {
+      view.fold_d = folded.d;
+      view.fold_g0 = folded.g0;
+      view.fold_len = folded.len;
+      view.G = folded.groups;
+      view.dil[0] = 1;
+      view.X[0] = parts[part].extent;
+    }
+    CUtensorMap mq, mdo, mk, mv;
+    if ((rc = fna_make_tensor_map_direct(&mq, c.q, dtype, B, view.X, Hq, D, tq, view.dil, q_ts, sep, fold)) != B200NA_OK) return rc;
+    if ((rc = fna_make_tensor_map_direct(&mdo, c.d_out, dtype, B, view.X, Hq, D, tq, view.dil, 0, sep, fold)) != B200NA_OK) return rc;
+    if ((rc = fna_make_tensor_map_direct(&mk, c.k, dtype, B, view.X, Hkv, D, tkv, view.dil, k_ts, sep, fold)) != B200NA_OK) return rc;
+    if ((rc = fna_make_tensor_map_direct(&mv, c.v, dtype, B, view.X, Hkv, D, tkv, view.dil, v_ts, sep, fold)) != B200NA_OK) return rc;
+    if (n_extra == 0) { mek = mk; mev = mv; }
+    if (!delta_done) {   // after every check of the first part
+      if ((rc = launch_delta(c.o, c.d_out, c.delta, tokens * B * Hq, D, dtype, stream)) != B200NA_OK)
+        return rc;
+      delta_done = true;
+    }
+    // pass 0: dQ (rows Q, dO; columns K, V, then the extra tokens); pass 1: dK, dV (rows K, V;
+    // columns Q, dO)
+    for (int pass = 0; pass < 2; ++pass) {
+      const bool key_rows = pass == 1;
+      BwdTcParams p = view;
+      if (!key_rows) {
+        p.n_extra = n_extra;
+        p.extra_tiles = (n_extra + kTile - 1) / kTile;
       }
+      long long n_rtiles = 1;
+      for (int a = 0; a < B200NA_MAX_DIM; ++a) {
+        p.Tr[a] = key_rows ? tkv[a] : tq[a];
+        p.Tc[a] = key_rows ? tq[a] : tkv[a];
+        const int need = (p.X[a] + p.dil[a] - 1) / p.dil[a];   // the largest dilation group
+        p.Rr[a] = (need + p.Tr[a] - 1) / p.Tr[a];
+        n_rtiles *= p.Rr[a];
+      }
+      if (n_rtiles > 0x7fffffffLL) return B200NA_ERR_UNSUPPORTED;
+      p.n_rtiles = (int)n_rtiles;
+      p.row_heads = key_rows ? Hkv : Hq;
+      p.total_work = n_rtiles * p.row_heads * B * p.G;
+      p.out0 = key_rows ? c.dk : c.dq;
+      p.out1 = key_rows ? c.dv : nullptr;
+      p.out0_stride = key_rows ? dk_ts : dq_ts;
+      p.out1_stride = dv_ts;
+      if ((rc = fna_work_counters(&p.work, stream)) != B200NA_OK) return rc;
+      p.trace = pass == g_bwd_trace_pass ? g_bwd_trace : nullptr;
+      void* args_q[] = {(void*)&mq, (void*)&mdo, (void*)&mk, (void*)&mv, (void*)&mek, (void*)&mev, (void*)&p};
+      void* args_k[] = {(void*)&mk, (void*)&mv, (void*)&mq, (void*)&mdo, (void*)&mek, (void*)&mev, (void*)&p};
+      if ((rc = launch_pass(p, Dk, dtype, ndim, key_rows, key_rows ? args_k : args_q, sms, stream)) !=
+          B200NA_OK)
+        return rc;
     }
-    if (pass == 0) {
-      p.n_extra = n_extra;
-      p.extra_tiles = (n_extra + kTile - 1) / kTile;
-    }
-    long long n_rtiles = 1;
-    for (int a = 0; a < B200NA_MAX_DIM; ++a) {
-      p.Tr[a] = dense ? flat_tile[a] : (key_rows ? tkv[a] : tq[a]);
-      p.Tc[a] = dense ? flat_tile[a] : (key_rows ? tq[a] : tkv[a]);
-      // rows per axis: the largest dilation group, or the extra tokens
-      const int need = dense ? (a == 0 ? n_extra : 1) : (p.X[a] + p.dil[a] - 1) / p.dil[a];
-      p.Rr[a] = (need + p.Tr[a] - 1) / p.Tr[a];
-      n_rtiles *= p.Rr[a];
-    }
-    if (n_rtiles > 0x7fffffffLL) return B200NA_ERR_UNSUPPORTED;
-    p.n_rtiles = (int)n_rtiles;
-    p.row_heads = key_rows ? Hkv : Hq;
-    p.total_work = n_rtiles * p.row_heads * B * p.G;
-    p.out0 = dense ? d_add_k : (key_rows ? dk : dq);
-    p.out1 = dense ? d_add_v : (key_rows ? dv : nullptr);
-    if ((rc = fna_work_counters(&p.work, stream)) != B200NA_OK) return rc;
-    p.trace = pass == g_bwd_trace_pass ? g_bwd_trace : nullptr;
-    const void* fn = bwd_kernel_variant(D, dtype == B200NA_BF16, kernel_ndim, key_rows);
-    const int smem_bytes = key_rows ? (D == 128 ? Smem<128, false>::kBytes : Smem<64, false>::kBytes)
-                                    : (D == 128 ? Smem<128, true>::kBytes : Smem<64, true>::kBytes);
-    if ((rc = ensure_smem_attribute(fn, smem_bytes)) != B200NA_OK) return rc;
-    const int grid = (int)(p.total_work < sms ? p.total_work : sms);
-    void* args_q[] = {(void*)&mq, (void*)&mdo, (void*)&mk, (void*)&mv, (void*)&mek, (void*)&mev, (void*)&p};
-    void* args_k[] = {(void*)&mk, (void*)&mv, (void*)&mq, (void*)&mdo, (void*)&mek, (void*)&mev, (void*)&p};
-    void* args_e[] = {(void*)&mek, (void*)&mev, (void*)&mqf, (void*)&mdof, (void*)&mek, (void*)&mev, (void*)&p};
-    B200NA_CUDA_TRY(cudaLaunchKernel(fn, dim3(grid), dim3(kThreads),
-                                     dense ? args_e : (key_rows ? args_k : args_q), smem_bytes,
-                                     stream));
   }
-  return B200NA_OK;
+  if (n_extra == 0) return B200NA_OK;
+  // gradients of the extra tokens: rows = the extra tokens, columns = all queries of the batch
+  // entry, flat
+  BwdTcParams p = base;
+  p.ndim = 1;
+  p.G = 1;
+  p.dense_rows = 1;
+  p.row_extent = n_extra;
+  for (int a = 0; a < B200NA_MAX_DIM; ++a) {
+    p.X[a] = a == 0 ? (int)tokens : 1;
+    p.kernel[a] = 1; p.stride[a] = 1; p.dil[a] = 1; p.causal[a] = 0;
+    p.Tr[a] = p.Tc[a] = flat_tile[a];
+    p.Rr[a] = 1;
+  }
+  p.Rr[0] = p.n_rtiles = (n_extra + kTile - 1) / kTile;
+  p.row_heads = Hkv;
+  p.total_work = (long long)p.n_rtiles * Hkv * B;
+  p.out0 = c.d_add_k;
+  p.out1 = c.d_add_v;
+  p.out0_stride = p.out1_stride = wkv;
+  if ((rc = fna_work_counters(&p.work, stream)) != B200NA_OK) return rc;
+  p.trace = g_bwd_trace_pass == 2 ? g_bwd_trace : nullptr;
+  void* args[] = {(void*)&mek, (void*)&mev, (void*)&mqf, (void*)&mdof, (void*)&mek, (void*)&mev, (void*)&p};
+  return launch_pass(p, Dk, dtype, 1, true, args, sms, stream);
+}
+}  // namespace
+}  // namespace b200na
+
+extern "C" B200NA_API int b200na_na_backward_direct(
+    const void* q, const void* k, const void* v, const void* o, const void* d_out, const float* lse,
+    const void* add_k, const void* add_v, int n_extra, void* dq, void* dk, void* dv, void* d_add_k,
+    void* d_add_v, float* delta_scratch, int ndim, const int* shape, const int* kernel,
+    const int* stride, const int* dilation, const int* causal, const int* q_tile,
+    const int* kv_tile, int B, int Hq, int Hkv, int D, int dtype, float scale,
+    b200na_stream_t stream) {
+  const b200na::BwdCall c = {q, k, v, o, d_out, lse, add_k, add_v, n_extra, dq, dk, dv, d_add_k,
+                             d_add_v, delta_scratch, 0, 0, 0, 0, 0, 0, false};
+  return b200na::backward_impl(c, ndim, shape, kernel, stride, dilation, causal, q_tile, kv_tile, B,
+                               Hq, Hkv, D, dtype, scale, reinterpret_cast<cudaStream_t>(stream));
+}
+
+extern "C" B200NA_API int b200na_na_backward_view(
+    const void* q, const void* k, const void* v, const void* o, const void* d_out, const float* lse,
+    const void* add_k, const void* add_v, int n_extra, void* dq, void* dk, void* dv, void* d_add_k,
+    void* d_add_v, float* delta_scratch, int ndim, const int* shape, const int* kernel,
+    const int* stride, const int* dilation, const int* causal, const int* q_tile,
+    const int* kv_tile, int B, int Hq, int Hkv, int D, int dtype, float scale,
+    long long q_token_stride, long long k_token_stride, long long v_token_stride,
+    long long dq_token_stride, long long dk_token_stride, long long dv_token_stride,
+    b200na_stream_t stream) {
+  const b200na::BwdCall c = {q, k, v, o, d_out, lse, add_k, add_v, n_extra, dq, dk, dv, d_add_k,
+                             d_add_v, delta_scratch, q_token_stride, k_token_stride, v_token_stride,
+                             dq_token_stride, dk_token_stride, dv_token_stride, true};
+  return b200na::backward_impl(c, ndim, shape, kernel, stride, dilation, causal, q_tile, kv_tile, B,
+                               Hq, Hkv, D, dtype, scale, reinterpret_cast<cudaStream_t>(stream));
 }
 
 #if defined(B200NA_BWD_TRACE) && B200NA_BWD_TRACE

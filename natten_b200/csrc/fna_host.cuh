@@ -10,8 +10,25 @@ namespace b200na {
 // Tensor map over a heads-last [B, X0, X1, X2, H, D] 16-bit tensor seen as (H*D, X0, X1, X2, B):
 // a box of 64 channels x tile[a] * dil[a] positions per axis, traversed with element stride
 // dil[a]. B200NA_ERR_UNSUPPORTED when a box exceeds 256 positions or a stride exceeds 8.
+// token_stride: elements between tokens (0 = H * D); ndim_sep > 0: the head is an axis of its own,
+// (D, H, the ndim_sep layout axes, B), so that channels past a narrow head read as zeros.
+struct FoldedAxis {
+  int d, g0, groups, len;   // dilation, first group, number of groups, tokens of the layout
+};
 int fna_make_tensor_map_direct(CUtensorMap* tm, const void* ptr, int dtype, int B, const int* X,
-                               int H, int D, const int* tile, const int* dil);
+                               int H, int D, const int* tile, const int* dil,
+                               long long token_stride = 0, int ndim_sep = 0,
+                               const FoldedAxis* fold = nullptr);
+
+// A dilated 1-D layout is (position, group) with both as tensor-map axes: a tile of a group is then
+// 128 positions whatever the dilation, where a box of 128 d tokens read with element stride d ends
+// at d = 2 (256 positions). Groups g < len % d are one token longer than the others, and a map has
+// one extent for all: one launch for each of the two kinds. At d = 2 and an odd length the strided
+// box in one launch is kept. Returns the number of launches (0: do not fold).
+struct FoldedPart {
+  int g0, groups, extent;
+};
+int fna_fold_parts(int ndim, int len, int d, FoldedPart (&parts)[2]);
 
 // One-time per-device setup of the attention kernels; returns the SM count and the address of the
 // device status word that bounded waits report into.
@@ -23,7 +40,8 @@ int fna_device_info(int* sms, int** status_ptr);
 // under stream capture gets a pair of its own from a pool of 3072 that is handed out in turn.
 int fna_work_counters(unsigned long long** pair, cudaStream_t stream);
 
-// delta[row] = sum_d o[row, d] * d_out[row, d] (fp32), rows of 64 or 128 16-bit elements.
+// delta[row] = sum_d o[row, d] * d_out[row, d] (fp32), rows of D 16-bit elements (a multiple of
+// 8, at most 128).
 int launch_delta(const void* o, const void* d_out, float* delta, int64_t rows, int D, int dtype,
                  cudaStream_t stream);
 

@@ -95,6 +95,10 @@ struct FnaParams {
   int direct;               // Q/K/V/O/LSE are in the caller's [B, *X, H, D] layout (no permutation)
   long long tok_stride[3];  // direct: elements between consecutive tokens of q, k, v (0 = H * D)
   int half_axis;            // direct: axis along which the query tile splits into its two halves
+  int fold_d;               // > 0: a dilated 1-D layout seen as (position in group, group): X[0] is the
+                            // extent of the G groups of this launch, token = position fold_d + fold_g0
+  int fold_g0;              // + group
+  int fold_len;             // tokens of the whole layout
   int n_extra;              // extra key/value tokens every query attends (0 = none)
   int extra_tiles;          // ceil(n_extra / 128): KV tiles appended to every item's walk
   int Bp, Hq, Hkv;
@@ -252,6 +256,7 @@ __device__ __forceinline__ void decode_item(const FnaParams& p, const WorkCursor
       it.ws_hi[a] = 0; it.we_lo[a] = 1; it.g[a] = 0;
     }
   }
+  if (NDIM == 1 && p.fold_d) it.g[1] = gl;   // the group is a tensor axis of its own
   it.qt = qt;
   if (p.dense && it.qt * kQTile >= p.Sq) it.skip = 1;
   it.n_na = it.n_tiles;
@@ -735,6 +740,8 @@ fna_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
             tok = tok * p.o_ext[a] + ((qa - p.q_org[a]) * p.dil[a] + it.g[a]);
           }
         }
+        if (NDIM == 1 && p.fold_d)
+          tok = (long long)it.b * p.fold_len + (long long)(it.q_lo[0] + tq[0]) * p.fold_d + p.fold_g0 + it.g[1];
         out_row = tok * p.Hq + it.h;
       } else {
         const int q_row = it.qt * kQTile + half * kHalf + row;
@@ -1013,7 +1020,8 @@ fna_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
               if (p.sep_heads) {
                 // (channel, head, then the layout axes and the batch entry): channels past the
                 // tensor's head dim come back as zeros
-                if (NDIM < 3) x[NDIM] = it.b;
+                if (NDIM == 1 && p.fold_d) x[2] = it.b;
+                else if (NDIM < 3) x[NDIM] = it.b;
                 ptx::tma_load_5d(q_sm + h * kTileBytes + db * kBlockBytes, &tm_q, bars.q_full,
                                  db * kBlockElems, it.h, x[0], x[1], x[2]);
               } else {
@@ -1046,6 +1054,11 @@ fna_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
 #pragma unroll
             for (int a = 0; a < B200NA_MAX_DIM; ++a)
               xk[a] = (a < NDIM) ? (walk.lo[a] - p.kv_org[a]) * p.dil[a] + it.g[a] : 0;
+            if (NDIM == 1) xk[1] = it.g[1];   // folded dilation; 0 otherwise
+            if (p.sep_heads) {   // (channel, head, layout axes, batch entry)
+              if (NDIM == 1 && p.fold_d) xk[2] = it.b;
+              else if (NDIM < 3) xk[NDIM] = it.b;
+            }
           }
           if (!is_extra) kv_tile_next<NDIM>(p, it, walk);
           // extra tokens are shared by the dilation groups of a batch entry
@@ -1071,7 +1084,7 @@ fna_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
               if (p.direct && !is_extra && p.sep_heads)
                 ptx::tma_load_5d(kv_sm + slot * kTileBytes + db * kBlockBytes,
                                  kv == 0 ? &tm_k : &tm_v, bars.kv_full + slot, db * kBlockElems, hk,
-                                 xk[0], NDIM < 2 ? it.b : xk[1], NDIM < 3 ? (NDIM < 2 ? 0 : it.b) : xk[2]);
+                                 xk[0], xk[1], xk[2]);
               else if (p.direct && !is_extra)
                 ptx::tma_load_5d(kv_sm + slot * kTileBytes + db * kBlockBytes,
                                  kv == 0 ? &tm_k : &tm_v, bars.kv_full + slot, hk * D + db * kBlockElems,
@@ -1186,13 +1199,41 @@ int make_tensor_map(CUtensorMap* tm, const void* ptr, int dtype, int Bp, int S, 
 // shared memory in the tile's own row order (axis 0 fastest). The box spans 128 bytes of one
 // head's channels and tile[a] * dil[a] positions per axis, traversed with element stride dil[a]:
 // it picks the tile's tokens of one dilation group; positions past an extent read as zeros.
+// `fold`: a dilated 1-D layout as (position in group, group), axes 1 and 2 of the array (2 and 3
+// with the head as an axis of its own): X[0] positions, fold->groups groups.
 int make_tensor_map_direct(CUtensorMap* tm, const void* ptr, int dtype, int B, const int* X,
                            int H, int D, const int* tile, const int* dil,
-                           long long token_stride = 0, int ndim_sep = 0) {
+                           long long token_stride, int ndim_sep, const FoldedAxis* fold) {
   EncodeTiledFn enc = nullptr;
   int rc = get_encode_fn(&enc);
   if (rc != B200NA_OK) return rc;
   const cuuint64_t es = (cuuint64_t)elem_bytes_of(dtype);
+  if (fold) {
+    const cuuint64_t row = (cuuint64_t)(token_stride > 0 ? token_stride : (long long)H * D) * es;
+    if (row % 16 != 0 || (D * es) % 16 != 0 || row < (cuuint64_t)H * D * es) return B200NA_ERR_ALIGNMENT;
+    const cuuint64_t by_pos = row * fold->d, by_batch = row * (cuuint64_t)fold->len;
+    const cuuint32_t ones[5] = {1, 1, 1, 1, 1};
+    const void* base = static_cast<const uint8_t*>(ptr) + row * fold->g0;
+    const cuuint32_t ch = (cuuint32_t)(128 / es), n = (cuuint32_t)tile[0];
+    const cuuint64_t dims_h[5] = {(cuuint64_t)D, (cuuint64_t)H, (cuuint64_t)X[0],
+                                  (cuuint64_t)fold->groups, (cuuint64_t)B};
+    const cuuint64_t str_h[4] = {(cuuint64_t)D * es, by_pos, row, by_batch};
+    const cuuint32_t box_h[5] = {ch, 1, n, 1, 1};
+    const cuuint64_t dims_t[5] = {(cuuint64_t)H * D, (cuuint64_t)X[0], (cuuint64_t)fold->groups, 1,
+                                  (cuuint64_t)B};
+    const cuuint64_t str_t[4] = {by_pos, row, by_batch, by_batch};
+    const cuuint32_t box_t[5] = {ch, n, 1, 1, 1};
+    const CUresult r = enc(tm, tma_type_of(dtype), 5, const_cast<void*>(base),
+                           ndim_sep ? dims_h : dims_t, ndim_sep ? str_h : str_t,
+                           ndim_sep ? box_h : box_t, ones, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                           CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) {
+      set_last_cuda_error(cudaErrorInvalidValue, "cuTensorMapEncodeTiled");
+      return B200NA_ERR_CUDA;
+    }
+    return B200NA_OK;
+  }
   if (ndim_sep > 0) {
     // Head dim below the kernel's: the head becomes an axis of its own, (D, H, then the ndim_sep
     // layout axes, then the batch entry), so that a 128-byte box of channels reads zeros past
@@ -1397,9 +1438,11 @@ int launch_fna(const void* q, const void* k, const void* v, FnaParams& p, int D,
       half_tile[a] = (a == p.half_axis && p.halves == 2) ? p.Tq[a] / 2 : p.Tq[a];
     const int B = p.Bp / p.G;
     const int sep = p.sep_heads ? p.ndim : 0;
-    if ((rc = make_tensor_map_direct(&tq, q, dtype, B, p.o_ext, p.Hq, D, half_tile, p.dil, p.tok_stride[0], sep)) != B200NA_OK) return rc;
-    if ((rc = make_tensor_map_direct(&tk, k, dtype, B, p.kv_ext, p.Hkv, D, p.Tkv, p.dil, p.tok_stride[1], sep)) != B200NA_OK) return rc;
-    if ((rc = make_tensor_map_direct(&tv, v, dtype, B, p.kv_ext, p.Hkv, D, p.Tkv, p.dil, p.tok_stride[2], sep)) != B200NA_OK) return rc;
+    const FoldedAxis folded = {p.fold_d, p.fold_g0, p.G, p.fold_len};
+    const FoldedAxis* fold = p.fold_d ? &folded : nullptr;
+    if ((rc = make_tensor_map_direct(&tq, q, dtype, B, p.o_ext, p.Hq, D, half_tile, p.dil, p.tok_stride[0], sep, fold)) != B200NA_OK) return rc;
+    if ((rc = make_tensor_map_direct(&tk, k, dtype, B, p.kv_ext, p.Hkv, D, p.Tkv, p.dil, p.tok_stride[1], sep, fold)) != B200NA_OK) return rc;
+    if ((rc = make_tensor_map_direct(&tv, v, dtype, B, p.kv_ext, p.Hkv, D, p.Tkv, p.dil, p.tok_stride[2], sep, fold)) != B200NA_OK) return rc;
   } else {
     if ((rc = make_tensor_map(&tq, q, dtype, p.Bp, p.Sq, p.Hq, D)) != B200NA_OK) return rc;
     if ((rc = make_tensor_map(&tk, k, dtype, p.Bp, p.Skv, p.Hkv, D)) != B200NA_OK) return rc;
@@ -1441,8 +1484,17 @@ int launch_fna(const void* q, const void* k, const void* v, FnaParams& p, int D,
 
 namespace b200na {
 int fna_make_tensor_map_direct(CUtensorMap* tm, const void* ptr, int dtype, int B, const int* X,
-                               int H, int D, const int* tile, const int* dil) {
-  return make_tensor_map_direct(tm, ptr, dtype, B, X, H, D, tile, dil);
+                               int H, int D, const int* tile, const int* dil,
+                               long long token_stride, int ndim_sep, const FoldedAxis* fold) {
+  return make_tensor_map_direct(tm, ptr, dtype, B, X, H, D, tile, dil, token_stride, ndim_sep, fold);
+}
+int fna_fold_parts(int ndim, int len, int d, FoldedPart (&parts)[2]) {
+  const int rest = len % d;
+  if (ndim != 1 || d == 1 || (d == 2 && rest != 0)) return 0;
+  int n = 0;
+  if (rest) parts[n++] = {0, rest, len / d + 1};
+  parts[n++] = {rest, d - rest, len / d};
+  return n;
 }
 int fna_work_counters(unsigned long long** pair, cudaStream_t stream) {
   DeviceState* st = nullptr;
@@ -1572,7 +1624,8 @@ int fna_direct_impl(const void* q, const void* k, const void* v, void* o, float*
                     int Hkv, int D, int dtype, float scale, const void* add_k, const void* add_v,
                     int n_extra, const long long* token_strides, b200na_stream_t stream,
                     const int* q_origin = nullptr, const int* q_extent = nullptr,
-                    const int* kv_origin = nullptr, const int* kv_extent = nullptr, int clip = 0) {
+                    const int* kv_origin = nullptr, const int* kv_extent = nullptr, int clip = 0,
+                    bool fold = false) {
   if (!q || !k || !v || !o || !shape || !kernel || !q_tile || !kv_tile)
     return B200NA_ERR_INVALID_ARGUMENT;
   // slabs: q / o / lse hold layout coordinates [q_origin, q_origin + q_extent), k / v hold
@@ -1661,7 +1714,26 @@ int fna_direct_impl(const void* q, const void* k, const void* v, void* o, float*
   p.o = o;
   p.lse = lse;
   p.n_extra = n_extra;
-  return launch_fna(q, k, v, p, D, dtype, reinterpret_cast<cudaStream_t>(stream), add_k, add_v);
+  cudaStream_t cs = reinterpret_cast<cudaStream_t>(stream);
+  FoldedPart parts[2];
+  const int n_parts = !fold ? 0 : fna_fold_parts(ndim, p.X[0], p.dil[0], parts);
+  for (int i = 0; i < n_parts; ++i) {
+    FnaParams f = p;
+    f.fold_d = p.dil[0];
+    f.fold_len = p.X[0];
+    f.fold_g0 = parts[i].g0;
+    f.G = parts[i].groups;
+    f.dil[0] = 1;
+    f.X[0] = f.o_ext[0] = f.kv_ext[0] = f.q_len[0] = parts[i].extent;
+    f.Rq[0] = (parts[i].extent + f.Tq[0] - 1) / f.Tq[0];
+    f.Rkv[0] = (parts[i].extent + f.Tkv[0] - 1) / f.Tkv[0];
+    f.Bp = B * f.G;
+    f.n_qtiles = f.Rq[0];
+    f.Sq = f.Rq[0] * f.Tq[0];
+    f.Skv = f.Rkv[0] * f.Tkv[0];
+    if ((rc = launch_fna(q, k, v, f, D, dtype, cs, add_k, add_v)) != B200NA_OK) return rc;
+  }
+  return n_parts ? B200NA_OK : launch_fna(q, k, v, p, D, dtype, cs, add_k, add_v);
 }
 }  // namespace
 }  // namespace b200na
@@ -1688,6 +1760,19 @@ extern "C" B200NA_API int b200na_na_forward_direct_strided(
   return b200na::fna_direct_impl(q, k, v, o, lse, ndim, shape, kernel, stride, dilation, causal,
                                  q_tile, kv_tile, B, Hq, Hkv, D, dtype, scale, add_k, add_v,
                                  n_extra, ts, stream);
+}
+
+extern "C" B200NA_API int b200na_na_forward_view(
+    const void* q, const void* k, const void* v, const void* add_k, const void* add_v,
+    int n_extra, void* o, float* lse, int ndim, const int* shape, const int* kernel,
+    const int* stride, const int* dilation, const int* causal, const int* q_tile,
+    const int* kv_tile, int B, int Hq, int Hkv, int D, int dtype, float scale,
+    long long q_token_stride, long long k_token_stride, long long v_token_stride,
+    b200na_stream_t stream) {
+  const long long ts[3] = {q_token_stride, k_token_stride, v_token_stride};
+  return b200na::fna_direct_impl(q, k, v, o, lse, ndim, shape, kernel, stride, dilation, causal,
+                                 q_tile, kv_tile, B, Hq, Hkv, D, dtype, scale, add_k, add_v,
+                                 n_extra, ts, stream, nullptr, nullptr, nullptr, nullptr, 0, true);
 }
 
 extern "C" B200NA_API int b200na_na_forward_direct_sharded(

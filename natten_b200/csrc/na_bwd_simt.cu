@@ -197,51 +197,69 @@ int launch_bwd(BwdPointers& a, const Params& p, cudaStream_t stream) {
   return launch_bwd_dm<T, 256>(a, p, stream);
 }
 
-// delta[row] = sum_d dO * O for the tensor-core backward: kLanes lanes per row, 16 bytes each.
+// delta[row] = sum_d dO * O for the tensor-core backward: kLanes (a power of two) lanes per row of
+// `chunks` <= kLanes 16-byte pieces.
 constexpr int kDeltaThreads = 256;
 template <class T, int kLanes>
 __global__ void __launch_bounds__(kDeltaThreads) delta_kernel(const T* __restrict__ o,
                                                               const T* __restrict__ d_out,
                                                               float* __restrict__ delta,
-                                                              int64_t rows, int vec) {
+                                                              int64_t rows, int chunks, int vec) {
   const int64_t i = (int64_t)blockIdx.x * kDeltaThreads + threadIdx.x;
+  const int64_t row = i / kLanes;
+  const int ch = (int)(i % kLanes);
   float acc = 0.f;
-  if (i < rows * kLanes) {
+  if (row < rows && ch < chunks) {
+    const int64_t at = (row * chunks + ch) * 8;
     if (vec) {
-      const uint4 x = *reinterpret_cast<const uint4*>(o + i * 8),
-                  y = *reinterpret_cast<const uint4*>(d_out + i * 8);
+      const uint4 x = *reinterpret_cast<const uint4*>(o + at),
+                  y = *reinterpret_cast<const uint4*>(d_out + at);
       const T* a = reinterpret_cast<const T*>(&x);
       const T* b = reinterpret_cast<const T*>(&y);
 #pragma unroll
       for (int e = 0; e < 8; ++e) acc = fmaf(ldf(a + e), ldf(b + e), acc);
     } else {   // o need not be 16-byte aligned
-      for (int e = 0; e < 8; ++e) acc = fmaf(ldf(o + i * 8 + e), ldf(d_out + i * 8 + e), acc);
+      for (int e = 0; e < 8; ++e) acc = fmaf(ldf(o + at + e), ldf(d_out + at + e), acc);
     }
   }
 #pragma unroll
   for (int off = kLanes / 2; off > 0; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
-  if (i < rows * kLanes && i % kLanes == 0) delta[i / kLanes] = acc;
+  if (row < rows && ch == 0) delta[row] = acc;
+}
+template <class T>
+int launch_delta_typed(const void* o, const void* d_out, float* delta, int64_t rows, int D,
+                       cudaStream_t stream) {
+  const int chunks = D / 8;
+  int lanes = 1;
+  while (lanes < chunks) lanes <<= 1;
+  const int64_t blocks = (rows * lanes + kDeltaThreads - 1) / kDeltaThreads;
+  if (blocks > 0x7fffffff || lanes > 16) return B200NA_ERR_UNSUPPORTED;
+  const int vec = (reinterpret_cast<uintptr_t>(o) | reinterpret_cast<uintptr_t>(d_out)) % 16 == 0;
+#define B200NA_DELTA(L)                                                       \
+  case L:                                                                     \
+    delta_kernel<T, L><<<(unsigned)blocks, kDeltaThreads, 0, stream>>>(       \
+        (const T*)o, (const T*)d_out, delta, rows, chunks, vec);              \
+    break
+  switch (lanes) {
+    B200NA_DELTA(1);
+    B200NA_DELTA(2);
+    B200NA_DELTA(4);
+    B200NA_DELTA(8);
+    B200NA_DELTA(16);
+  }
+#undef B200NA_DELTA
+  B200NA_CUDA_TRY(cudaGetLastError());
+  return B200NA_OK;
 }
 
 }  // namespace
 
 int launch_delta(const void* o, const void* d_out, float* delta, int64_t rows, int D, int dtype,
                  cudaStream_t stream) {
-  const int lanes = D / 8;   // the tensor-core backward takes 16-bit operands, head dim 64 or 128
-  const int64_t blocks = (rows * lanes + kDeltaThreads - 1) / kDeltaThreads;
-  if (blocks > 0x7fffffff) return B200NA_ERR_UNSUPPORTED;
-  const int vec = (reinterpret_cast<uintptr_t>(o) | reinterpret_cast<uintptr_t>(d_out)) % 16 == 0;
-#define B200NA_DELTA(T, L)                                                       \
-  delta_kernel<T, L><<<(unsigned)blocks, kDeltaThreads, 0, stream>>>(            \
-      (const T*)o, (const T*)d_out, delta, rows, vec)
-  if (dtype == B200NA_F16 && lanes == 8) B200NA_DELTA(__half, 8);
-  else if (dtype == B200NA_F16 && lanes == 16) B200NA_DELTA(__half, 16);
-  else if (dtype == B200NA_BF16 && lanes == 8) B200NA_DELTA(__nv_bfloat16, 8);
-  else if (dtype == B200NA_BF16 && lanes == 16) B200NA_DELTA(__nv_bfloat16, 16);
-  else return B200NA_ERR_INVALID_ARGUMENT;
-#undef B200NA_DELTA
-  B200NA_CUDA_TRY(cudaGetLastError());
-  return B200NA_OK;
+  // the tensor-core backward takes 16-bit operands, head dims that are multiples of 8
+  if (dtype == B200NA_F16) return launch_delta_typed<__half>(o, d_out, delta, rows, D, stream);
+  if (dtype == B200NA_BF16) return launch_delta_typed<__nv_bfloat16>(o, d_out, delta, rows, D, stream);
+  return B200NA_ERR_INVALID_ARGUMENT;
 }
 }  // namespace b200na
 
