@@ -6,7 +6,9 @@ from __future__ import annotations
 
 import ctypes
 import os
-from typing import Optional, Sequence
+import sys
+import types
+from typing import Callable, Optional, Sequence
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 # NATTEN_B200_LIB overrides the library path (e.g. an instrumented build of the same sources).
@@ -23,6 +25,7 @@ F32, F16, BF16, E4M3, E5M2 = 0, 1, 2, 3, 4
 SYMBOLS = (
     "b200na_strerror", "b200na_version", "b200na_token_permute", "b200na_token_unpermute",
     "b200na_fna_forward", "b200na_fna_forward_sharded", "b200na_na_forward_direct_sharded", "b200na_fna_forward_extra_kv", "b200na_na_forward_direct", "b200na_na_forward_direct_strided",
+    "b200na_na_forward_view", "b200na_na_backward_view", "b200na_column_sum", "b200na_column_sum_scratch",
     "b200na_fmha_forward",
     "b200na_na_forward", "b200na_na_forward_workspace_bytes", "b200na_na_forward_static", "b200na_na_forward_simt", "b200na_na_backward_simt", "b200na_na_backward_direct", "b200na_merge",
     "b200na_device_status",
@@ -73,12 +76,21 @@ def _load() -> ctypes.CDLL:
         c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_int,
         ip, ip, ip, ip, ip, ip, ip, c_int, c_int, c_int, c_int, c_int, c_float, c_i64, c_i64, c_i64,
         c_void_p]
+    lib.b200na_na_forward_view.restype = c_int
+    lib.b200na_na_forward_view.argtypes = lib.b200na_na_forward_direct_strided.argtypes
+    lib.b200na_column_sum_scratch.restype = c_i64
+    lib.b200na_column_sum_scratch.argtypes = [c_i64, c_int]
+    lib.b200na_column_sum.restype = c_int
+    lib.b200na_column_sum.argtypes = [c_void_p, c_void_p, c_i64, c_int, c_int, c_void_p, c_void_p]
     lib.b200na_na_backward_simt.restype = c_int
     lib.b200na_na_backward_simt.argtypes = [c_void_p] * 8 + [c_int] + [c_void_p] * 6 + [
         c_int, ip, ip, ip, ip, ip, c_int, c_int, c_int, c_int, c_int, c_float, c_void_p]
     lib.b200na_na_backward_direct.restype = c_int
     lib.b200na_na_backward_direct.argtypes = [c_void_p] * 8 + [c_int] + [c_void_p] * 6 + [
         c_int, ip, ip, ip, ip, ip, ip, ip, c_int, c_int, c_int, c_int, c_int, c_float, c_void_p]
+    lib.b200na_na_backward_view.restype = c_int
+    lib.b200na_na_backward_view.argtypes = (lib.b200na_na_backward_direct.argtypes[:-1] + [c_i64] * 6
+                                            + [c_void_p])
     lib.b200na_na_forward_direct_sharded.restype = c_int
     lib.b200na_na_forward_direct_sharded.argtypes = [c_void_p] * 5 + [c_int, c_void_p, c_void_p,
                                                      c_int] + [ip] * 10 + [
@@ -128,16 +140,31 @@ def strerror(code: int) -> str:
     return lib.b200na_strerror(int(code)).decode()
 
 
-# Kernel launches issued through this binding since it was last reset (each successful
-# kernel-launching C-ABI call counts one); read by the benchmark.
-launches = 0
+# `launches`: kernel launches of the package since it was last set; read by the benchmark. The ones
+# issued here are counted by `check`, the ones of the native front (_native.py) by itself.
+_counted = 0
+native_launches: Callable[[], int] = int
+
+
+class _Module(types.ModuleType):
+    @property
+    def launches(self) -> int:
+        return _counted + native_launches()
+
+    @launches.setter
+    def launches(self, value: int) -> None:
+        global _counted
+        _counted = value - native_launches()
+
+
+sys.modules[__name__].__class__ = _Module
 
 
 def check(code: int, where: str, kernel_launches: int = 1) -> None:
-    global launches
+    global _counted
     if code != OK:
         raise NattenB200Error(code, where, strerror(code))
-    launches += kernel_launches
+    _counted += kernel_launches
     if CHECK_STATUS and kernel_launches > 0:
         raise_on_kernel_timeout(where)
 

@@ -20,10 +20,30 @@ LIB_PATH = os.path.join(LIB_DIR, "libnatten_b200.so")
 # millisecond and a host switch that holds one producer arrive back. Used by one GPU test
 # (tests/test_gpu_robustness.py) to make a wait expire; the package never loads it.
 HOOK_LIB_PATH = os.path.join(LIB_DIR, "libnatten_b200_testhooks.so")
-SOURCES = ["capi.cu", "tokperm.cu", "merge.cu", "na_simt.cu", "na_bwd_simt.cu", "fna_sm100.cu", "fna_bwd_sm100.cu", "na_fused.cu"]
+SOURCES = ["capi.cu", "tokperm.cu", "merge.cu", "na_simt.cu", "na_bwd_simt.cu", "fna_sm100.cu", "fna_bwd_sm100.cu", "na_fused.cu", "colsum.cu"]
 HEADERS = ["common.cuh", "ptx.cuh", "fna_host.cuh", "fna_device.cuh", "fna_instrument.cuh", "simt_tile.cuh", os.path.join("..", "..", "include", "natten_b200.h")]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-std=c++17", "-lineinfo",
               "-Xcompiler", "-fPIC", "-Xcompiler", "-fvisibility=hidden"]
+
+
+# The native front of the operators (a CPython module against the installed torch).
+BINDING_SRC = os.path.join(CSRC, "torch_binding.cpp")
+BINDING_PATH = os.path.join(LIB_DIR, "torch_binding.so")
+
+
+def _binding_command() -> list:
+    import sysconfig
+    import torch
+    root = os.path.dirname(torch.__file__)
+    cuda = os.path.dirname(os.path.dirname(os.path.realpath(_nvcc())))
+    return (["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
+             f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"]
+            + [f"-isystem{d}" for d in (os.path.join(root, "include"),
+                                        os.path.join(root, "include/torch/csrc/api/include"),
+                                        os.path.join(cuda, "include"),
+                                        sysconfig.get_paths()["include"])]
+            + [BINDING_SRC, "-o", BINDING_PATH, "-L" + os.path.join(root, "lib"), "-lc10",
+               "-ltorch_cpu", "-ltorch", "-ltorch_python", "-lc10_cuda", "-ldl"])
 
 
 def _nvcc() -> str:
@@ -62,6 +82,10 @@ def build(force: bool = False, verbose: bool = False) -> str:
         hook_proc = subprocess.Popen([nvcc] + NVCC_FLAGS + ["-DB200NA_TEST_HOOKS=1", "-c", hook_src,
                                                             "-o", hook_obj],
                                      stdout=subprocess.PIPE, stderr=subprocess.STDOUT)
+    binding_proc = None
+    if force or _stale(BINDING_PATH, [BINDING_SRC, hdrs[-1]]):
+        binding_proc = subprocess.Popen(_binding_command(), stdout=subprocess.PIPE,
+                                        stderr=subprocess.STDOUT)
     for src, pr in procs:
         out, _ = pr.communicate()
         if verbose or pr.returncode != 0:
@@ -73,6 +97,11 @@ def build(force: bool = False, verbose: bool = False) -> str:
         if hook_proc.returncode != 0:
             sys.stderr.write(out.decode())
             raise RuntimeError("nvcc failed on fna_sm100.cu (test-hook build)")
+    if binding_proc is not None:
+        out, _ = binding_proc.communicate()
+        if binding_proc.returncode != 0:
+            sys.stderr.write(out.decode())
+            raise RuntimeError("g++ failed on torch_binding.cpp")
     link = [nvcc, "-shared", "-gencode", "arch=compute_100a,code=sm_100a"]
     if force or procs or _stale(LIB_PATH, objs):
         subprocess.run(link + ["-o", LIB_PATH] + objs + ["-cudart", "static"], check=True)

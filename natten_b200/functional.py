@@ -12,7 +12,6 @@ unfused extra-token composition register no formula, so differentiating through 
 """
 from __future__ import annotations
 
-import bisect
 import ctypes
 import functools
 import math
@@ -21,7 +20,7 @@ from typing import Any, Dict, List, Optional, Tuple, Union
 import torch
 from torch import Tensor
 
-from . import _lib, ops
+from . import _lib, _native, ops
 from .log import get_logger
 from .checks import (CausalArgType, DimensionType, additional_kv_tensor_checks, check_all_args,
                      check_args_against_input, check_tile_shape, fmha_tensor_checks,
@@ -103,6 +102,13 @@ def _stream(t: Tensor):
     return ctypes.c_void_p(torch.cuda.current_stream(t.device).cuda_stream)
 
 
+def _native_eligible() -> bool:
+    """Whether eager calls may leave for the native front: not while torch.compile traces, and not
+    where this file does more than the operator (debug logging, status checks, forced kernels)."""
+    return (not torch.compiler.is_compiling() and ops.USE_TORCH_OPS and not _lib.CHECK_STATUS
+            and not BACKWARD_ON_CUDA_CORES and not logger.debug_enabled)
+
+
 def _require_cuda(*tensors: Tensor) -> None:
     for t in tensors:
         if t is not None and not t.is_cuda:
@@ -150,23 +156,6 @@ def _axis_tile_cost(X: int, k: int, s: int, d: int, causal: bool, tq: int, tkv: 
     return total
 
 
-def _axis_inverse_tile_cost(X: int, k: int, s: int, d: int, causal: bool, tq: int,
-                            tkv: int) -> int:
-    """Query tiles visited along one axis, summed over that axis' key tiles (largest group), by a
-    pass whose stationary tile holds keys: the walk of a key tile starts at the first query that
-    attends one of its keys and ends after the last one."""
-    L = group_extent(X, d, 0)
-    starts = [window_start(i, k, s, L, causal) for i in range(L)]
-    ends = [window_end(i, starts[i], k, L, causal) for i in range(L)]
-    total = 0
-    for k_lo in range(0, L, tkv):
-        k_hi = min(k_lo + tkv, L) - 1
-        first = bisect.bisect_right(ends, k_lo)       # first query whose window ends beyond k_lo
-        last = bisect.bisect_right(starts, k_hi)      # first query whose window starts beyond k_hi
-        total += max(1, -(-(last - first) // tq))
-    return total
-
-
 def _pow2_compositions(total_log2: int, n: int):
     if n == 1:
         yield (1 << total_log2,)
@@ -191,35 +180,9 @@ def _choose_tile_shapes(shape: DimensionType, kernel_size: DimensionType, stride
                         ) -> Tuple[DimensionType, DimensionType]:
     """Picks (q_tile_shape, kv_tile_shape) - 256 or 128 query tokens, 128 key/value tokens - that
     minimise the tile products the kernel has to compute (the reference instead offers a fixed list:
-    src/natten/backends/configs/cutlass_blackwell/__init__.py:45-64)."""
-    n = len(shape)
-    if n == 1:
-        return (Q_TILE_SIZE,), (KV_TILE_SIZE,)
-    cost: Dict[Tuple[int, int, int, bool], int] = {}
-    for a in range(n):
-        for eq in range(9):
-            for ek in range(8):
-                for aligned in (False, True):
-                    cost[(a, 1 << eq, 1 << ek, aligned)] = _axis_tile_cost(
-                        shape[a], kernel_size[a], stride[a], dilation[a], is_causal[a], 1 << eq,
-                        1 << ek, aligned)
-    best = None
-    for q_log2, weight in ((8, 2.0), (7, SMALL_Q_TILE_PENALTY)):
-        # cost in 128-row x 128-key products: a 256-token query tile makes two per key/value tile
-        for tq in _pow2_compositions(q_log2, n):
-            for tkv in _pow2_compositions(7, n):
-                # tiles the kernel can gather from the caller's layout start at the window; tile
-                # shapes that need token-permuted copies are tied to the tile grid
-                aligned = direct_layout_supported(tq, tkv, dilation)
-                c = weight
-                for a in range(n):
-                    c *= cost[(a, tq[a], tkv[a], aligned)]
-                # ties: prefer tiles that are long along the last (memory-contiguous) axis
-                key = (c, -tq[-1], -tkv[-1])
-                if best is None or key < best[0]:
-                    best = (key, tq, tkv)
-    assert best is not None
-    return best[1], best[2]
+    src/natten/backends/configs/cutlass_blackwell/__init__.py:45-64). The search is native: it runs
+    once per problem, on the first call."""
+    return _native.tiles(False, shape, kernel_size, stride, dilation, is_causal)
 
 
 # ------------------------------------------------------------------------------------------------
@@ -350,6 +313,13 @@ def attention(query: Tensor, key: Tensor, value: Tensor, is_causal: bool = False
               torch_compile: bool = False, return_lse: bool = False
               ) -> Union[Tensor, Tuple[Tensor, Tensor]]:
     """Dense dot-product attention on heads-last ``[B, N, H, D]`` tensors."""
+    if (seqlens_Q is None and seqlens_KV is None and cumulative_seqlen_Q is None
+            and cumulative_seqlen_KV is None and max_seqlen_Q is None and max_seqlen_KV is None
+            and backend is None and q_tile_size is None and kv_tile_size is None
+            and _native_eligible()):
+        result = _native.attention(query, key, value, is_causal, scale, bool(return_lse))
+        if result is not None:
+            return result
     fmha_tensor_checks(query, key, value)
     if any(x is not None for x in (seqlens_Q, seqlens_KV, cumulative_seqlen_Q,
                                    cumulative_seqlen_KV, max_seqlen_Q, max_seqlen_KV)):
@@ -636,33 +606,7 @@ def choose_backward_tile_shapes(shape: DimensionType, kernel_size: DimensionType
 
 @functools.lru_cache(maxsize=256)
 def _choose_backward_tile_shapes(shape, kernel_size, stride, dilation, is_causal):
-    n = len(shape)
-    if n == 1:
-        return (BACKWARD_TILE_SIZE,), (BACKWARD_TILE_SIZE,)
-    cost: Dict[Tuple[int, int, int], Tuple[int, int]] = {}
-    for a in range(n):
-        for eq in range(8):
-            for ek in range(8):
-                args = (shape[a], kernel_size[a], stride[a], dilation[a], is_causal[a], 1 << eq,
-                        1 << ek)
-                cost[(a, 1 << eq, 1 << ek)] = (_axis_tile_cost(*args, True),
-                                               _axis_inverse_tile_cost(*args))
-    best = None
-    for tq in _pow2_compositions(7, n):
-        for tkv in _pow2_compositions(7, n):
-            if not backward_layout_supported(tq, tkv, dilation):
-                continue
-            c_dq = c_dkdv = 1
-            for a in range(n):
-                c_dq *= cost[(a, tq[a], tkv[a])][0]
-                c_dkdv *= cost[(a, tq[a], tkv[a])][1]
-            c = c_dq + c_dkdv
-            key = (c, -tq[-1], -tkv[-1])
-            if best is None or key < best[0]:
-                best = (key, tq, tkv)
-    if best is None:  # no 128-token box fits: the caller falls back to the CUDA-core kernels
-        return (BACKWARD_TILE_SIZE,) + (1,) * (n - 1), (BACKWARD_TILE_SIZE,) + (1,) * (n - 1)
-    return best[1], best[2]
+    return _native.tiles(True, shape, kernel_size, stride, dilation, is_causal)
 
 
 if ops.USE_TORCH_OPS:
@@ -894,6 +838,13 @@ def na1d(query: Tensor, key: Tensor, value: Tensor, kernel_size, stride=1, dilat
          kernel_schedule=None, torch_compile: bool = False, return_lse: bool = False):
     """1-D neighborhood attention on ``[batch, seqlen, heads, head_dim]`` tensors
     (reference: src/natten/functional.py:567-753)."""
+    if (attention_kwargs is None and backend is None and q_tile_shape is None
+            and kv_tile_shape is None and backward_q_tile_shape is None
+            and backward_kv_tile_shape is None and _native_eligible()):
+        result = _native.na(1, query, key, value, kernel_size, stride, dilation, is_causal, scale,
+                            additional_keys, additional_values, bool(return_lse))
+        if result is not None:
+            return result
     return _na(1, query, key, value, kernel_size, stride, dilation, is_causal, scale,
                additional_keys, additional_values, attention_kwargs, backend, q_tile_shape,
                kv_tile_shape, backward_q_tile_shape, backward_kv_tile_shape, backward_kv_splits,
@@ -910,6 +861,13 @@ def na2d(query: Tensor, key: Tensor, value: Tensor, kernel_size, stride=1, dilat
          kernel_schedule=None, torch_compile: bool = False, return_lse: bool = False):
     """2-D neighborhood attention on ``[batch, X, Y, heads, head_dim]`` tensors
     (reference: src/natten/functional.py:756-952)."""
+    if (attention_kwargs is None and backend is None and q_tile_shape is None
+            and kv_tile_shape is None and backward_q_tile_shape is None
+            and backward_kv_tile_shape is None and _native_eligible()):
+        result = _native.na(2, query, key, value, kernel_size, stride, dilation, is_causal, scale,
+                            additional_keys, additional_values, bool(return_lse))
+        if result is not None:
+            return result
     return _na(2, query, key, value, kernel_size, stride, dilation, is_causal, scale,
                additional_keys, additional_values, attention_kwargs, backend, q_tile_shape,
                kv_tile_shape, backward_q_tile_shape, backward_kv_tile_shape, backward_kv_splits,
@@ -926,6 +884,13 @@ def na3d(query: Tensor, key: Tensor, value: Tensor, kernel_size, stride=1, dilat
          kernel_schedule=None, torch_compile: bool = False, return_lse: bool = False):
     """3-D neighborhood attention on ``[batch, X, Y, Z, heads, head_dim]`` tensors
     (reference: src/natten/functional.py:955-1151)."""
+    if (attention_kwargs is None and backend is None and q_tile_shape is None
+            and kv_tile_shape is None and backward_q_tile_shape is None
+            and backward_kv_tile_shape is None and _native_eligible()):
+        result = _native.na(3, query, key, value, kernel_size, stride, dilation, is_causal, scale,
+                            additional_keys, additional_values, bool(return_lse))
+        if result is not None:
+            return result
     return _na(3, query, key, value, kernel_size, stride, dilation, is_causal, scale,
                additional_keys, additional_values, attention_kwargs, backend, q_tile_shape,
                kv_tile_shape, backward_q_tile_shape, backward_kv_tile_shape, backward_kv_splits,

@@ -8,9 +8,17 @@ differentiable.
 from typing import Any, Optional
 
 from torch import Tensor, nn
+from torch.nn.modules.module import _has_any_global_hook
 
+from . import _native
 from .checks import check_all_args
-from .functional import neighborhood_attention_generic
+from .functional import _native_eligible, neighborhood_attention_generic
+
+
+def _is_bare_linear(m: nn.Module) -> bool:
+    """An nn.Linear that does nothing but its product: no subclass, hook or patched forward."""
+    return (type(m) is nn.Linear and not m._forward_hooks and not m._forward_pre_hooks
+            and not m._backward_hooks and not m._backward_pre_hooks and "forward" not in m.__dict__)
 
 
 class NeighborhoodAttentionGeneric(nn.Module):
@@ -44,6 +52,18 @@ class NeighborhoodAttentionGeneric(nn.Module):
         if x.shape[-1] != self.embed_dim:
             raise ValueError(f"Expected embedding dimension {self.embed_dim}, got {x.shape[-1]} "
                              f"({x.shape=}).")
+        # One native call for projection, attention and projection where nothing hangs between them.
+        # In training it is one autograd node: the attention's gradients are written straight into
+        # the fused projection's gradient (no copies of q, k, v gradients), and the bias gradients
+        # are summed by a kernel that reads them at the memory's rate.
+        if _native_eligible() and not _has_any_global_hook():
+            qkv, proj = self.qkv, self.proj
+            if _is_bare_linear(qkv) and _is_bare_linear(proj):
+                y = _native.layer(self.na_dim, x, qkv.weight, qkv.bias, proj.weight, proj.bias,
+                                  self.num_heads, self.kernel_size, self.stride, self.dilation,
+                                  self.is_causal, self.scale)
+                if y is not None:
+                    return self.proj_drop(y)
         lead = x.shape[:-1]
         # [..., 3, heads, head_dim]: q, k, v are strided views of one projection output
         q, k, v = self.qkv(x).unflatten(-1, (3, self.num_heads, self.head_dim)).unbind(-3)

@@ -1,0 +1,108 @@
+"""The native front of the operators (csrc/torch_binding.cpp) and the kernel paths it opened: dilated
+1-D layouts folded into tensor-map axes, narrow head dims in the backward, layers as one autograd
+node, column sums. Against the oracle with the 16-bit tolerance of the other files (2e-2 of the
+largest entry), or against the Python front."""
+import numpy as np
+import pytest
+import torch
+
+import natten_b200 as nb
+import natten_b200._lib as L
+import oracle
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("shape,ks,st,di,ca,hq,hkv,D,n_extra,B", [
+    ((1200,), (33,), (1,), (3,), (True,), 2, 2, 64, 0, 2),      # length a multiple of the dilation
+    ((1201,), (65,), (4,), (3,), (False,), 2, 1, 128, 20, 2),   # two kinds of groups, extra tokens
+    ((515,), (2,), (1,), (257,), (False,), 1, 1, 32, 0, 1),     # one or two keys per group, folded + narrow
+    ((777,), (40,), (1,), (16,), (True,), 4, 2, 24, 130, 2),    # narrow, ragged, GQA, extras
+    ((300,), (33,), (1,), (2,), (False,), 2, 2, 64, 0, 2),      # folded at dilation 2 ...
+    ((301,), (33,), (1,), (2,), (False,), 2, 2, 64, 0, 2),      # ... and the strided box beside it
+    ((33, 30), (3, 5), (1, 2), (3, 2), (False, True), 4, 2, 8, 0, 2),
+    ((31, 29), (7, 7), (1, 1), (1, 1), (False, False), 3, 3, 40, 33, 3),
+    ((5, 12, 20), (3, 5, 6), (1, 1, 2), (1, 1, 1), (True, False, False), 2, 2, 80, 0, 1),
+    ((5, 12, 20), (3, 5, 6), (1, 1, 2), (1, 1, 1), (True, False, False), 2, 2, 120, 9, 1),
+])
+def test_folded_and_narrow_problems(shape, ks, st, di, ca, hq, hkv, D, n_extra, B):
+    torch.manual_seed(41)
+    fn = {1: nb.na1d, 2: nb.na2d, 3: nb.na3d}[len(shape)]
+    q, d_out = (torch.randn(B, *shape, hq, D).half() for _ in range(2))
+    k, v = (torch.randn(B, *shape, hkv, D).half() for _ in range(2))
+    extras = [torch.randn(B, n_extra, hkv, D).half() for _ in range(2)] if n_extra else []
+    leaves = [t.cuda().requires_grad_() for t in [q, k, v] + extras]
+    add = dict(additional_keys=leaves[3], additional_values=leaves[4]) if n_extra else {}
+    before = L.launches
+    out, lse = fn(*leaves[:3], ks, st, di, ca, return_lse=True, **add)
+    assert "NaFunction" in out.grad_fn.name()
+    out.backward(d_out.cuda())
+    assert L.launches - before >= 4 and L.device_status() == 0
+    f = [t.float().numpy() for t in (q, k, v)]
+    ex = dict(add_k=extras[0].float().numpy(), add_v=extras[1].float().numpy()) if n_extra else {}
+    want_o, want_l = oracle.na_forward(*f, ks, st, di, ca, **ex)
+    assert np.abs(out.detach().float().cpu().numpy() - want_o).max() <= 2e-2
+    assert np.abs(lse.detach().cpu().numpy() - want_l).max() <= 2e-2
+    want = oracle.na_backward(*f, d_out.float().numpy(), ks, st, di, ca, **ex)
+    for t, w in zip(leaves, want):
+        assert np.abs(t.grad.float().cpu().numpy() - w).max() <= 2e-2 * max(1.0, np.abs(w).max())
+
+
+@pytest.mark.parametrize("cls,shape,heads,dim,bias", [
+    (nb.NeighborhoodAttention1D, (130,), 2, 64, True), (nb.NeighborhoodAttention2D, (14, 17), 3, 32, True),
+    (nb.NeighborhoodAttention2D, (14, 17), 2, 128, False), (nb.NeighborhoodAttention3D, (6, 9, 11), 2, 64, True)])
+def test_layer_as_one_node_matches_the_layer_in_parts(cls, shape, heads, dim, bias):
+    """A forward hook sends the layer through its modules one by one: same output, same gradients
+    up to the rounding of sums taken in another order (2^-8 of the largest entry: one bf16 step)."""
+    torch.manual_seed(43)
+    layer = cls(heads * dim, heads, 3, dilation=2, qkv_bias=bias).cuda().bfloat16()
+    x, d_y = (torch.randn(2, *shape, heads * dim, device="cuda").bfloat16() for _ in range(2))
+    results = []
+    for hooked in (False, True):
+        handle = layer.qkv.register_forward_hook(lambda *a: None) if hooked else None
+        xi = x.clone().requires_grad_()
+        y = layer(xi)
+        assert ("LayerFunction" in y.grad_fn.name()) != hooked
+        results.append([y.detach()] + list(torch.autograd.grad(y, [xi, *layer.parameters()], d_y)))
+        with torch.no_grad():
+            assert torch.equal(layer(x), y)
+        if hooked:
+            handle.remove()
+    assert L.device_status() == 0
+    for a, b in zip(*results):
+        assert (a.float() - b.float()).abs().max().item() <= 2 ** -8 * b.float().abs().max().item()
+
+
+@pytest.mark.parametrize("rows,cols", [(1, 8), (31, 264), (4097, 96), (100352, 384)])
+def test_column_sums(rows, cols):
+    """fp32 sums rounded once: half a bf16 step (8 significant bits: 2^-8 of the result) plus the fp32
+    summation error,
+    at most rows 2^-24 of the sum of magnitudes; the same bits twice."""
+    torch.manual_seed(47)
+    m = torch.randn(rows, cols, device="cuda").bfloat16()
+    outs = []
+    for _ in range(2):
+        out = torch.empty(cols, device="cuda", dtype=torch.bfloat16)
+        scratch = torch.empty(L.lib.b200na_column_sum_scratch(rows, cols), device="cuda", dtype=torch.uint8)
+        L.check(L.lib.b200na_column_sum(m.data_ptr(), out.data_ptr(), rows, cols, L.BF16,
+                                        scratch.data_ptr(), torch.cuda.current_stream().cuda_stream), "")
+        outs.append(out)
+    want = m.double().sum(0)
+    bound = 2 ** -8 * want.abs() + rows * 2 ** -24 * m.double().abs().sum(0)
+    assert ((outs[0].double() - want).abs() <= bound * 1.01).all() and torch.equal(*outs)
+
+
+def test_native_front_leaves_other_calls_to_the_python_front():
+    q = torch.randn(1, 12, 12, 2, 64, device="cuda").half()
+    for bad in (dict(kernel_size=13), dict(kernel_size=3, stride=4), dict(kernel_size=(3, 3, 3)),
+                dict(kernel_size=True), dict(kernel_size=3, is_causal=(1, 0))):
+        with pytest.raises(ValueError):
+            nb.na2d(q, q, q, **bad)
+    with pytest.raises(RuntimeError):
+        nb.na2d(q.cpu(), q.cpu(), q.cpu(), 3)
+    with pytest.raises(ValueError):
+        nb.na2d(q, q, q.float(), 3)
+    x = q.clone().requires_grad_()
+    (g,) = torch.autograd.grad(nb.na2d(x, q, q, 3).float().sum(), x, create_graph=True)
+    with pytest.raises(RuntimeError):
+        g.float().sum().backward()
