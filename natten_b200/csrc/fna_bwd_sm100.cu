@@ -409,7 +409,7 @@ fna_bwd_kernel(const __grid_constant__ CUtensorMap tm_r1, const __grid_constant_
     ptx::fence_barrier_init();
   }
   // per-axis prefix bit tables over the COLUMN tile, for the masks of boundary tiles
-  build_prefix_tables(pref, p.ndim, p.Tc, threadIdx.x, kThreads);
+  build_prefix_tables(pref, p.ndim, p.Tc, warp, lane, kThreads / 32);
   if (warp == kMmaWarp) {
     ptx::tmem_alloc(tmem_slot, kTmemCols);
     ptx::tmem_relinquish();

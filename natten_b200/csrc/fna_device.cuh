@@ -79,29 +79,27 @@ __device__ __forceinline__ uint4 pack_out16(const uint32_t* f, float mul) {
 
 // Per-axis prefix bit tables over a 128-token tile of shape T (tokens ordered axis 0 fastest):
 // pref[off_a + x], off_a = sum_{b<a} (T[b] + 1), has bit j set iff the in-tile coordinate of
-// token j along axis a is < x. Filled cooperatively by `n_threads` threads; 136 entries suffice.
+// token j along axis a is < x. Filled by the whole warps of the block; 136 entries suffice.
+// A lane is a token: its coordinate is worked out once and a ballot gives a word of the table. (With a
+// thread per entry and a loop over its 128 tokens, two divisions each, this was 25 us of every
+// launch - most of the time of a kernel with one work item per CTA.)
 __device__ __forceinline__ void build_prefix_tables(uint4* pref, int ndim,
-                                                    const int (&T)[B200NA_MAX_DIM], int tid,
-                                                    int n_threads) {
-  int off = 0;
+                                                    const int (&T)[B200NA_MAX_DIM], int warp,
+                                                    int lane, int n_warps) {
+  uint32_t* const words = reinterpret_cast<uint32_t*>(pref);
+  int off = 0, below = 1;
   for (int a = 0; a < ndim; ++a) {
-    int below = 1;
-    for (int b = 0; b < a; ++b) below *= T[b];
-    for (int x = tid; x <= T[a]; x += n_threads) {
-      uint32_t wds[4];
-#pragma unroll
-      for (int wd = 0; wd < 4; ++wd) {
-        uint32_t bits = 0;
-#pragma unroll 1
-        for (int j = 0; j < 32; ++j) {
-          const int t = ((wd * 32 + j) / below) % T[a];
-          if (t < x) bits |= 1u << j;
-        }
-        wds[wd] = bits;
+    // n_warps / 4 warps share a word column wd and take its entries in turn
+    const int wd = warp & 3, step = n_warps >> 2;
+    if (warp < step * 4) {
+      const int c = ((wd * 32 + lane) / below) % T[a];
+      for (int x = warp >> 2; x <= T[a]; x += step) {
+        const uint32_t bits = __ballot_sync(0xffffffffu, c < x);
+        if (lane == 0) words[(off + x) * 4 + wd] = bits;
       }
-      pref[off + x] = make_uint4(wds[0], wds[1], wds[2], wds[3]);
     }
     off += T[a] + 1;
+    below *= T[a];
   }
 }
 

@@ -469,7 +469,7 @@ fna_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
     ptx::fence_barrier_init();
   }
   // per-axis prefix bit tables over the key/value tile, for the masks of boundary tiles
-  build_prefix_tables(pref, p.ndim, p.Tkv, threadIdx.x, kThreads);
+  build_prefix_tables(pref, p.ndim, p.Tkv, warp, lane, kThreads / 32);
   if (warp == kMmaWarp) {
     ptx::tmem_alloc(tmem_slot, kTmemCols);
     ptx::tmem_relinquish();

@@ -485,6 +485,7 @@ struct NaFunction : torch::autograd::Function<NaFunction> {
     saved.insert(saved.end(), in.begin(), in.end());
     ctx->save_for_backward(saved);
     ctx->saved_data["call"] = c10::IValue::make_capsule(call);
+    ctx->set_materialize_grads(false);   // no zeros for the logsumexp's (ignored) gradient
     return {f.out, f.lse};
   }
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
@@ -494,7 +495,8 @@ struct NaFunction : torch::autograd::Function<NaFunction> {
     variable_list g;
     {
       at::AutoDispatchBelowADInplaceOrView below;
-      g = gradients(call->c, saved, grads[0]);
+      // only the logsumexp was differentiated: zeros
+      g = gradients(call->c, saved, grads[0].defined() ? grads[0] : at::zeros_like(saved[0]));
     }
     g.emplace_back();
     return seal(std::move(g));
