@@ -26,11 +26,12 @@
 //     C1 (K) and C2 (V) column tiles have rings of their own there: a C2 stage is free after dP,
 //     a C1 stage only after the dQ product.
 //   * Row statistics (LSE, delta) are per thread in pass dQ; in pass dKdV they belong to the
-//     columns and are staged through shared memory per column tile.
+//     columns and a warp of their own stages them through shared memory, up to four tiles ahead.
 //   * Warp roles: 16 softmax warps (four threads per row, 32 columns each: the P / dS arithmetic
 //     is latency-bound, more warps per sub-partition hide it), 1 MMA-issue warp (pass dQ: a
-//     second one for the dQ products, in another sub-partition), 1 load warp that also decodes
-//     work items and classifies tiles (descriptor / record rings as in the forward kernel). Every mbarrier wait is bounded; on expiry the CTA records a status word
+//     second one for the dQ products, in another sub-partition; pass dKdV: that warp fetches the
+//     columns' LSE and delta), 1 load warp that also decodes work items and classifies tiles
+//     (descriptor / record rings as in the forward kernel). Every mbarrier wait is bounded; on expiry the CTA records a status word
 //     (shared with the forward kernel) and drains.
 #include <cuda.h>
 #include <cuda_bf16.h>
@@ -54,6 +55,8 @@ constexpr int kSoftmaxThreads = 512;
 constexpr int kMmaWarp = 16;
 constexpr int kLoadWarp = 17;
 constexpr int kMma2Warp = 18;       // pass dQ: issues the dQ products (kMmaWarp issues S and dP)
+constexpr int kStatWarp = 18;       // pass dKdV: fetches the columns' statistics, up to kStatBufs
+constexpr int kStatBufs = 4;        // tiles ahead of the threads that use them
 constexpr int kThreads = 608;
 // Registers are allocated to warps in groups of four, so 19 warps cost as much as 20: 96 per
 // thread; the 16-column chunks of the P / dS loop keep the live set well below that.
@@ -66,10 +69,11 @@ constexpr int kDescBytes = 128;
 constexpr int kTileRecs = 8;
 
 // status word: (role << 8) | barrier id; roles 5 = softmax, 6 = mma, 7 = load, 9 = second mma
-// issuer of pass dQ (backward kernel)
+// issuer of pass dQ, 10 = column statistics of pass dKdV (backward kernel)
 enum : int { kStRFull = 1, kStREmpty, kStCFull, kStCEmpty, kStSdpFull, kStDsFull, kStAccFull,
              kStAccEmpty, kStDescFull, kStDescEmpty, kStRecFull, kStRecEmpty, kStSmemAlign,
-             kStSdpFree, kStDsFree, kStVFull, kStVEmpty, kStDpFull, kStPFull };
+             kStSdpFree, kStDsFree, kStVFull, kStVEmpty, kStDpFull, kStPFull,
+             kStStatFull, kStStatEmpty };
 
 struct BwdTcParams {
   int ndim;
@@ -146,14 +150,26 @@ static_assert(sizeof(Item) <= kDescBytes, "descriptor slot too small");
 // Window of a query along one axis, group coordinates: [st, en).
 __device__ __forceinline__ void fwd_window(const BwdTcParams& p, int a, int i, int L, int& st,
                                            int& en) {
-  st = win_start(i, p.kernel[a], p.stride[a], L, p.causal[a]);
-  en = win_end(i, st, p.kernel[a], L, p.causal[a]);
+  const int k = p.kernel[a];
+  if (p.stride[a] == 1) {   // the stride-group leader is the query itself: no division
+    st = p.causal[a] ? imax(imin(i, L - 1) - (k - 1), 0) : imin(imax(i - (k >> 1), 0), L - k);
+  } else {
+    st = win_start(i, k, p.stride[a], L, p.causal[a]);
+  }
+  en = win_end(i, st, k, L, p.causal[a]);
 }
 // Queries whose window holds key j (the inverse window): [lo, hi); empty for j outside [0, L).
 __device__ __forceinline__ void inv_window(const BwdTcParams& p, int a, int j, int L, int& lo,
                                            int& hi) {
   if (j >= L) {
     lo = hi = L;
+    return;
+  }
+  if (p.stride[a] == 1) {
+    // unit stride, start = i - k / 2 cut to [0, L - k] (causal: i - k + 1 cut at 0): solved for i
+    const int k = p.kernel[a], wl = k >> 1;
+    lo = p.causal[a] ? j : (j < k ? 0 : j - k + 1 + wl);
+    hi = p.causal[a] ? imin(j + k, L) : (j >= L - k ? L : j + 1 + wl);
     return;
   }
   int x = 0, y = L;
@@ -264,14 +280,15 @@ struct Smem {
   static constexpr int kCol2Off = kColOff + kRing1 * kStage1Bytes;   // C2 ring (kPipe only)
   static constexpr int kPrefOff = kCol2Off + (kPipe ? kStages * kTileBytes : 0);
   static constexpr int kPrefEntries = 136;
-  static constexpr int kStatOff = kPrefOff + kPrefEntries * 16;   // column stats [2][2][128] fp32
-  static constexpr int kDescOff = kStatOff + (kPipe ? 0 : 2 * 2 * kTile * 4);
+  static constexpr int kStatOff = kPrefOff + kPrefEntries * 16;   // column stats [kStatBufs][2][128] fp32
+  static constexpr int kDescOff = kStatOff + (kPipe ? 0 : kStatBufs * 2 * kTile * 4);
   static constexpr int kRecOff = kDescOff + kDescSlots * kDescBytes;
   static constexpr int kBarOff = kRecOff + kTileRecs * 16;
   // r_full, r_empty, sdp_full, sdp_free, acc_full, acc_empty, ds_full[2], ds_free[2],
   // desc_full[], desc_empty[], rec_full[8], rec_empty[8], c_full[R1], c_empty[R1], v_full[S],
-  // v_empty[S]
-  static constexpr int kNumBars = 10 + 2 * kDescSlots + 2 * kTileRecs + 2 * kRing1 + 2 * kStages;
+  // v_empty[S]; pass dKdV: stat_full[], stat_empty[]
+  static constexpr int kNumBars = 10 + 2 * kDescSlots + 2 * kTileRecs + 2 * kRing1 + 2 * kStages +
+                                  (kPipe ? 0 : 2 * kStatBufs);
   static constexpr int kMiscOff = kBarOff + kNumBars * 8;
   static constexpr int kBytes = kMiscOff + 16;
   static_assert(kBytes <= 227 * 1024, "shared memory budget of one CTA");
@@ -282,6 +299,7 @@ struct Bars {
   // pass dKdV only: these share the slots of ds_free[0] and ds_full[1], which pass dQ alone uses
   uint64_t *dp_full, *p_full;
   uint64_t *desc_full, *desc_empty, *rec_full, *rec_empty, *c_full, *c_empty, *v_full, *v_empty;
+  uint64_t *stat_full, *stat_empty;   // pass dKdV only
 };
 
 constexpr int kTileInterior = 1, kTileBoundary = 2, kTileRagged = 3;
@@ -341,7 +359,7 @@ fna_bwd_kernel(const __grid_constant__ CUtensorMap tm_r1, const __grid_constant_
   uint8_t* col_sm = smem + SM::kColOff;
   uint8_t* col2_sm = smem + SM::kCol2Off;
   uint4* pref = reinterpret_cast<uint4*>(smem + SM::kPrefOff);
-  float* colstat = reinterpret_cast<float*>(smem + SM::kStatOff);  // [2 buf][lse | delta][128]
+  float* colstat = reinterpret_cast<float*>(smem + SM::kStatOff);  // [kStatBufs][lse | delta][128]
   uint8_t* desc_sm = smem + SM::kDescOff;
   int4* tile_rec = reinterpret_cast<int4*>(smem + SM::kRecOff);
   uint64_t* bar_base = reinterpret_cast<uint64_t*>(smem + SM::kBarOff);
@@ -367,6 +385,8 @@ fna_bwd_kernel(const __grid_constant__ CUtensorMap tm_r1, const __grid_constant_
   bars.c_empty = bars.c_full + kRing1;
   bars.v_full = bars.c_empty + kRing1;
   bars.v_empty = bars.v_full + kStages;
+  bars.stat_full = bars.v_empty + kStages;
+  bars.stat_empty = bars.stat_full + kStatBufs;
 
   // read through a shuffle so that the compiler knows the value is warp-uniform: role branches
   // are then uniform, and address arithmetic inside them can use the uniform datapath
@@ -391,13 +411,18 @@ fna_bwd_kernel(const __grid_constant__ CUtensorMap tm_r1, const __grid_constant_
     ptx::mbar_init(bars.acc_empty, kSoftmaxWarps);
     for (int s = 0; s < kDescSlots; ++s) {
       ptx::mbar_init(bars.desc_full + s, 1);
-      // softmax warps + the MMA-issuing threads
-      ptx::mbar_init(bars.desc_empty + s, kSoftmaxWarps + (kPipe ? 2 : 1));
+      // softmax warps + the MMA-issuing threads (pass dKdV: + the statistics warp)
+      ptx::mbar_init(bars.desc_empty + s, kSoftmaxWarps + 2);
     }
     for (int s = 0; s < kTileRecs; ++s) {
       ptx::mbar_init(bars.rec_full + s, 1);
-      ptx::mbar_init(bars.rec_empty + s, kSoftmaxWarps);
+      ptx::mbar_init(bars.rec_empty + s, kSoftmaxWarps + (kPipe ? 0 : 1));
     }
+    if (!kPipe)
+      for (int s = 0; s < kStatBufs; ++s) {
+        ptx::mbar_init(bars.stat_full + s, 1);
+        ptx::mbar_init(bars.stat_empty + s, kSoftmaxWarps);
+      }
     for (int s = 0; s < kRing1; ++s) {
       ptx::mbar_init(bars.c_full + s, 1);
       ptx::mbar_init(bars.c_empty + s, 1);
@@ -446,16 +471,14 @@ fna_bwd_kernel(const __grid_constant__ CUtensorMap tm_r1, const __grid_constant_
     constexpr float kLog2e = 1.4426950408889634f;
     uint32_t ph_sdp = 0, ph_dp = 0, ph_acc = 0, tseq = 0, dseq = 0;
     BTRACE_DECL(4 * 40)
-    // in-tile coordinates of this thread's row, and of the column whose statistics it fetches
-    int tr[B200NA_MAX_DIM], tcol[B200NA_MAX_DIM];
+    // in-tile coordinates of this thread's row
+    int tr[B200NA_MAX_DIM];
     {
-      int rl = row, cl = row;
+      int rl = row;
 #pragma unroll
       for (int a = 0; a < B200NA_MAX_DIM; ++a) {
         tr[a] = (a < NDIM) ? rl % p.Tr[a] : 0;
         rl /= (a < NDIM) ? p.Tr[a] : 1;
-        tcol[a] = (a < NDIM) ? cl % p.Tc[a] : 0;
-        cl /= (a < NDIM) ? p.Tc[a] : 1;
       }
     }
     for (uint32_t seq = 0;; ++seq) {
@@ -508,32 +531,15 @@ fna_bwd_kernel(const __grid_constant__ CUtensorMap tm_r1, const __grid_constant_
         ++tseq;
         const bool interior = rec.x == kTileInterior;
         const int base3[B200NA_MAX_DIM] = {rec.y, rec.z, rec.w};
-        // double-buffered by a count that runs across items, so that the buffer a thread fills
-        // is never one a slower thread may still be reading
-        float* stat = colstat + (tseq & 1) * 2 * kTile;
-        if (kKeyRows) {
-          // the statistics belong to the columns (queries): 128 threads fetch one column each
-          if (part == 0) {
-            const int hq = it.h * p.rep + iter / n_per_head;
-            bool ok = true;
-            long long tok = it.b;
-#pragma unroll
-            for (int a = 0; a < B200NA_MAX_DIM; ++a) {
-              if (a < NDIM) {
-                const int i = base3[a] + tcol[a];
-                ok = ok && i < it.L[a];
-                tok = tok * p.X[a] + (i * p.dil[a] + it.g[a]);
-              }
-            }
-            if (NDIM == 1 && p.fold_d)
-              tok = (long long)it.b * p.fold_len + (long long)(base3[0] + tcol[0]) * p.fold_d +
-                    p.fold_g0 + it.g[1];
-            // a column past the extent gets -LSE = -inf, i.e. P = 0
-            // stored negated, so that the packed additions below take them as they are
-            stat[row] = ok ? -p.lse[tok * p.Hq + hq] * kLog2e : -INFINITY;
-            stat[kTile + row] = ok ? -p.delta[tok * p.Hq + hq] : 0.f;
-          }
-          named_bar_sync(1, kSoftmaxThreads);
+        // pass dKdV: the statistics belong to the columns (queries); the statistics warp has them
+        // in shared memory before the products arrive
+        const uint32_t sbuf = (tseq - 1) % kStatBufs;
+        const float* stat = colstat + sbuf * 2 * kTile;
+        if (kKeyRows &&
+            !__all_sync(0xffffffffu, wait_bar(bars.stat_full + sbuf, ((tseq - 1) / kStatBufs) & 1,
+                                              abort_flag, p.status, (5 << 8) | kStStatFull))) {
+          alive = false;
+          break;
         }
         uint32_t mw = ~0u;  // mask bits of this thread's 32 columns (boundary tiles only)
         if (rec.x == kTileRagged) {
@@ -667,7 +673,10 @@ fna_bwd_kernel(const __grid_constant__ CUtensorMap tm_r1, const __grid_constant_
           ptx::tmem_st_wait();
           ptx::tc_fence_before_sync();
           __syncwarp();
-          if (lane == 0) ptx::mbar_arrive(bars.ds_full);
+          if (lane == 0) {
+            ptx::mbar_arrive(bars.ds_full);
+            ptx::mbar_arrive(bars.stat_empty + sbuf);
+          }
           if (lane == 0 && (warp == 0 || warp == 15)) BTRACE(warp == 0 ? 2 : 3, 14);
         }
       }
@@ -931,6 +940,91 @@ fna_bwd_kernel(const __grid_constant__ CUtensorMap tm_r1, const __grid_constant_
           }
         }
       }
+    }
+  } else if (kKeyRows && warp == kStatWarp) {
+    // ============ column statistics of pass dKdV ============================================
+    // LSE and delta of a column tile's 128 queries, four per lane. Fetched by the softmax threads
+    // themselves at the head of each tile, the loads' latency and the barrier behind them stood
+    // between a tile's dS and the next tile's P: S of that tile is there by then.
+    int tcol[4][B200NA_MAX_DIM];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      int cl = q * 32 + lane;
+#pragma unroll
+      for (int a = 0; a < B200NA_MAX_DIM; ++a) {
+        tcol[q][a] = (a < NDIM) ? cl % p.Tc[a] : 0;
+        cl /= (a < NDIM) ? p.Tc[a] : 1;
+      }
+    }
+    constexpr float kLog2e = 1.4426950408889634f;
+    uint32_t tseq = 0;
+    bool alive = true;
+    for (uint32_t seq = 0; alive; ++seq) {
+      const uint32_t dslot = seq % kDescSlots;
+      if (!__all_sync(0xffffffffu, wait_bar(bars.desc_full + dslot, (seq / kDescSlots) & 1,
+                                            abort_flag, p.status, (10 << 8) | kStDescFull)))
+        break;
+      const Item& it = *reinterpret_cast<const Item*>(desc_sm + dslot * kDescBytes);
+      const int n_tiles = it.n_tiles;
+      if (n_tiles < 0) break;
+      const int n_per_head = it.n_per_head;
+      int hq = it.h * p.rep, in_head = 0;
+      for (int iter = 0; iter < n_tiles; ++iter) {
+        if (!__all_sync(0xffffffffu,
+                        wait_bar(bars.rec_full + tseq % kTileRecs, (tseq / kTileRecs) & 1,
+                                 abort_flag, p.status, (10 << 8) | kStRecFull))) {
+          alive = false;
+          break;
+        }
+        const int4 rec = tile_rec[tseq % kTileRecs];
+        __syncwarp();
+        if (lane == 0) ptx::mbar_arrive(bars.rec_empty + tseq % kTileRecs);
+        const int base3[B200NA_MAX_DIM] = {rec.y, rec.z, rec.w};
+        float l[4], d[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          bool ok = true;
+          long long tok = it.b;
+#pragma unroll
+          for (int a = 0; a < B200NA_MAX_DIM; ++a) {
+            if (a < NDIM) {
+              const int i = base3[a] + tcol[q][a];
+              ok = ok && i < it.L[a];
+              tok = tok * p.X[a] + (i * p.dil[a] + it.g[a]);
+            }
+          }
+          if (NDIM == 1 && p.fold_d)
+            tok = (long long)it.b * p.fold_len + (long long)(base3[0] + tcol[q][0]) * p.fold_d +
+                  p.fold_g0 + it.g[1];
+          // stored negated, so that the packed additions take them as they are; a column past the
+          // extent gets -LSE = -inf, i.e. P = 0
+          l[q] = ok ? -p.lse[tok * p.Hq + hq] * kLog2e : -INFINITY;
+          d[q] = ok ? -p.delta[tok * p.Hq + hq] : 0.f;
+        }
+        const uint32_t sbuf = tseq % kStatBufs;
+        if (!__all_sync(0xffffffffu,
+                        wait_bar(bars.stat_empty + sbuf, ((tseq / kStatBufs) & 1) ^ 1, abort_flag,
+                                 p.status, (10 << 8) | kStStatEmpty))) {
+          alive = false;
+          break;
+        }
+        float* stat = colstat + sbuf * 2 * kTile;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          stat[q * 32 + lane] = l[q];
+          stat[kTile + q * 32 + lane] = d[q];
+        }
+        __syncwarp();
+        if (lane == 0) ptx::mbar_arrive(bars.stat_full + sbuf);
+        ++tseq;
+        if (++in_head == n_per_head) {  // next query head of the group
+          in_head = 0;
+          ++hq;
+        }
+      }
+      if (!alive) break;
+      __syncwarp();
+      if (lane == 0) ptx::mbar_arrive(bars.desc_empty + dslot);
     }
   } else if (warp == kLoadWarp) {
     // ============ TMA loads, work-item decode, tile classification ==========================
