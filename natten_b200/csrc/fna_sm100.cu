@@ -301,9 +301,7 @@ struct Smem {
   static constexpr int kKVOff = kH * kTileBytes;
   static constexpr int kPrefOff = kKVOff + kStages * kTileBytes;
   static constexpr int kPrefEntries = 136;                  // sum(T_a + 1) <= 128 + 1 + 2 + 2
-  static constexpr int kXchgOff = kPrefOff + kPrefEntries * 16;   // row max / row sum exchange
-  static constexpr int kXchgBytes = (2 * 2 * 2 + 2 * 2) * kHalf * 4;
-  static constexpr int kDescOff = kXchgOff + kXchgBytes;          // work-item descriptor ring
+  static constexpr int kDescOff = kPrefOff + kPrefEntries * 16;   // work-item descriptor ring
   static constexpr int kRecOff = kDescOff + kDescSlots * kDescBytes;  // per-tile records
   static constexpr int kBarOff = kRecOff + kTileRecs * 16;
   // barriers: q_full, q_empty, s_full[2], p_full[2], o_full[2], o_empty[2], desc_full[4],
@@ -413,8 +411,6 @@ fna_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
   uint8_t* q_sm = smem + SM::kQOff;
   uint8_t* kv_sm = smem + SM::kKVOff;
   uint4* pref = reinterpret_cast<uint4*>(smem + SM::kPrefOff);
-  float* xmax = reinterpret_cast<float*>(smem + SM::kXchgOff);        // [2 parity][2 half][2 part][128]
-  float* xsum = xmax + 2 * 2 * 2 * kHalf;                             // [2 half][2 part][128]
   uint8_t* desc_sm = smem + SM::kDescOff;
   int4* tile_rec = reinterpret_cast<int4*>(smem + SM::kRecOff);
   uint64_t* bar_base = reinterpret_cast<uint64_t*>(smem + SM::kBarOff);
@@ -494,19 +490,18 @@ fna_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
 
   if (warp < kSoftmaxWarps) {
     // ======================= softmax + correction + epilogue ===============================
-    // Two threads share a query row: `part` 0 owns key columns [0, 64) of every tile and output
-    // columns [0, D/2), `part` 1 the other halves. A lone warp cannot keep a sub-partition's
-    // issue slots busy, so halving the per-thread work halves the softmax latency that sits
-    // between the two MMAs of a half.
+    // Two threads of one warp share a query row: `part` 0 (lanes 0-15) owns key columns [0, 64) of
+    // every tile and output columns [0, D/2), `part` 1 (lanes 16-31) the other halves; a warp owns
+    // 16 rows. What is decided per row (the running maximum, whether it has to move) is then
+    // decided inside the warp: no barrier between warps stands on the way from the logits to P.
     const int half = warp >> 3;
-    const int part = (warp >> 2) & 1;
-    const int row = ((warp & 3) << 5) | lane;          // row inside the half = TMEM lane
-    const uint32_t lane_addr = tmem_base + ((uint32_t)((warp & 3) << 5) << 16);
-    const uint32_t s_addr = lane_addr + s_col(half);
-    const uint32_t my_s = s_addr + part * 64;                 // my 64 fp32 logit columns
-    const uint32_t my_p = s_addr + part * 64;                 // my 32 packed P columns (in place)
-    const uint32_t my_o = lane_addr + o_col(half) + part * (D / 2);
-    const int bar_id = 1 + half;
+    const int part = lane >> 4;
+    const int row0 = ((warp & 3) << 5) | ((warp & 4) << 2);   // first row of the warp in the half
+    const int row = row0 | (lane & 15);                // row inside the half = TMEM lane
+    const uint32_t lane_addr = tmem_base + ((uint32_t)row0 << 16);
+    const uint32_t s_addr = lane_addr + s_col(half);   // 64 fp32 logit columns per part; 32 packed
+                                                       // P columns overwrite them in place
+    const uint32_t o_addr = lane_addr + o_col(half);
     const float c = p.scale_log2;
     uint32_t ph_s = 0, ph_o = 0;
     uint32_t tseq = 0;  // tiles consumed so far, indexes the per-tile record ring
@@ -595,108 +590,118 @@ fna_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         PROF_MARK(0)
         if (row == 0 && part == 0) TRACE(half, 1)
         ptx::tc_fence_after_sync();
-        // Pass 1: row maximum of the raw logits over this thread's 64 columns. Chunk 1 is read
-        // first and dropped, chunk 0 stays in registers for pass 2.
         uint32_t sr[32];
-        float mx0 = -INFINITY, mx1 = -INFINITY, mx2 = -INFINITY, mx3 = -INFINITY;
-        ptx::tmem_ld32(my_s + 32, sr);
-        ptx::tmem_ld_wait();
-        if (!interior) {
+        // packed P of 32 columns: two (16-bit operands) or four probabilities (e4m3) per word
+        constexpr int kPkWords = kF8 ? 8 : 16;
+        auto load_chunk = [&](int ch) {
+          ptx::tmem_ld32_x2<64>(s_addr + ch * 32, sr);
+          ptx::tmem_ld_wait();
+          if (!interior) {
+            const uint32_t mw = ch ? mw1 : mw0;
 #pragma unroll
-          for (int j = 0; j < 32; ++j)
-            if (!((mw1 >> j) & 1u)) sr[j] = 0xff800000u;  // -inf
-        }
-#pragma unroll
-        for (int j = 0; j < 32; j += 4) {
-          mx0 = ptx::max3(mx0, __uint_as_float(sr[j]), __uint_as_float(sr[j + 1]));
-          mx1 = ptx::max3(mx1, __uint_as_float(sr[j + 2]), __uint_as_float(sr[j + 3]));
-        }
-        ptx::tmem_ld32(my_s, sr);
-        ptx::tmem_ld_wait();
-        PROF_MARK(1)
-        if (!interior) {
-#pragma unroll
-          for (int j = 0; j < 32; ++j)
-            if (!((mw0 >> j) & 1u)) sr[j] = 0xff800000u;
-        }
-#pragma unroll
-        for (int j = 0; j < 32; j += 4) {
-          mx2 = ptx::max3(mx2, __uint_as_float(sr[j]), __uint_as_float(sr[j + 1]));
-          mx3 = ptx::max3(mx3, __uint_as_float(sr[j + 2]), __uint_as_float(sr[j + 3]));
-        }
-        const float my_max = fmaxf(fmaxf(mx0, mx1), fmaxf(mx2, mx3));
-        float* xm = xmax + (((iter & 1) * 2 + half) * 2) * kHalf;
-        xm[part * kHalf + row] = my_max;
-        named_bar_sync(bar_id, kSoftmaxThreadsPerHalf);
-        const float m_new = ptx::max3(m, my_max, xm[(part ^ 1) * kHalf + row]);
-        // Lazy rescale: keep the stale maximum while the true one is at most 2^8 larger.
-        const bool grow = (m_new - m) * c > kRescaleThreshold;  // NaN (-inf - -inf) -> false
-        if (__any_sync(0xffffffffu, grow)) {
-          const float f = grow ? ptx::ex2((m - m_new) * c) : 1.f;
-          if (grow) {
-            sum *= f;
-            m = m_new;
+            for (int j = 0; j < 32; ++j)
+              if (!((mw >> j) & 1u)) sr[j] = 0xff800000u;  // -inf
           }
-          if (iter > 0) {
-            // O_half is quiescent here: P.V of the previous tile completed before s_full fired.
+        };
+        auto chunk_max = [&](float& mx0, float& mx1) {
 #pragma unroll
-            for (int ch = 0; ch < D / 32; ++ch) {
-              uint32_t orr[16];
-              ptx::tmem_ld16(my_o + ch * 16, orr);
-              ptx::tmem_ld_wait();
-#pragma unroll
-              for (int j = 0; j < 16; ++j) orr[j] = __float_as_uint(__uint_as_float(orr[j]) * f);
-              ptx::tmem_st16(my_o + ch * 16, orr);
-            }
+          for (int j = 0; j < 32; j += 4) {
+            mx0 = ptx::max3(mx0, __uint_as_float(sr[j]), __uint_as_float(sr[j + 1]));
+            mx1 = ptx::max3(mx1, __uint_as_float(sr[j + 2]), __uint_as_float(sr[j + 3]));
           }
-        }
-        const float neg_mc = (m == -INFINITY) ? 0.f : -m * c;
-        // Pass 2: p = 2^(s*c - m*c), 32 columns at a time; each packed chunk of P overwrites
-        // logit columns this same thread has already consumed, so no other thread is involved.
-        // x = s c - m c and the row sums in packed (two-wide) arithmetic: half the instructions
-        // of the scalar forms for these two steps
-        const uint64_t c2 = ptx::f32x2(c, c), nmc2 = ptx::f32x2(neg_mc, neg_mc);
+        };
+        // p = 2^(s c - m c) of the loaded chunk; scale-and-subtract and row sums in packed
+        // (two-wide) arithmetic: half the instructions of the scalar forms
+        const uint64_t c2 = ptx::f32x2(c, c);
         uint64_t acc0 = ptx::f32x2(0.f, 0.f), acc1 = acc0;
+        auto chunk_exp = [&](uint64_t nmc2, uint32_t (&pk)[kPkWords]) {
 #pragma unroll
-        for (int ch = 0; ch < 2; ++ch) {
-          if (ch == 1) {
-            ptx::tmem_ld32(my_s + 32, sr);
-            ptx::tmem_ld_wait();
-            if (!interior) {
-#pragma unroll
-              for (int j = 0; j < 32; ++j)
-                if (!((mw1 >> j) & 1u)) sr[j] = 0xff800000u;
-            }
-          }
-          if (kF8) {
-            // 8-bit operands: P is rounded to e4m3, four probabilities per TMEM column
-            uint32_t pk[8];
-#pragma unroll
-            for (int j = 0; j < 32; j += 4) {
-              float x0, x1, x2, x3;
-              ptx::f32x2_split(ptx::fma_f32x2(ptx::f32x2(sr[j], sr[j + 1]), c2, nmc2), x0, x1);
-              ptx::f32x2_split(ptx::fma_f32x2(ptx::f32x2(sr[j + 2], sr[j + 3]), c2, nmc2), x2, x3);
-              const float p0 = ptx::ex2(x0), p1 = ptx::ex2(x1), p2 = ptx::ex2(x2), p3 = ptx::ex2(x3);
-              acc0 = ptx::add_f32x2(acc0, ptx::f32x2(p0, p1));
-              acc1 = ptx::add_f32x2(acc1, ptx::f32x2(p2, p3));
+          for (int j = 0; j < 32; j += 4) {
+            float x0, x1, x2, x3;
+            ptx::f32x2_split(ptx::fma_f32x2(ptx::f32x2(sr[j], sr[j + 1]), c2, nmc2), x0, x1);
+            ptx::f32x2_split(ptx::fma_f32x2(ptx::f32x2(sr[j + 2], sr[j + 3]), c2, nmc2), x2, x3);
+            const float p0 = ptx::ex2(x0), p1 = ptx::ex2(x1), p2 = ptx::ex2(x2), p3 = ptx::ex2(x3);
+            acc0 = ptx::add_f32x2(acc0, ptx::f32x2(p0, p1));
+            acc1 = ptx::add_f32x2(acc1, ptx::f32x2(p2, p3));
+            if constexpr (kF8) {
               pk[j >> 2] = ptx::pack4_e4m3(p0, p1, p2, p3);
-            }
-            ptx::tmem_st8(my_p + ch * 8, pk);
-          } else {
-            uint32_t pk[16];
-#pragma unroll
-            for (int j = 0; j < 32; j += 4) {
-              float x0, x1, x2, x3;
-              ptx::f32x2_split(ptx::fma_f32x2(ptx::f32x2(sr[j], sr[j + 1]), c2, nmc2), x0, x1);
-              ptx::f32x2_split(ptx::fma_f32x2(ptx::f32x2(sr[j + 2], sr[j + 3]), c2, nmc2), x2, x3);
-              const float p0 = ptx::ex2(x0), p1 = ptx::ex2(x1), p2 = ptx::ex2(x2), p3 = ptx::ex2(x3);
-              acc0 = ptx::add_f32x2(acc0, ptx::f32x2(p0, p1));
-              acc1 = ptx::add_f32x2(acc1, ptx::f32x2(p2, p3));
+            } else {
               pk[j >> 1] = pack2<kType>(p0, p1);
               pk[(j >> 1) + 1] = pack2<kType>(p2, p3);
             }
-            ptx::tmem_st16(my_p + ch * 16, pk);
           }
+        };
+        auto store_chunk = [&](int ch, const uint32_t (&pk)[kPkWords]) {
+          if constexpr (kF8) ptx::tmem_st8_x2<64>(s_addr + ch * kPkWords, pk);
+          else ptx::tmem_st16_x2<64>(s_addr + ch * kPkWords, pk);
+        };
+        // The running maximum is lazy: it stays while the true one is at most 2^8 larger. After an
+        // item's first tile that is nearly always so, hence P is computed with the maximum at hand
+        // in one pass over the logits, and kept only if no row of the warp has outgrown it (P is
+        // stored after that is known: the logits it overwrites are still there to start again).
+        // A row without keys so far (its window starts in a later tile) has no maximum yet. In the
+        // one-half shape a boundary tile's masks and the packed P together spill: 128 x 128, 13 x 13
+        // windows, dilation 2 took 1052 us in one pass everywhere, 935 us this way.
+        // 15 x 44 x 80 video in 8 bits: 2051 -> 1859 us; long causal sequences: the same time (the
+        // softmax gets 5 % shorter, the wait for the next logits longer).
+        bool again = iter == 0 || (kH == 1 && !interior) || __any_sync(0xffffffffu, m == -INFINITY);
+        if (!again) {
+          const float neg_mc = -m * c;
+          const uint64_t nmc2 = ptx::f32x2(neg_mc, neg_mc);
+          float mx0 = -INFINITY, mx1 = -INFINITY;
+          uint32_t pk0[kPkWords], pk1[kPkWords];
+          load_chunk(0);
+          chunk_max(mx0, mx1);
+          chunk_exp(nmc2, pk0);
+          load_chunk(1);
+          PROF_MARK(1)
+          chunk_max(mx0, mx1);
+          again = __any_sync(0xffffffffu, (fmaxf(mx0, mx1) - m) * c > kRescaleThreshold);
+          if (!again) {
+            chunk_exp(nmc2, pk1);
+            store_chunk(0, pk0);
+            store_chunk(1, pk1);
+          }
+        }
+        if (again) {
+          // Row maxima first (chunk 1 is read and dropped, chunk 0 stays in registers), then P; the
+          // accumulated row sums and output rows are rescaled where the maximum moves.
+          float mx0 = -INFINITY, mx1 = -INFINITY;
+          load_chunk(1);
+          chunk_max(mx0, mx1);
+          load_chunk(0);
+          chunk_max(mx0, mx1);
+          const float my_max = fmaxf(mx0, mx1);
+          const float m_new = ptx::max3(m, my_max, __shfl_xor_sync(0xffffffffu, my_max, 16));
+          const bool grow = (m_new - m) * c > kRescaleThreshold;  // NaN (-inf - -inf) -> false
+          if (__any_sync(0xffffffffu, grow)) {
+            const float f = grow ? ptx::ex2((m - m_new) * c) : 1.f;
+            if (grow) {
+              sum *= f;
+              m = m_new;
+            }
+            if (iter > 0) {
+              // O_half is quiescent here: P.V of the previous tile completed before s_full fired.
+#pragma unroll
+              for (int ch = 0; ch < D / 32; ++ch) {
+                uint32_t orr[16];
+                ptx::tmem_ld16_x2<D / 2>(o_addr + ch * 16, orr);
+                ptx::tmem_ld_wait();
+#pragma unroll
+                for (int j = 0; j < 16; ++j) orr[j] = __float_as_uint(__uint_as_float(orr[j]) * f);
+                ptx::tmem_st16_x2<D / 2>(o_addr + ch * 16, orr);
+              }
+            }
+          }
+          const float neg_mc = (m == -INFINITY) ? 0.f : -m * c;
+          const uint64_t nmc2 = ptx::f32x2(neg_mc, neg_mc);
+          acc0 = acc1 = ptx::f32x2(0.f, 0.f);
+          uint32_t pk[kPkWords];
+          chunk_exp(nmc2, pk);
+          store_chunk(0, pk);
+          load_chunk(1);
+          chunk_exp(nmc2, pk);
+          store_chunk(1, pk);
         }
         {
           float s0, s1, s2, s3;
@@ -721,10 +726,7 @@ fna_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
       // ---- epilogue: O / sum -> global, LSE ----
       // Everything that does not need the accumulator comes before the wait for the last P.V:
       // the row sums are final once the last tile's exponentials are.
-      float* xs = xsum + half * 2 * kHalf;
-      xs[part * kHalf + row] = sum;
-      named_bar_sync(bar_id, kSoftmaxThreadsPerHalf);
-      const float total = sum + xs[(part ^ 1) * kHalf + row];
+      const float total = sum + __shfl_xor_sync(0xffffffffu, sum, 16);
       // Row of O / LSE this thread writes: a row of the permuted [B', S, H, D] operand, or - in
       // direct mode - the token of the caller's [B, *X, H, D] layout the query row stands for.
       long long out_row;
@@ -756,47 +758,51 @@ fna_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
       PROF_MARK(4)
       ptx::tc_fence_after_sync();
       // This thread's share of its output row: D/2 elements = kChunks 16-byte chunks. A store of
-      // one chunk per lane would touch 32 rows (32 separate lines) per instruction, and the
+      // one chunk per lane would touch 16 rows (32 separate lines) per instruction, and the
       // load/store unit would spend more time on the epilogue than the arithmetic does. The
       // chunks go through a 1 KB warp-private staging buffer instead, kRowsPerRound rows at a
       // time, and come back out with consecutive lanes holding consecutive chunks of one row:
       // every store instruction then writes whole rows.
       constexpr int kChunks = (D / 2) * kES / 16;       // 8 (128 bytes) or 4 (64 bytes)
-      constexpr int kRowsPerRound = 64 / kChunks;       // rows whose chunks fill the 1 KB buffer
+      constexpr int kRowChunks = 2 * kChunks;
+      constexpr int kRowsPerRound = 64 / kRowChunks;    // rows whose chunks fill the 1 KB buffer
       constexpr int kPer = 16 / kES;                    // output elements per chunk
       uint4 pk[kChunks];
 #pragma unroll
       for (int ch = 0; ch < D / 64; ++ch) {
         uint32_t orr[32];
-        ptx::tmem_ld32(my_o + ch * 32, orr);
+        ptx::tmem_ld32_x2<D / 2>(o_addr + ch * 32, orr);
         ptx::tmem_ld_wait();
 #pragma unroll
         for (int v4 = 0; v4 < 32 / kPer; ++v4)
           pk[ch * (32 / kPer) + v4] = pack_out16<kType>(orr + v4 * kPer, inv);
       }
       // rows of the output tensor are d_real elements wide; chunks past that are not stored
-      uint8_t* const orow = valid ? o_ptr + (out_row * p.d_real + part * (D / 2)) * kES : nullptr;
-      const int my_chunks = imin(imax((p.d_real - part * (D / 2)) / kPer, 0), kChunks);
+      uint8_t* const orow = valid ? o_ptr + out_row * p.d_real * kES : nullptr;
+      const int row_chunks = p.d_real / kPer;
       uint4* const stage = reinterpret_cast<uint4*>(smem + SM::kStageOff + warp * SM::kStageBytes);
+      // XOR placement inside a part's chunks of a row: conflict-free both ways
+      auto place = [](int lr, int pt) { return kChunks == 8 ? lr * 2 + pt : lr & 3; };
 #pragma unroll
-      for (int rd = 0; rd < 32 / kRowsPerRound; ++rd) {
+      for (int rd = 0; rd < 16 / kRowsPerRound; ++rd) {
         __syncwarp();
-        if (lane / kRowsPerRound == rd) {
+        if ((lane & 15) / kRowsPerRound == rd) {
           const int lr = lane % kRowsPerRound;
 #pragma unroll
-          for (int cidx = 0; cidx < kChunks; ++cidx)  // XOR placement: conflict-free both ways
-            stage[lr * kChunks + (cidx ^ (lr % kChunks))] = pk[cidx];
+          for (int cidx = 0; cidx < kChunks; ++cidx)
+            stage[lr * kRowChunks + part * kChunks + (cidx ^ place(lr, part))] = pk[cidx];
         }
         __syncwarp();
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
           const int idx = i * 32 + lane;
-          const int lr = idx / kChunks, cidx = (idx % kChunks) ^ (lr % kChunks);
+          const int lr = idx / kRowChunks, pt = (idx / kChunks) & 1;
+          const int cidx = pt * kChunks + ((idx % kChunks) ^ place(lr, pt));
           const uint4 val = stage[idx];
-          // the row's address lives in the lane that owns the row (null: padding row)
+          // the row's address lives in the lanes that own the row (null: padding row)
           const unsigned long long rp = __shfl_sync(
               0xffffffffu, (unsigned long long)(uintptr_t)orow, rd * kRowsPerRound + lr);
-          if (rp != 0ull && cidx < my_chunks)
+          if (rp != 0ull && cidx < row_chunks)
             *reinterpret_cast<uint4*>((uint8_t*)(uintptr_t)rp + cidx * 16) = val;
         }
       }
