@@ -184,6 +184,8 @@ B200NA_API int b200na_na_forward_direct_strided(
  * as (position in group, group), two axes of the tensor map, so that a tile is 128 positions of one
  * group whatever the dilation. Two launches instead of one when the dilation (> 1) does not divide
  * the length: the groups then have two different lengths.
+ * Tiles may hold fewer tokens: prod(q_tile) up to 256 (above 128 its last non-unit extent is even),
+ * prod(kv_tile) up to 128 (exactly 128 with extra tokens).
  */
 B200NA_API int b200na_na_forward_view(
     const void* q, const void* k, const void* v, const void* add_k, const void* add_v,
@@ -371,7 +373,8 @@ B200NA_API int b200na_na_backward_direct(
  *   - D any multiple of 8 up to 128 (below 64 / 128 the tensor maps return zeros for the missing
  *     channels; a 3-D layout then needs B == 1, otherwise B200NA_ERR_UNSUPPORTED);
  *   - any 1-D dilation (see b200na_na_forward_view; two launches per pass when it does not divide
- *     the length).
+ *     the length);
+ *   - tiles of up to 128 tokens (kv_tile: exactly 128 with extra tokens).
  */
 B200NA_API int b200na_na_backward_view(
     const void* q, const void* k, const void* v, const void* o, const void* d_out, const float* lse,

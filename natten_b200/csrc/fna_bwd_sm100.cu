@@ -51,7 +51,6 @@ namespace {
 constexpr int kTile = 128;          // tokens per row tile and per column tile
 constexpr int kParts = 4;           // threads per row: each owns 32 of a column tile's 128 columns
 constexpr int kSoftmaxWarps = 16;   // 4 column parts x 4 warps (one thread per row and part)
-constexpr int kSoftmaxThreads = 512;
 constexpr int kMmaWarp = 16;
 constexpr int kLoadWarp = 17;
 constexpr int kMma2Warp = 18;       // pass dQ: issues the dQ products (kMmaWarp issues S and dP)
@@ -96,6 +95,7 @@ struct BwdTcParams {
   int n_rtiles;             // row tiles per (batch, group, head)
   int row_heads;            // heads the row tiles carry: Hq (pass dQ) or Hkv (pass dKdV)
   long long total_work;     // n_rtiles * row_heads * B * G
+  int r_rows, c_rows;       // tokens of a row tile and of a column tile (at most 128)
   int d_real;               // head dim of the tensors (<= the kernel's D; the rest reads as zeros)
   int sep_heads;            // tensor maps list the head as an axis of its own (d_real < D)
   int fold_d, fold_g0, fold_len;   // > 0: dilated 1-D layout as (position in group, group), X[0] =
@@ -433,6 +433,10 @@ fna_bwd_kernel(const __grid_constant__ CUtensorMap tm_r1, const __grid_constant_
     }
     ptx::fence_barrier_init();
   }
+  if (p.r_rows < kTile) zero_tail_rows(row_sm, 2, kDBlocks, p.r_rows, kThreads);
+  if (p.c_rows < kTile)   // the column rings lie one behind the other
+    zero_tail_rows(col_sm, kPipe ? kRing1 + kStages : 2 * kStages, kDBlocks, p.c_rows, kThreads);
+  ptx::fence_proxy_async();
   // per-axis prefix bit tables over the COLUMN tile, for the masks of boundary tiles
   build_prefix_tables(pref, p.ndim, p.Tc, warp, lane, kThreads / 32);
   if (warp == kMmaWarp) {
@@ -474,7 +478,7 @@ fna_bwd_kernel(const __grid_constant__ CUtensorMap tm_r1, const __grid_constant_
     // in-tile coordinates of this thread's row
     int tr[B200NA_MAX_DIM];
     {
-      int rl = row;
+      int rl = imin(row, p.r_rows - 1);
 #pragma unroll
       for (int a = 0; a < B200NA_MAX_DIM; ++a) {
         tr[a] = (a < NDIM) ? rl % p.Tr[a] : 0;
@@ -489,10 +493,9 @@ fna_bwd_kernel(const __grid_constant__ CUtensorMap tm_r1, const __grid_constant_
       const Item& it = *reinterpret_cast<const Item*>(desc_sm + dslot * kDescBytes);
       const int n_tiles = it.n_tiles;
       if (n_tiles < 0) break;
-      const int n_per_head = it.n_per_head;
       // span of columns this thread's row interacts with, per axis; token index of the row
       int lo_a[B200NA_MAX_DIM], hi_a[B200NA_MAX_DIM];
-      bool row_valid = true;
+      bool row_valid = row < p.r_rows;
       long long row_tok = it.b;
 #pragma unroll
       for (int a = 0; a < B200NA_MAX_DIM; ++a) {
@@ -543,7 +546,7 @@ fna_bwd_kernel(const __grid_constant__ CUtensorMap tm_r1, const __grid_constant_
         }
         uint32_t mw = ~0u;  // mask bits of this thread's 32 columns (boundary tiles only)
         if (rec.x == kTileRagged) {
-          // last tile of the extra tokens: rec.y of its columns exist
+          // the first rec.y columns exist: last tile of the extra tokens, tile of fewer keys
           const int vcols = imin(imax(rec.y - part * 32, 0), 32);
           mw = vcols >= 32 ? ~0u : ((1u << vcols) - 1u);
         } else if (!interior) {
@@ -983,7 +986,7 @@ fna_bwd_kernel(const __grid_constant__ CUtensorMap tm_r1, const __grid_constant_
         float l[4], d[4];
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-          bool ok = true;
+          bool ok = q * 32 + lane < p.c_rows;
           long long tok = it.b;
 #pragma unroll
           for (int a = 0; a < B200NA_MAX_DIM; ++a) {
@@ -1075,7 +1078,7 @@ fna_bwd_kernel(const __grid_constant__ CUtensorMap tm_r1, const __grid_constant_
         // the stationary row tiles: R1, R2 of head it.h
         if (!wait_bar(bars.r_empty, ph_re, abort_flag, p.status, (7 << 8) | kStREmpty)) break;
         ph_re ^= 1;
-        ptx::mbar_arrive_expect_tx(bars.r_full, 2 * kTileBytes);
+        ptx::mbar_arrive_expect_tx(bars.r_full, 2 * p.r_rows * (D * 2));
         {
           const int x0 = it.r_lo[0] * p.dil[0] + g0, x1 = it.r_lo[1] * p.dil[1] + g1,
                     x2 = it.r_lo[2] * p.dil[2] + g2;
@@ -1107,8 +1110,13 @@ fna_bwd_kernel(const __grid_constant__ CUtensorMap tm_r1, const __grid_constant_
             const int k0 = tw.org[0] + tc[0] * p.Tc[0],
                       k1 = NDIM > 1 ? tw.org[1] + tc[1] * p.Tc[1] : 0,
                       k2 = NDIM > 2 ? tw.org[2] + tc[2] * p.Tc[2] : 0;
-            rec = make_int4(tw.template interior<NDIM>(tc) ? kTileInterior : kTileBoundary, k0, k1,
-                            k2);
+            rec = make_int4(kTileBoundary, k0, k1, k2);
+            if (tw.template interior<NDIM>(tc)) {
+              rec.x = kTileInterior;
+              // a tile of fewer keys: only its columns exist (pass dKdV: columns that do not exist
+              // have P = 0 by their statistics)
+              if (!kKeyRows && p.c_rows < kTile) rec = make_int4(kTileRagged, p.c_rows, 0, 0);
+            }
             x0 = k0 * p.dil[0] + g0; x1 = k1 * p.dil[1] + g1; x2 = k2 * p.dil[2] + g2;
             tw.template next<NDIM>(tc);
           }
@@ -1124,7 +1132,8 @@ fna_bwd_kernel(const __grid_constant__ CUtensorMap tm_r1, const __grid_constant_
               alive = false; break;
             }
             BTRACE(1, 6);
-            ptx::mbar_arrive_expect_tx(bars.v_full + slot2, kTileBytes);
+            const int bytes = is_extra ? kTileBytes : p.c_rows * (D * 2);
+            ptx::mbar_arrive_expect_tx(bars.v_full + slot2, bytes);
             for (int db = 0; db < kDBlocks; ++db)
               load_tile(col2_sm + slot2 * kTileBytes + db * kBlockBytes,
                         is_extra ? &tm_e2 : &tm_c2, bars.v_full + slot2, col_head, db, x0, x1, x2, b,
@@ -1138,7 +1147,7 @@ fna_bwd_kernel(const __grid_constant__ CUtensorMap tm_r1, const __grid_constant_
               alive = false; break;
             }
             BTRACE(1, 7);
-            ptx::mbar_arrive_expect_tx(bars.c_full + slot, kTileBytes);
+            ptx::mbar_arrive_expect_tx(bars.c_full + slot, bytes);
             for (int db = 0; db < kDBlocks; ++db)
               load_tile(col_sm + slot * kTileBytes + db * kBlockBytes,
                         is_extra ? &tm_e1 : &tm_c1, bars.c_full + slot, col_head, db, x0, x1, x2, b,
@@ -1148,7 +1157,7 @@ fna_bwd_kernel(const __grid_constant__ CUtensorMap tm_r1, const __grid_constant_
                           (7 << 8) | kStCEmpty)) {
               alive = false; break;
             }
-            ptx::mbar_arrive_expect_tx(bars.c_full + slot, 2 * kTileBytes);
+            ptx::mbar_arrive_expect_tx(bars.c_full + slot, 2 * p.c_rows * (D * 2));
             uint8_t* dst = col_sm + slot * 2 * kTileBytes;
             for (int db = 0; db < kDBlocks; ++db) {
               load_tile(dst + db * kBlockBytes, &tm_c1, bars.c_full + slot, col_head, db, x0, x1, x2,
@@ -1327,7 +1336,10 @@ int backward_impl(const BwdCall& c, int ndim, const int* shape, const int* kerne
     nq *= tq[a];
     nkv *= tkv[a];
   }
-  if (nq != kTile || nkv != kTile) return B200NA_ERR_INVALID_ARGUMENT;
+  if (nq < 1 || nq > kTile || nkv < 1 || nkv > kTile) return B200NA_ERR_INVALID_ARGUMENT;
+  if (!c.views && (nq != kTile || nkv != kTile)) return B200NA_ERR_INVALID_ARGUMENT;
+  // the extra tokens' 128-row tiles go through the key/value ring
+  if (n_extra > 0 && nkv != kTile) return B200NA_ERR_INVALID_ARGUMENT;
   if (tokens * B > 0x7fffffffLL || (long long)Hq * D > 0x7fffffffLL) return B200NA_ERR_UNSUPPORTED;
   base.B = B; base.Hq = Hq; base.Hkv = Hkv; base.rep = Hq / Hkv;
   base.d_real = D;
@@ -1397,6 +1409,8 @@ int backward_impl(const BwdCall& c, int ndim, const int* shape, const int* kerne
       }
       if (n_rtiles > 0x7fffffffLL) return B200NA_ERR_UNSUPPORTED;
       p.n_rtiles = (int)n_rtiles;
+      p.r_rows = (int)(key_rows ? nkv : nq);
+      p.c_rows = (int)(key_rows ? nq : nkv);
       p.row_heads = key_rows ? Hkv : Hq;
       p.total_work = n_rtiles * p.row_heads * B * p.G;
       p.out0 = key_rows ? c.dk : c.dq;
@@ -1419,6 +1433,7 @@ int backward_impl(const BwdCall& c, int ndim, const int* shape, const int* kerne
   p.ndim = 1;
   p.G = 1;
   p.dense_rows = 1;
+  p.r_rows = p.c_rows = kTile;
   p.row_extent = n_extra;
   for (int a = 0; a < B200NA_MAX_DIM; ++a) {
     p.X[a] = a == 0 ? (int)tokens : 1;

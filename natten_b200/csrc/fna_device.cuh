@@ -79,7 +79,8 @@ __device__ __forceinline__ uint4 pack_out16(const uint32_t* f, float mul) {
 
 // Per-axis prefix bit tables over a 128-token tile of shape T (tokens ordered axis 0 fastest):
 // pref[off_a + x], off_a = sum_{b<a} (T[b] + 1), has bit j set iff the in-tile coordinate of
-// token j along axis a is < x. Filled by the whole warps of the block; 136 entries suffice.
+// token j along axis a is < x. Tokens past a tile of fewer than 128 have a coordinate beyond its
+// last axis: they are in no mask. Filled by the whole warps of the block; 136 entries suffice.
 // A lane is a token: its coordinate is worked out once and a ballot gives a word of the table. (With a
 // thread per entry and a loop over its 128 tokens, two divisions each, this was 25 us of every
 // launch - most of the time of a kernel with one work item per CTA.)
@@ -92,7 +93,8 @@ __device__ __forceinline__ void build_prefix_tables(uint4* pref, int ndim,
     // n_warps / 4 warps share a word column wd and take its entries in turn
     const int wd = warp & 3, step = n_warps >> 2;
     if (warp < step * 4) {
-      const int c = ((wd * 32 + lane) / below) % T[a];
+      int c = (wd * 32 + lane) / below;
+      if (a + 1 < ndim) c %= T[a];
       for (int x = warp >> 2; x <= T[a]; x += step) {
         const uint32_t bits = __ballot_sync(0xffffffffu, c < x);
         if (lane == 0) words[(off + x) * 4 + wd] = bits;
@@ -100,6 +102,19 @@ __device__ __forceinline__ void build_prefix_tables(uint4* pref, int ndim,
     }
     off += T[a] + 1;
     below *= T[a];
+  }
+}
+
+// Rows [rows, 128) of `n` 128-row shared-memory tiles (each `blocks` 128-byte column blocks wide) set
+// to zero: a tensor-map box of fewer rows never writes them, and a product would otherwise meet
+// whatever the memory held (0 * NaN). Once per launch, by all threads, before the block's barrier.
+__device__ __forceinline__ void zero_tail_rows(uint8_t* tiles, int n, int blocks, int rows,
+                                               int n_threads) {
+  const int per_block = (128 - rows) * 8;   // 16-byte pieces
+  for (int i = threadIdx.x; i < n * blocks * per_block; i += n_threads) {
+    const int blk = i / per_block;
+    *reinterpret_cast<uint4*>(tiles + (size_t)blk * 128 * 128 + rows * 128 + (i - blk * per_block) * 16) =
+        make_uint4(0u, 0u, 0u, 0u);
   }
 }
 

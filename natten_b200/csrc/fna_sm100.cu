@@ -103,6 +103,8 @@ struct FnaParams {
   int extra_tiles;          // ceil(n_extra / 128): KV tiles appended to every item's walk
   int Bp, Hq, Hkv;
   int halves;               // 128-row halves of a query tile: 2 (256-token tile) or 1 (128)
+  int q_rows;               // tokens of half a query tile and of a key/value tile: 128, fewer where
+  int kv_rows;              // no 128 of a shape fit the layout and its windows as well
   int d_real;               // head dim of the tensors (<= the kernel's D; the rest reads as zeros)
   int sep_heads;            // direct: tensor maps list the head as an axis of its own (d_real < D)
   int Sq, Skv;              // rows per batch' in the q / kv tensors
@@ -464,6 +466,9 @@ fna_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
     }
     ptx::fence_barrier_init();
   }
+  if (p.q_rows < kHalf) zero_tail_rows(q_sm, kH, kDBlocks, p.q_rows, kThreads);
+  if (p.kv_rows < kKVTile) zero_tail_rows(kv_sm, kStages, kDBlocks, p.kv_rows, kThreads);
+  ptx::fence_proxy_async();
   // per-axis prefix bit tables over the key/value tile, for the masks of boundary tiles
   build_prefix_tables(pref, p.ndim, p.Tkv, warp, lane, kThreads / 32);
   if (warp == kMmaWarp) {
@@ -509,7 +514,7 @@ fna_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
     // in-tile coordinates of this thread's query row (fixed for the whole kernel)
     int tq[B200NA_MAX_DIM];
     {
-      int rl = half * kHalf + row;
+      int rl = half * p.q_rows + imin(row, p.q_rows - 1);   // rows past the tile: its last one again
 #pragma unroll
       for (int a = 0; a < B200NA_MAX_DIM; ++a) {
         tq[a] = (a < NDIM) ? rl % p.Tq[a] : 0;
@@ -548,8 +553,8 @@ fna_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
       bool alive = true;
       for (int iter = 0; iter < n_tiles; ++iter) {
         // The load warp classified the tile when it fetched it: x = 0 nothing to mask, 1 window
-        // boundary (y, z, w = first key coordinate of the tile per axis), 2 ragged last tile of
-        // the extra tokens (y = valid columns). The record is there long before the logits are,
+        // boundary (y, z, w = first key coordinate of the tile per axis), 2 the first y columns
+        // (ragged last tile of the extra tokens; a tile of fewer than 128 keys inside the window). The record is there long before the logits are,
         // so the masks are ready when the wait for the logits ends.
         if (!__all_sync(0xffffffffu,
                         wait_bar(bars.rec_full + tseq % kTileRecs, (tseq / kTileRecs) & 1,
@@ -733,7 +738,7 @@ fna_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
       bool valid;
       if (p.direct) {
         long long tok = it.b;
-        valid = true;
+        valid = row < p.q_rows;
 #pragma unroll
         for (int a = 0; a < B200NA_MAX_DIM; ++a) {
           if (a < NDIM) {
@@ -1012,7 +1017,7 @@ fna_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         const int n_tiles = it.n_tiles, n_na = it.n_na, bp = it.bp, hk = it.hk;
         if (!wait_bar(bars.q_empty, ph_qe, abort_flag, p.status, (3 << 8) | kStQEmpty)) break;
         ph_qe ^= 1;
-        ptx::mbar_arrive_expect_tx(bars.q_full, kH * kTileBytes);
+        ptx::mbar_arrive_expect_tx(bars.q_full, kH * p.q_rows * (D * kES));
         for (int h = 0; h < kH; ++h)
           for (int db = 0; db < kDBlocks; ++db) {
             if (p.direct) {
@@ -1051,8 +1056,9 @@ fna_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
             const int valid = p.n_extra - (iter - n_na) * kKVTile;
             rec = make_int4(valid >= kKVTile ? 0 : 2, valid, 0, 0);
           } else {
-            rec = make_int4(kv_tile_interior<NDIM>(p, it, walk) ? 0 : 1, walk.lo[0],
-                            NDIM > 1 ? walk.lo[1] : 0, NDIM > 2 ? walk.lo[2] : 0);
+            rec = make_int4(1, walk.lo[0], NDIM > 1 ? walk.lo[1] : 0, NDIM > 2 ? walk.lo[2] : 0);
+            if (kv_tile_interior<NDIM>(p, it, walk))
+              rec = make_int4(p.kv_rows == kKVTile ? 0 : 2, p.kv_rows, 0, 0);
           }
           // direct mode: coordinates of the tile's first key in the caller's layout
           int xk[B200NA_MAX_DIM] = {0, 0, 0};
@@ -1085,7 +1091,8 @@ fna_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
               ptx::mbar_arrive(bars.rec_full + tseq % kTileRecs);
               ++tseq;
             }
-            ptx::mbar_arrive_expect_tx(bars.kv_full + slot, kTileBytes);
+            ptx::mbar_arrive_expect_tx(bars.kv_full + slot,
+                                       is_extra ? kTileBytes : p.kv_rows * (D * kES));
             for (int db = 0; db < kDBlocks; ++db) {
               if (p.direct && !is_extra && p.sep_heads)
                 ptx::tma_load_5d(kv_sm + slot * kTileBytes + db * kBlockBytes,
@@ -1603,6 +1610,8 @@ int fna_forward_impl(
   }
   if ((tq != kQTile && tq != kHalf) || tkv != kKVTile) return B200NA_ERR_INVALID_ARGUMENT;
   p.halves = (int)(tq / kHalf);
+  p.q_rows = kHalf;
+  p.kv_rows = kKVTile;
   if (Bp % p.G != 0) return B200NA_ERR_INVALID_ARGUMENT;
   if (sq > 0x7fffffffLL || skv > 0x7fffffffLL) return B200NA_ERR_UNSUPPORTED;
   p.dense = 0;
@@ -1631,7 +1640,7 @@ int fna_direct_impl(const void* q, const void* k, const void* v, void* o, float*
                     int n_extra, const long long* token_strides, b200na_stream_t stream,
                     const int* q_origin = nullptr, const int* q_extent = nullptr,
                     const int* kv_origin = nullptr, const int* kv_extent = nullptr, int clip = 0,
-                    bool fold = false) {
+                    bool views = false) {
   if (!q || !k || !v || !o || !shape || !kernel || !q_tile || !kv_tile)
     return B200NA_ERR_INVALID_ARGUMENT;
   // slabs: q / o / lse hold layout coordinates [q_origin, q_origin + q_extent), k / v hold
@@ -1703,8 +1712,13 @@ int fna_direct_impl(const void* q, const void* k, const void* v, void* o, float*
     tq *= p.Tq[a]; tkv *= p.Tkv[a];
     tokens *= p.X[a];
   }
-  if ((tq != kQTile && tq != kHalf) || tkv != kKVTile) return B200NA_ERR_INVALID_ARGUMENT;
-  p.halves = (int)(tq / kHalf);
+  if (tq < 1 || tq > kQTile || tkv < 1 || tkv > kKVTile) return B200NA_ERR_INVALID_ARGUMENT;
+  // tiles of fewer tokens: not with extra tokens, whose 128-row tiles go through the same ring
+  if (!views && ((tq != kQTile && tq != kHalf) || tkv != kKVTile)) return B200NA_ERR_INVALID_ARGUMENT;
+  if (n_extra > 0 && tkv != kKVTile) return B200NA_ERR_INVALID_ARGUMENT;
+  p.halves = tq > kHalf ? 2 : 1;
+  p.q_rows = (int)(tq / p.halves);
+  p.kv_rows = (int)tkv;
   // a 256-token query tile is fetched as two boxes, split along its last non-unit axis
   if (p.halves == 2 && p.Tq[p.half_axis] % 2 != 0) return B200NA_ERR_UNSUPPORTED;
   if (sq > 0x7fffffffLL || skv > 0x7fffffffLL || tokens * B > 0x7fffffffLL ||
@@ -1722,7 +1736,7 @@ int fna_direct_impl(const void* q, const void* k, const void* v, void* o, float*
   p.n_extra = n_extra;
   cudaStream_t cs = reinterpret_cast<cudaStream_t>(stream);
   FoldedPart parts[2];
-  const int n_parts = !fold ? 0 : fna_fold_parts(ndim, p.X[0], p.dil[0], parts);
+  const int n_parts = !views ? 0 : fna_fold_parts(ndim, p.X[0], p.dil[0], parts);
   for (int i = 0; i < n_parts; ++i) {
     FnaParams f = p;
     f.fold_d = p.dil[0];
@@ -1865,6 +1879,8 @@ extern "C" B200NA_API int b200na_fmha_forward(const void* q, const void* k, cons
   p.Rkv[0] = (Nk + kKVTile - 1) / kKVTile;
   p.dense = 1;
   p.halves = 2;
+  p.q_rows = kHalf;
+  p.kv_rows = kKVTile;
   p.Bp = B; p.Hq = Hq; p.Hkv = Hkv;
   p.Sq = Nq; p.Skv = Nk;
   p.scale = scale;

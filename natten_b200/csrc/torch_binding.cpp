@@ -151,7 +151,7 @@ bool direct_supported(std::array<int, kMaxDim> q, const std::array<int, kMaxDim>
     total *= q[a];
     if (q[a] > 1) split = a;
   }
-  if (total != kHalfQTile) {
+  if (total > kHalfQTile) {
     if (q[split] % 2) return false;
     q[split] /= 2;
   }
@@ -238,18 +238,224 @@ Tiles choose_backward(const Problem& p) {
   }
   return t;
 }
+// ---- tiles of any size up to the kernels' (the entries for views) -------------------------------------
+// A tile need not hold exactly 128 (256) tokens, nor powers of two of them: 15 rows are one tile of 15.
+// The rows that remain are zeros in shared memory and masked. Tiles computed against powers of two:
+// 14 x 21 x 22 with 14 x 21 x 9 windows -49 %, 10 x 49 x 19 with 8 x 6 x 5 -32 %, 29 x 21 with 11 x 8
+// -19 %; none where extents and windows are powers of two already.
+
+// Column tokens a stationary tile meets along an axis, and of these [lo, hi), counted from the first,
+// inside the window of every row; `count` tiles of the axis are alike.
+struct Run {
+  int span, lo, hi;
+  long long count;
+};
+using Runs = std::vector<Run>;
+void add_run(Runs& r, int span, int lo, int hi) {
+  for (auto it = r.rbegin(); it != r.rend() && it - r.rbegin() < 4; ++it)
+    if (it->span == span && it->lo == lo && it->hi == hi) {
+      ++it->count;
+      return;
+    }
+  r.push_back({span, lo, hi, 1});
+}
+// Windows of one axis (the largest dilation group): queries attend [start, end).
+struct AxisWindows {
+  int L = 0;
+  std::vector<int> start, end;
+};
+AxisWindows axis_windows(const Problem& p, int a) {
+  AxisWindows w;
+  w.L = ceil_div(p.shape[a], p.dilation[a]);
+  w.start.resize(w.L);
+  w.end.resize(w.L);
+  for (int i = 0; i < w.L; ++i) {
+    w.start[i] = window_start(i, p.kernel[a], p.stride[a], w.L, p.causal[a]);
+    w.end[i] = window_end(i, w.start[i], p.kernel[a], w.L, p.causal[a]);
+  }
+  return w;
+}
+Runs query_runs(const AxisWindows& w, int tile) {
+  Runs r;
+  for (int lo = 0; lo < w.L; lo += tile) {
+    const int hi = std::min(lo + tile, w.L) - 1;
+    add_run(r, w.end[hi] - w.start[lo], w.start[hi] - w.start[lo], w.end[lo] - w.start[lo]);
+  }
+  return r;
+}
+Runs key_runs(const AxisWindows& w, int tile) {
+  Runs r;
+  const auto first = [&](int j) { return (int)(std::upper_bound(w.end.begin(), w.end.end(), j) - w.end.begin()); };
+  const auto last = [&](int j) { return (int)(std::upper_bound(w.start.begin(), w.start.end(), j) - w.start.begin()); };
+  for (int lo = 0; lo < w.L; lo += tile) {
+    const int hi = std::min(lo + tile, w.L) - 1, f = first(lo);
+    add_run(r, last(hi) - f, first(hi) - f, last(lo) - f);
+  }
+  return r;
+}
+// column tiles of all the axis' stationary tiles, and how many of these need no mask
+std::array<double, 2> tiles_met(const Runs& runs, int tile) {
+  long long all = 0, inside = 0;
+  for (const Run& r : runs) {
+    all += r.count * std::max(1, ceil_div(r.span, tile));
+    inside += r.count * std::max(0, std::max(r.hi, 0) / tile - ceil_div(r.lo, tile));
+  }
+  return {(double)all, (double)inside};
+}
+// Sizes worth trying for a length: those that cut it into equal parts, and the powers of two.
+std::vector<int> part_sizes(int length, int most) {
+  std::vector<int> out;
+  for (int n = 1; n <= length; ++n) {
+    const int t = ceil_div(length, n);
+    if (t <= most && (out.empty() || out.back() != t)) out.push_back(t);
+  }
+  for (int t = 1; t <= most && t < 2 * length; t *= 2) out.push_back(t);
+  std::sort(out.begin(), out.end());
+  out.erase(std::unique(out.begin(), out.end()), out.end());
+  return out;
+}
+// Tiles of `nd` axes with sizes out of `sizes`, at most `most` tokens: the last axis takes the largest
+// size that fits the others.
+void tiles_within(const std::vector<int>* const (&sizes)[kMaxDim], int nd, int most,
+                  std::vector<std::array<int, kMaxDim>>& out) {
+  const std::vector<int> one{1};
+  const auto& s0 = nd >= 2 ? *sizes[0] : one;
+  const auto& s1 = nd >= 3 ? *sizes[1] : one;
+  for (int a : s0)
+    for (int b : s1) {
+      if (a * b > most) break;
+      const auto& s = *sizes[nd - 1];
+      const auto it = std::upper_bound(s.begin(), s.end(), most / (a * b));
+      if (it == s.begin()) continue;
+      std::array<int, kMaxDim> t{1, 1, 1};
+      t[0] = a;
+      if (nd >= 3) t[1] = b;
+      t[nd - 1] = *std::prev(it);
+      out.push_back(t);
+    }
+}
+int tokens_of(const std::array<int, kMaxDim>& t) { return t[0] * t[1] * t[2]; }
+
+// An item's own cost (descriptor, first loads, epilogue) in tiles, and what a tile without a mask
+// costs of one with: from the kernels' cycle counters (3650 against 4800 cycles a tile, about 5000 an
+// item; the backward masks half as many values).
+constexpr double kItemTiles = 1.3, kForwardInside = 0.8, kBackwardInside = 0.9;
+// A column tile of fewer than 128 tokens is charged more than its share of the tiles: at 9 % fewer tiles
+// (56 x 56, 7 x 7) and 5 % fewer (128 x 128, 13 x 13, dilation 2) the forward came out 4 % and 5 % slower
+// than with full ones, where tiles drop by 20 % and more 18 to 27 % faster.
+constexpr double kRaggedForward = 1.1, kRaggedBackward = 1.06;
+
+// Tile pair of least cost. `exact_kv`: key/value tiles of exactly 128 tokens (extra tokens).
+bool choose_view(const Problem& p, bool backward, bool exact_kv, Tiles* best) {
+  AxisWindows win[kMaxDim];
+  std::vector<int> sizes[kMaxDim];
+  const std::vector<int>* const size_lists[kMaxDim] = {&sizes[0], &sizes[1], &sizes[2]};
+  for (int a = 0; a < p.nd; ++a) win[a] = axis_windows(p, a);
+  std::vector<std::array<int, kMaxDim>> qs;
+  for (int most = 128; most <= (backward ? 128 : 256); most *= 2) {
+    for (int a = 0; a < p.nd; ++a) sizes[a] = part_sizes(win[a].L, most);
+    tiles_within(size_lists, p.nd, most, qs);
+  }
+  // worked out as they are asked for: runs by rows, tiles met by rows and columns
+  constexpr int kRows = 257, kCols = 129;
+  std::vector<Runs> runs[2][kMaxDim];
+  std::vector<std::array<double, 2>> met[2][kMaxDim];
+  for (int pass = 0; pass < (backward ? 2 : 1); ++pass)
+    for (int a = 0; a < p.nd; ++a) {
+      runs[pass][a].resize(kRows);
+      met[pass][a].assign(kRows * kCols, {-1, 0});
+    }
+  const auto runs_of = [&](int pass, int a, int rows) -> const Runs& {
+    Runs& r = runs[pass][a][rows];
+    if (r.empty()) r = pass ? key_runs(win[a], rows) : query_runs(win[a], rows);
+    return r;
+  };
+  const auto column_tiles = [&](int pass, int a, int rows, int cols) -> const std::array<double, 2>& {
+    auto& m = met[pass][a][rows * kCols + cols];
+    if (m[0] < 0) m = tiles_met(runs_of(pass, a, rows), cols);
+    return m;
+  };
+  std::map<int, std::vector<int>> cuts[kMaxDim];   // key/value sizes worth trying, by query rows
+  double least = 1e300;
+  std::vector<std::array<int, kMaxDim>> kvs;
+  for (const auto& q : qs) {
+    const int nq = tokens_of(q);
+    if (backward ? !box_fits(q, p) : !direct_supported(q, {1, 1, 1}, p)) continue;
+    double q_items = 1;
+    kvs.clear();
+    const std::vector<int>* cut[kMaxDim] = {};
+    for (int a = 0; a < p.nd; ++a) {
+      q_items *= ceil_div(win[a].L, q[a]);
+      std::vector<int>& c = cuts[a][q[a]];
+      if (c.empty()) {
+        int last = 0;
+        for (const Run& r : runs_of(0, a, q[a])) {
+          const int span = std::min(r.span, 128);
+          if (span == last) continue;
+          last = span;
+          const std::vector<int> s = part_sizes(span, 128);
+          c.insert(c.end(), s.begin(), s.end());
+        }
+        std::sort(c.begin(), c.end());
+        c.erase(std::unique(c.begin(), c.end()), c.end());
+      }
+      cut[a] = &c;
+    }
+    if (exact_kv) kvs = compositions(7, p.nd);
+    else tiles_within(cut, p.nd, 128, kvs);
+    for (const auto& kv : kvs) {
+      if (!box_fits(kv, p)) continue;
+      const bool full = tokens_of(kv) == kKVTile;
+      double all = 1, in = 1;
+      for (int a = 0; a < p.nd; ++a) {
+        const auto& m = column_tiles(0, a, q[a], kv[a]);
+        all *= m[0];
+        in *= m[1];
+      }
+      double cost = all + kItemTiles * q_items;
+      if (full) cost -= (1 - (backward ? kBackwardInside : kForwardInside)) * in;
+      else cost *= backward ? kRaggedBackward : kRaggedForward;
+      if (!backward) {
+        cost *= nq <= kHalfQTile ? kSmallQTilePenalty : 2.0;
+      } else {
+        double k_items = 1;
+        all = in = 1;
+        for (int a = 0; a < p.nd; ++a) {
+          k_items *= ceil_div(win[a].L, kv[a]);
+          const auto& m = column_tiles(1, a, kv[a], q[a]);
+          all *= m[0];
+          in *= m[1];
+        }
+        cost += (all + kItemTiles * k_items - (1 - kBackwardInside) * in) *
+                (nq == kHalfQTile ? 1.0 : kRaggedBackward);
+      }
+      // ties go to full tiles, then to such as are long along the last (contiguous) axis
+      cost -= 1e-9 * cost * ((full ? 512 : 0) + q[p.nd - 1] + kv[p.nd - 1] / 256.0);
+      if (cost < least) {
+        least = cost;
+        best->q = q;
+        best->kv = kv;
+      }
+    }
+  }
+  return least < 1e300;
+}
+
 // Plans are kept per problem (at most kMaxPlans, then the store starts over).
-Tiles plan(const Problem& p, bool backward) {
+Tiles plan(const Problem& p, bool backward, bool extra) {
   if (p.nd == 1) return backward ? choose_backward(p) : choose_forward(p);
   constexpr size_t kMaxPlans = 1024;
   static std::mutex mu;
-  static std::map<Problem, Tiles> store[2];
+  static std::map<Problem, Tiles> stores[2][2];
+  auto& store = stores[extra];
   {
     std::lock_guard<std::mutex> lk(mu);
     auto it = store[backward].find(p);
     if (it != store[backward].end()) return it->second;
   }
-  const Tiles t = backward ? choose_backward(p) : choose_forward(p);
+  Tiles t;
+  // no pair that fits a tensor-map box: tiles the caller then finds unusable
+  if (!choose_view(p, backward, extra, &t)) t = backward ? choose_backward(p) : choose_forward(p);
   std::lock_guard<std::mutex> lk(mu);
   if (store[backward].size() >= kMaxPlans) store[backward].clear();
   store[backward][p] = t;
@@ -326,7 +532,7 @@ struct Pointers {
 
 // Kernel choice for a forward call. kNone: not taken here.
 enum class Path { kNone, kTensorCore, kCudaCore };
-Path forward_path(const Problem& p, const Sizes& z, Tiles* tiles) {
+Path forward_path(const Problem& p, const Sizes& z, bool extra, Tiles* tiles) {
   bool tensor_core = reads_natively(z.dt, z.D);
   if (p.nd == 3 && !is_8bit(z.dt))
     for (int a = 0; a < 3; ++a)
@@ -337,7 +543,7 @@ Path forward_path(const Problem& p, const Sizes& z, Tiles* tiles) {
     return Path::kCudaCore;
   }
   if (p.nd == 3 && z.B > 1 && z.D != 128 && (is_8bit(z.dt) || z.D != 64)) return Path::kNone;
-  *tiles = plan(p, false);
+  *tiles = plan(p, false, extra);
   if (p.nd > 1 && !direct_supported(tiles->q, tiles->kv, p)) return Path::kNone;
   return Path::kTensorCore;
 }
@@ -366,10 +572,10 @@ struct GradPointers {
   long long dq_ts, dk_ts, dv_ts;   // tensor-core path only; the CUDA-core path needs 0 (contiguous)
   void *dak, *dav;
 };
-bool backward_on_tensor_cores(const Problem& p, const Sizes& z, Tiles* t) {
+bool backward_on_tensor_cores(const Problem& p, const Sizes& z, bool extra, Tiles* t) {
   if (!is_16bit(z.dt) || !reads_natively(z.dt, z.D)) return false;
   if (p.nd == 3 && z.B > 1 && z.D != 64 && z.D != 128) return false;
-  *t = plan(p, true);
+  *t = plan(p, true, extra);
   return p.nd == 1 || (box_fits(t->q, p) && box_fits(t->kv, p));
 }
 void run_backward(const Problem& p, const Sizes& z, float scale, bool tensor_core, const Tiles& t,
@@ -515,7 +721,7 @@ struct NaFunction : torch::autograd::Function<NaFunction> {
       p.causal = {c.p.causal[0], 0, 0};
     }
     Tiles t;
-    const bool tc = backward_on_tensor_cores(p, c.z, &t) && p.kernel[0] >= 2;
+    const bool tc = backward_on_tensor_cores(p, c.z, extra, &t) && p.kernel[0] >= 2;
     View qv, kv, vv;
     if (tc) {
       qv = as_view(q); kv = as_view(k); vv = as_view(v);
@@ -625,7 +831,7 @@ struct LayerFunction : torch::autograd::Function<LayerFunction> {
         const Tensor dqkv = at::empty({T, 3 * E}, x.options());
         const Tensor delta = at::empty(lse.sizes(), lse.options());
         Tiles t;
-        const bool tc = backward_on_tensor_cores(c.p, c.z, &t);
+        const bool tc = backward_on_tensor_cores(c.p, c.z, false, &t);
         TORCH_CHECK(tc, "natten_b200: layer backward without tensor-core tiles");
         const Pointers d = slices_of(dqkv, c.z.Hq, c.z.D);
         const GradPointers gp{const_cast<void*>(d.q), const_cast<void*>(d.k), const_cast<void*>(d.v),
@@ -832,7 +1038,7 @@ PyObject* py_na(PyObject*, PyObject* const* a, Py_ssize_t n) {
     if (!dense_taken(c.z) || tokens > 0x7fffffff) Py_RETURN_NONE;
     c.dense = true;
   } else {
-    c.path = forward_path(c.p, c.z, &c.tiles);
+    c.path = forward_path(c.p, c.z, ak.defined(), &c.tiles);
     if (c.path == Path::kNone) Py_RETURN_NONE;
   }
   return finish(c, q, k, v, ak, av, a[11] == Py_True);
@@ -891,12 +1097,12 @@ PyObject* py_layer(PyObject*, PyObject* const* a, Py_ssize_t n) {
   for (int i = 0; i < nd; ++i)
     whole = whole && c.p.kernel[i] == c.p.shape[i] && (nd == 1 || !c.p.causal[i]);
   if (whole) Py_RETURN_NONE;
-  c.path = forward_path(c.p, c.z, &c.tiles);
+  c.path = forward_path(c.p, c.z, false, &c.tiles);
   if (c.path != Path::kTensorCore) Py_RETURN_NONE;
   Tensor y;
   if (any_requires_grad({&x, &w1, &b1, &w2, &b2})) {
     Tiles t;
-    if (!backward_on_tensor_cores(c.p, c.z, &t)) Py_RETURN_NONE;
+    if (!backward_on_tensor_cores(c.p, c.z, false, &t)) Py_RETURN_NONE;
     auto call = c10::make_intrusive<SharedCall>();
     call->c = c;
     {
@@ -918,10 +1124,11 @@ PyObject* py_layer(PyObject*, PyObject* const* a, Py_ssize_t n) {
   END_HANDLE_TH_ERRORS
 }
 
-// tiles(backward, shape, kernel, stride, dilation, is_causal) -> (q tile, kv tile)
+// tiles(backward, shape, kernel, stride, dilation, is_causal[, extra]) -> (q tile, kv tile); with
+// `extra` (whether there are extra tokens) the plan of the entries for views
 PyObject* py_tiles(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
-  TORCH_CHECK(n == 6 && PyTuple_Check(a[1]) && PyTuple_GET_SIZE(a[1]) >= 1 && PyTuple_GET_SIZE(a[1]) <= 3,
+  TORCH_CHECK((n == 6 || n == 7) && PyTuple_Check(a[1]) && PyTuple_GET_SIZE(a[1]) >= 1 && PyTuple_GET_SIZE(a[1]) <= 3,
               "tiles(backward, shape, kernel, stride, dilation, is_causal)");
   Problem p;
   p.nd = (int)PyTuple_GET_SIZE(a[1]);
@@ -929,7 +1136,9 @@ PyObject* py_tiles(PyObject*, PyObject* const* a, Py_ssize_t n) {
                   parse_dims(a[3], p.nd, 1, 0, &p.stride) && parse_dims(a[4], p.nd, 1, 0, &p.dilation) &&
                   parse_flags(a[5], p.nd, &p.causal),
               "tiles(): expected tuples of positive integers and flags");
-  const Tiles t = plan(p, a[0] == Py_True);
+  const bool backward = a[0] == Py_True;
+  const Tiles t = n == 7 ? plan(p, backward, a[6] == Py_True)
+                         : (backward ? choose_backward(p) : choose_forward(p));
   PyObject* out = PyTuple_New(2);
   for (int i = 0; i < 2; ++i) {
     PyObject* x = PyTuple_New(p.nd);

@@ -185,6 +185,16 @@ def _choose_tile_shapes(shape: DimensionType, kernel_size: DimensionType, stride
     return _native.tiles(False, shape, kernel_size, stride, dilation, is_causal)
 
 
+@functools.lru_cache(maxsize=512)
+def view_tile_shapes(backward: bool, extra: bool, shape: DimensionType, kernel_size: DimensionType,
+                     stride: DimensionType, dilation: DimensionType, is_causal: CausalArgType
+                     ) -> Tuple[DimensionType, DimensionType]:
+    """(q_tile_shape, kv_tile_shape) where the caller names none: any number of tokens up to the
+    kernels' 256 (backward: 128) and 128, the plan of eager and compiled calls alike. `extra`: there
+    are extra tokens."""
+    return _native.tiles(backward, shape, kernel_size, stride, dilation, is_causal, extra)
+
+
 # ------------------------------------------------------------------------------------------------
 # Token permute / unpermute (reference: src/natten/token_permute/frontend.py:42-137)
 # ------------------------------------------------------------------------------------------------
@@ -501,7 +511,10 @@ def na_forward_op(query: Tensor, key: Tensor, value: Tensor, additional_keys: Op
         return ops.na_forward_simt(query, key, value, additional_keys, additional_values,
                                    list(kernel_size), list(stride), list(dilation),
                                    list(is_causal), scale)
-    if not q_tile_shape or not kv_tile_shape:
+    if not q_tile_shape and not kv_tile_shape and not permuted_layout:
+        q_tile_shape, kv_tile_shape = view_tile_shapes(False, additional_keys is not None, shape,
+                                                       kernel_size, stride, dilation, is_causal)
+    elif not q_tile_shape or not kv_tile_shape:
         auto_q, auto_kv = choose_tile_shapes(shape, kernel_size, stride, dilation, is_causal)
         q_tile_shape = tuple(q_tile_shape) or auto_q
         kv_tile_shape = tuple(kv_tile_shape) or auto_kv
@@ -556,9 +569,12 @@ def _na_backward(ctx, d_out, d_lse):
                    and query.shape[-1] in TENSOR_CORE_HEAD_DIMS
                    and not BACKWARD_ON_CUDA_CORES)
     if tensor_core:
-        q_tile, kv_tile = choose_backward_tile_shapes(
-            tuple(int(x) for x in query.shape[1:1 + na_dim]), kernel_size, stride, dilation,
-            is_causal)
+        problem = (tuple(int(x) for x in query.shape[1:1 + na_dim]), tuple(kernel_size),
+                   tuple(stride), tuple(dilation), tuple(bool(c) for c in is_causal))
+        if any(ctx.bwd_tiles):
+            q_tile, kv_tile = choose_backward_tile_shapes(*problem)
+        else:
+            q_tile, kv_tile = view_tile_shapes(True, ctx.has_extra, *problem)
         q_tile = ctx.bwd_tiles[0] or q_tile      # the caller's choice wins
         kv_tile = ctx.bwd_tiles[1] or kv_tile
         tensor_core = backward_layout_supported(q_tile, kv_tile, dilation)
@@ -692,7 +708,7 @@ def direct_layout_supported(q_tile_shape: DimensionType, kv_tile_shape: Dimensio
     dilation <= 8). A 256-token query tile is fetched as two halves split along its last non-unit
     axis, a 128-token one whole."""
     q_box = list(q_tile_shape)
-    if math.prod(q_box) != KV_TILE_SIZE:
+    if math.prod(q_box) > KV_TILE_SIZE:
         split = 0
         for a, t in enumerate(q_box):
             if t > 1:
@@ -714,6 +730,8 @@ def fna_forward_direct(query: Tensor, key: Tensor, value: Tensor, kernel_size: D
     permute -> kernel -> unpermute (src/natten/backends/blackwell_fna.py:111-165) in one launch,
     the tile gathers (dilation included) done by the kernel's tensor-map loads."""
     q, k, v = query, key, value   # token-strided views are fine, see ops.na_forward_direct
+    if not _inside_op and not ops.full_tiles(q_tile_shape, kv_tile_shape):
+        _lib.check(_lib.ERR_INVALID_ARGUMENT, "fna_forward_direct")
     ak = additional_keys.contiguous() if additional_keys is not None else None
     av = additional_values.contiguous() if additional_values is not None else None
     op = getattr(ops.na_forward_direct, "raw", ops.na_forward_direct) if _inside_op \

@@ -163,6 +163,11 @@ def fmha_forward(query: Tensor, key: Tensor, value: Tensor, is_causal: bool,
     return out, lse
 
 
+def full_tiles(q_tile_shape, kv_tile_shape) -> bool:
+    """Tiles of exactly the kernels' numbers of tokens. Others go through the entries for views."""
+    return math.prod(q_tile_shape) in (128, 256) and math.prod(kv_tile_shape) == 128
+
+
 def _na_direct_fake(query, key, value, additional_keys, additional_values, kernel_size, stride,
                     dilation, is_causal, scale, q_tile_shape, kv_tile_shape):
     return _attn_fake(query)
@@ -186,7 +191,9 @@ def na_forward_direct(query: Tensor, key: Tensor, value: Tensor,
     na_dim = query.dim() - 3
     n_extra = additional_keys.shape[1] if additional_keys is not None else 0
     with torch.cuda.device(query.device):
-        _lib.check(_lib.lib.b200na_na_forward_direct_strided(
+        entry = (_lib.lib.b200na_na_forward_direct_strided if full_tiles(q_tile_shape, kv_tile_shape)
+                 else _lib.lib.b200na_na_forward_view)
+        _lib.check(entry(
             _ptr(query), _ptr(key), _ptr(value), _ptr(additional_keys), _ptr(additional_values),
             n_extra, _ptr(out), _ptr(lse), na_dim, _lib.ints(query.shape[1:1 + na_dim]),
             _lib.ints(kernel_size), _lib.ints(stride), _lib.ints(dilation),
@@ -311,15 +318,17 @@ def na_backward_direct(query: Tensor, key: Tensor, value: Tensor, out: Tensor, d
     n_extra = additional_keys.shape[1] if additional_keys is not None else 0
     delta = torch.empty(query.shape[:-1], dtype=torch.float32, device=query.device)
     with torch.cuda.device(query.device):
-        _lib.check(_lib.lib.b200na_na_backward_direct(
+        full = full_tiles(q_tile_shape, kv_tile_shape)
+        entry = _lib.lib.b200na_na_backward_direct if full else _lib.lib.b200na_na_backward_view
+        _lib.check(entry(
             _ptr(query), _ptr(key), _ptr(value), _ptr(out), _ptr(d_out), _ptr(lse),
             _ptr(additional_keys), _ptr(additional_values), n_extra, _ptr(dq), _ptr(dk), _ptr(dv),
             _ptr(dak) if n_extra else None, _ptr(dav) if n_extra else None, _ptr(delta), na_dim,
             _lib.ints(query.shape[1:1 + na_dim]), _lib.ints(kernel_size), _lib.ints(stride),
             _lib.ints(dilation), _lib.ints(_flags(is_causal)), _lib.ints(q_tile_shape),
             _lib.ints(kv_tile_shape), query.shape[0], query.shape[-2], key.shape[-2],
-            query.shape[-1], DTYPE_CODE[query.dtype], float(scale), _stream(query)),
-            "b200na_na_backward_direct", kernel_launches=4 if n_extra else 3)
+            query.shape[-1], DTYPE_CODE[query.dtype], float(scale), *(() if full else (0,) * 6),
+            _stream(query)), "b200na_na_backward_direct", kernel_launches=4 if n_extra else 3)
     return dq, dk, dv, dak, dav
 
 
