@@ -644,12 +644,13 @@ fna_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         // item's first tile that is nearly always so, hence P is computed with the maximum at hand
         // in one pass over the logits, and kept only if no row of the warp has outgrown it (P is
         // stored after that is known: the logits it overwrites are still there to start again).
-        // A row without keys so far (its window starts in a later tile) has no maximum yet. In the
-        // one-half shape a boundary tile's masks and the packed P together spill: 128 x 128, 13 x 13
-        // windows, dilation 2 took 1052 us in one pass everywhere, 935 us this way.
+        // A row without keys so far (its window starts in a later tile) has no maximum yet. The
+        // one-half shape, chosen for small windows, meets boundary tiles nearly always; masks and
+        // packed P together spill there: 128 x 128, 13 x 13 windows, dilation 2 took 1052 us in one
+        // pass everywhere, 983 us with one pass for the other tiles, 935 us in two passes.
         // 15 x 44 x 80 video in 8 bits: 2051 -> 1859 us; long causal sequences: the same time (the
         // softmax gets 5 % shorter, the wait for the next logits longer).
-        bool again = iter == 0 || (kH == 1 && !interior) || __any_sync(0xffffffffu, m == -INFINITY);
+        bool again = kH == 1 || iter == 0 || __any_sync(0xffffffffu, m == -INFINITY);
         if (!again) {
           const float neg_mc = -m * c;
           const uint64_t nmc2 = ptx::f32x2(neg_mc, neg_mc);

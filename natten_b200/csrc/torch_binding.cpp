@@ -339,11 +339,14 @@ int tokens_of(const std::array<int, kMaxDim>& t) { return t[0] * t[1] * t[2]; }
 // An item's own cost (descriptor, first loads, epilogue) in tiles, and what a tile without a mask
 // costs of one with: from the kernels' cycle counters (3650 against 4800 cycles a tile, about 5000 an
 // item; the backward masks half as many values).
-constexpr double kItemTiles = 1.3, kForwardInside = 0.8, kBackwardInside = 0.9;
+constexpr double kItemTiles = 1.3, kForwardInside = 0.9, kBackwardInside = 0.9;
 // A column tile of fewer than 128 tokens is charged more than its share of the tiles: at 9 % fewer tiles
 // (56 x 56, 7 x 7) and 5 % fewer (128 x 128, 13 x 13, dilation 2) the forward came out 4 % and 5 % slower
 // than with full ones, where tiles drop by 20 % and more 18 to 27 % faster.
 constexpr double kRaggedForward = 1.1, kRaggedBackward = 1.06;
+// The plan of powers of two stays unless another is estimated this much cheaper: the estimate is good to
+// some percent (15 x 30 x 52, 7 x 15 x 15: estimated 7 % cheaper, the training step 2 % slower).
+constexpr double kWorthwhile = 0.9;
 
 // Tile pair of least cost. `exact_kv`: key/value tiles of exactly 128 tokens (extra tokens).
 bool choose_view(const Problem& p, bool backward, bool exact_kv, Tiles* best) {
@@ -376,16 +379,38 @@ bool choose_view(const Problem& p, bool backward, bool exact_kv, Tiles* best) {
     return m;
   };
   std::map<int, std::vector<int>> cuts[kMaxDim];   // key/value sizes worth trying, by query rows
+  const auto cost = [&](const std::array<int, kMaxDim>& q, const std::array<int, kMaxDim>& kv) {
+    const int nq = tokens_of(q);
+    const bool full = tokens_of(kv) == kKVTile;
+    double all = 1, in = 1, q_items = 1;
+    for (int a = 0; a < p.nd; ++a) {
+      const auto& m = column_tiles(0, a, q[a], kv[a]);
+      q_items *= ceil_div(win[a].L, q[a]);
+      all *= m[0];
+      in *= m[1];
+    }
+    double c = all + kItemTiles * q_items;
+    if (full) c -= (1 - (backward ? kBackwardInside : kForwardInside)) * in;
+    else c *= backward ? kRaggedBackward : kRaggedForward;
+    if (!backward) return c * (nq <= kHalfQTile ? kSmallQTilePenalty : 2.0);
+    double k_items = 1;
+    all = in = 1;
+    for (int a = 0; a < p.nd; ++a) {
+      k_items *= ceil_div(win[a].L, kv[a]);
+      const auto& m = column_tiles(1, a, kv[a], q[a]);
+      all *= m[0];
+      in *= m[1];
+    }
+    return c + (all + kItemTiles * k_items - (1 - kBackwardInside) * in) *
+                   (nq == kHalfQTile ? 1.0 : kRaggedBackward);
+  };
   double least = 1e300;
   std::vector<std::array<int, kMaxDim>> kvs;
   for (const auto& q : qs) {
-    const int nq = tokens_of(q);
     if (backward ? !box_fits(q, p) : !direct_supported(q, {1, 1, 1}, p)) continue;
-    double q_items = 1;
     kvs.clear();
     const std::vector<int>* cut[kMaxDim] = {};
     for (int a = 0; a < p.nd; ++a) {
-      q_items *= ceil_div(win[a].L, q[a]);
       std::vector<int>& c = cuts[a][q[a]];
       if (c.empty()) {
         int last = 0;
@@ -405,39 +430,20 @@ bool choose_view(const Problem& p, bool backward, bool exact_kv, Tiles* best) {
     else tiles_within(cut, p.nd, 128, kvs);
     for (const auto& kv : kvs) {
       if (!box_fits(kv, p)) continue;
-      const bool full = tokens_of(kv) == kKVTile;
-      double all = 1, in = 1;
-      for (int a = 0; a < p.nd; ++a) {
-        const auto& m = column_tiles(0, a, q[a], kv[a]);
-        all *= m[0];
-        in *= m[1];
-      }
-      double cost = all + kItemTiles * q_items;
-      if (full) cost -= (1 - (backward ? kBackwardInside : kForwardInside)) * in;
-      else cost *= backward ? kRaggedBackward : kRaggedForward;
-      if (!backward) {
-        cost *= nq <= kHalfQTile ? kSmallQTilePenalty : 2.0;
-      } else {
-        double k_items = 1;
-        all = in = 1;
-        for (int a = 0; a < p.nd; ++a) {
-          k_items *= ceil_div(win[a].L, kv[a]);
-          const auto& m = column_tiles(1, a, kv[a], q[a]);
-          all *= m[0];
-          in *= m[1];
-        }
-        cost += (all + kItemTiles * k_items - (1 - kBackwardInside) * in) *
-                (nq == kHalfQTile ? 1.0 : kRaggedBackward);
-      }
       // ties go to full tiles, then to such as are long along the last (contiguous) axis
-      cost -= 1e-9 * cost * ((full ? 512 : 0) + q[p.nd - 1] + kv[p.nd - 1] / 256.0);
-      if (cost < least) {
-        least = cost;
+      const double c = cost(q, kv) * (1 - 1e-9 * ((tokens_of(kv) == kKVTile ? 512 : 0) + q[p.nd - 1] +
+                                                  kv[p.nd - 1] / 256.0));
+      if (c < least) {
+        least = c;
         best->q = q;
         best->kv = kv;
       }
     }
   }
+  const Tiles even = backward ? choose_backward(p) : choose_forward(p);
+  if ((backward ? box_fits(even.q, p) && box_fits(even.kv, p) : direct_supported(even.q, even.kv, p)) &&
+      cost(even.q, even.kv) * kWorthwhile <= least)
+    *best = even;
   return least < 1e300;
 }
 

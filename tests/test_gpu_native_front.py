@@ -106,3 +106,63 @@ def test_native_front_leaves_other_calls_to_the_python_front():
     (g,) = torch.autograd.grad(nb.na2d(x, q, q, 3).float().sum(), x, create_graph=True)
     with pytest.raises(RuntimeError):
         g.float().sum().backward()
+
+
+RAGGED = [   # shape, window, stride, dilation, causal, forward (q, kv) tile, backward (q, kv) tile
+    ((20, 17), (5, 4), (1, 1), (1, 1), (False, False), (1, 1), (1, 1), (1, 1), (1, 1)),
+    ((20, 17), (5, 4), (2, 1), (1, 1), (False, True), (15, 16), (11, 11), (9, 14), (14, 9)),
+    ((31, 40), (7, 9), (1, 1), (2, 1), (False, False), (3, 42), (127, 1), (1, 127), (127, 1)),
+    ((30, 41), (13, 6), (1, 1), (1, 2), (True, False), (43, 2), (5, 25), (43, 2), (3, 42)),
+    ((7, 9, 11), (3, 5, 11), (1, 2, 1), (1, 1, 1), (True, False, False), (7, 3, 6), (7, 3, 6), (7, 3, 6), (5, 5, 5)),
+    ((7, 9, 11), (4, 9, 3), (1, 1, 1), (1, 1, 2), (False, False, False), (2, 9, 14), (2, 9, 7), (2, 9, 6), (7, 9, 2)),
+    ((300,), (33,), (1,), (3,), (True,), (254,), (101,), (100,), (77,)),
+]
+
+
+@pytest.mark.parametrize("shape,ks,st,di,ca,tq,tkv,bq,bkv", RAGGED)
+@pytest.mark.parametrize("D", [64, 128])
+def test_tiles_of_any_size(shape, ks, st, di, ca, tq, tkv, bq, bkv, D):
+    """Forward and backward with tiles of fewer than 128 tokens, through the C entries for views. What
+    shared memory holds from an earlier launch (here: NaN, in tiles of 128 rows) must not matter."""
+    torch.manual_seed(53)
+    nd, B, Hq, Hkv = len(shape), 2, 4, 2
+    q, d_out = (torch.randn(B, *shape, Hq, D, device="cuda").bfloat16() for _ in range(2))
+    k, v = (torch.randn(B, *shape, Hkv, D, device="cuda").bfloat16() for _ in range(2))
+    out, lse = torch.empty_like(q), torch.empty(q.shape[:-1], device="cuda")
+    delta = torch.empty_like(lse)
+    dq, dk, dv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
+    scale, stream = D ** -0.5, torch.cuda.current_stream().cuda_stream
+    poison = torch.full((1, 2048, 148, D), float("nan"), device="cuda").bfloat16().requires_grad_()
+    geometry = [nd] + [L.ints([int(x) for x in a]) for a in (shape, ks, st, di, ca)]
+    sizes = [B, Hq, Hkv, D, L.BF16, scale]
+    with torch.no_grad():
+        nb.na1d(poison, poison, poison, 512)
+    L.check(L.lib.b200na_na_forward_view(
+        q.data_ptr(), k.data_ptr(), v.data_ptr(), 0, 0, 0, out.data_ptr(), lse.data_ptr(), *geometry,
+        L.ints(tq), L.ints(tkv), *sizes, 0, 0, 0, stream), "b200na_na_forward_view")
+    torch.autograd.grad(nb.na1d(poison, poison, poison, 512), poison, poison.detach())
+    L.check(L.lib.b200na_na_backward_view(
+        q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), d_out.data_ptr(), lse.data_ptr(), 0, 0,
+        0, dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), 0, 0, delta.data_ptr(), *geometry, L.ints(bq),
+        L.ints(bkv), *sizes, 0, 0, 0, 0, 0, 0, stream), "b200na_na_backward_view")
+    assert L.device_status() == 0
+    f = [t.float().cpu().numpy() for t in (q, k, v)]
+    want_o, want_l = oracle.na_forward(*f, ks, st, di, ca)
+    assert np.abs(out.float().cpu().numpy() - want_o).max() <= 2e-2
+    assert np.abs(lse.cpu().numpy() - want_l).max() <= 2e-2
+    want = oracle.na_backward(*f, d_out.float().cpu().numpy(), ks, st, di, ca)
+    for g, w in zip((dq, dk, dv), want):
+        assert np.abs(g.float().cpu().numpy() - w).max() <= 2e-2 * max(1.0, np.abs(w).max())
+
+
+@pytest.mark.parametrize("shape,ks,st,di", [((14, 21, 22), (14, 21, 9), (1, 1, 4), (1, 1, 1)),
+                                            ((20, 103), (5, 7), (1, 1), (4, 4)), ((13, 29), (11, 8), (1, 1), (1, 1))])
+def test_planned_tiles_8bit(shape, ks, st, di):
+    """Shapes whose planned tiles are no powers of two, 8-bit operands: one e4m3 step (1/8)."""
+    torch.manual_seed(59)
+    q, k, v = (torch.randn(1, *shape, 2, 128).to(torch.float8_e4m3fn) for _ in range(3))
+    ca = (False,) * len(shape)
+    out = {2: nb.na2d, 3: nb.na3d}[len(shape)](q.cuda(), k.cuda(), v.cuda(), ks, st, di, ca)
+    assert L.device_status() == 0
+    want, _ = oracle.na_forward(*[t.float().numpy() for t in (q, k, v)], ks, st, di, ca)
+    assert np.abs(out.float().cpu().numpy() - want).max() <= 0.125 * max(1.0, np.abs(want).max())
