@@ -309,6 +309,17 @@ B200NA_API int b200na_fmha_forward(const void* q, const void* k, const void* v, 
                         b200na_stream_t stream);
 
 /*
+ * The same, not causal, with the keys cut into b200na_fmha_splits(...) parts (1: do not cut) where the
+ * query tiles alone leave most of the GPU idle. scratch: splits * B * Nq * Hq * (D + 1) floats, 16-byte
+ * aligned (unused and may be NULL when splits is 1): the parts' rows and logsumexps in fp32, added up
+ * by a second kernel.
+ */
+B200NA_API int b200na_fmha_splits(int B, int Nq, int Nk, int Hq, int D, int dtype, int causal);
+B200NA_API int b200na_fmha_forward_split(const void* q, const void* k, const void* v, void* o, float* lse,
+                                         int B, int Nq, int Nk, int Hq, int Hkv, int D, int dtype,
+                                         float scale, float* scratch, b200na_stream_t stream);
+
+/*
  * Neighborhood attention forward on the ORIGINAL token layout with CUDA-core fp32 arithmetic.
  * This is the path for fp32 operands (the reference serves fp32 through its CUTLASS 2.x / Flex
  * backends: src/natten/backends/fna.py, flex.py; semantics csrc/include/natten/cuda/reference/

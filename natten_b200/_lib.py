@@ -26,7 +26,7 @@ SYMBOLS = (
     "b200na_strerror", "b200na_version", "b200na_token_permute", "b200na_token_unpermute",
     "b200na_fna_forward", "b200na_fna_forward_sharded", "b200na_na_forward_direct_sharded", "b200na_fna_forward_extra_kv", "b200na_na_forward_direct", "b200na_na_forward_direct_strided",
     "b200na_na_forward_view", "b200na_na_backward_view", "b200na_column_sum", "b200na_column_sum_scratch",
-    "b200na_fmha_forward",
+    "b200na_fmha_forward", "b200na_fmha_splits", "b200na_fmha_forward_split",
     "b200na_na_forward", "b200na_na_forward_workspace_bytes", "b200na_na_forward_static", "b200na_na_forward_simt", "b200na_na_backward_simt", "b200na_na_backward_direct", "b200na_merge",
     "b200na_device_status",
 )
@@ -111,6 +111,10 @@ def _load() -> ctypes.CDLL:
     lib.b200na_na_forward_static.argtypes = [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int,
                                              ip, ip, ip, ip, ip, ip, ip, c_int, c_int, c_int,
                                              c_int, c_int, c_float, c_void_p]
+    lib.b200na_fmha_splits.restype = c_int
+    lib.b200na_fmha_splits.argtypes = [c_int] * 7
+    lib.b200na_fmha_forward_split.restype = c_int
+    lib.b200na_fmha_forward_split.argtypes = [c_void_p] * 5 + [c_int] * 7 + [c_float, c_void_p, c_void_p]
     lib.b200na_fmha_forward.restype = c_int
     lib.b200na_fmha_forward.argtypes = [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int,
                                         c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_int,

@@ -91,6 +91,9 @@ struct FnaParams {
   int clip;                    // windows are cut to the keys [clip_lo, clip_hi) that are present
   int clip_lo[B200NA_MAX_DIM];
   int clip_hi[B200NA_MAX_DIM];
+  int splits, split_tiles;  // > 1: dense attention, an item walks split_tiles key/value tiles of its
+  float* part_o;            // query tile and leaves its rows in fp32, [splits][B, Nq, Hq][D], with
+  float* part_lse;          // their logsumexps [splits][B, Nq, Hq], for the kernel that adds them up
   int dense;                // dense attention: one axis, window = all keys (or causal prefix)
   int direct;               // Q/K/V/O/LSE are in the caller's [B, *X, H, D] layout (no permutation)
   long long tok_stride[3];  // direct: elements between consecutive tokens of q, k, v (0 = H * D)
@@ -175,9 +178,14 @@ __device__ __forceinline__ void axis_window(const FnaParams& p, int a, int i, in
 // coordinates and walks causal axes from the far end, see there).
 struct WorkCursor {
   long long w;
-  int qt, h, bp;
+  int qt, h, bp, split;
   __device__ __forceinline__ void init(const FnaParams& p, long long w0) {
     w = w0;
+    split = 0;
+    if (p.splits > 1) {
+      split = (int)(w0 % p.splits);
+      w0 /= p.splits;
+    }
     qt = (int)(w0 % p.n_qtiles);
     const long long rest = w0 / p.n_qtiles;
     h = (int)(rest % p.Hq);
@@ -260,7 +268,14 @@ __device__ __forceinline__ void decode_item(const FnaParams& p, const WorkCursor
   }
   if (NDIM == 1 && p.fold_d) it.g[1] = gl;   // the group is a tensor axis of its own
   it.qt = qt;
-  if (p.dense && it.qt * kQTile >= p.Sq) it.skip = 1;
+  if (p.dense && it.qt * p.Tq[0] >= p.Sq) it.skip = 1;
+  if (NDIM == 1 && p.splits > 1) {
+    it.g[1] = cur.split;   // no groups in dense attention
+    it.kv_t0[0] = cur.split * p.split_tiles;
+    it.kv_lo[0] = it.kv_t0[0] * p.Tkv[0];
+    it.kv_n[0] = imin(p.split_tiles, it.kv_n[0] - it.kv_t0[0]);
+    it.n_tiles = it.kv_n[0];
+  }
   it.n_na = it.n_tiles;
   it.n_tiles += p.extra_tiles;
 }
@@ -647,10 +662,13 @@ fna_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         // A row without keys so far (its window starts in a later tile) has no maximum yet. The
         // one-half shape, chosen for small windows, meets boundary tiles nearly always; masks and
         // packed P together spill there: 128 x 128, 13 x 13 windows, dilation 2 took 1052 us in one
-        // pass everywhere, 983 us with one pass for the other tiles, 935 us in two passes.
+        // pass everywhere, 983 us with one pass for the other tiles, 935 us in two passes. The windows
+        // of 3-D layouts do hold whole tiles: 15 x 30 x 52, 7 x 15 x 15, forward 682 us in two
+        // passes, 655 us this way.
         // 15 x 44 x 80 video in 8 bits: 2051 -> 1859 us; long causal sequences: the same time (the
         // softmax gets 5 % shorter, the wait for the next logits longer).
-        bool again = kH == 1 || iter == 0 || __any_sync(0xffffffffu, m == -INFINITY);
+        bool again = iter == 0 || (kH == 1 && (NDIM != 3 || !interior)) ||
+                     __any_sync(0xffffffffu, m == -INFINITY);
         if (!again) {
           const float neg_mc = -m * c;
           const uint64_t nmc2 = ptx::f32x2(neg_mc, neg_mc);
@@ -763,6 +781,34 @@ fna_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
       ph_o ^= 1;
       PROF_MARK(4)
       ptx::tc_fence_after_sync();
+      if (NDIM == 1 && p.splits > 1) {
+        // a part of the keys: normalised rows in fp32, to be weighed by their logsumexps
+        const long long prow = (long long)it.g[1] * p.Bp * p.Sq * p.Hq + out_row;
+#pragma unroll
+        for (int ch = 0; ch < D / 64; ++ch) {
+          uint32_t orr[32];
+          ptx::tmem_ld32_x2<D / 2>(o_addr + ch * 32, orr);
+          ptx::tmem_ld_wait();
+          const int col = part * (D / 2) + ch * 32;
+          float* const dst = p.part_o + prow * p.d_real + col;
+          if (valid) {
+#pragma unroll
+            for (int j = 0; j < 32; j += 4)
+              if (col + j < p.d_real)
+                *reinterpret_cast<float4*>(dst + j) =
+                    make_float4(__uint_as_float(orr[j]) * inv, __uint_as_float(orr[j + 1]) * inv,
+                                __uint_as_float(orr[j + 2]) * inv, __uint_as_float(orr[j + 3]) * inv);
+          }
+        }
+        if (valid && part == 0) p.part_lse[prow] = logf(total) + m * p.scale;
+        ptx::tc_fence_before_sync();
+        ptx::mbar_arrive(bars.o_empty + half);
+        release_item(bars, seq);
+        itp = nxt;
+        ws[0] = nws[0];
+        we[0] = nwe[0];
+        continue;
+      }
       // This thread's share of its output row: D/2 elements = kChunks 16-byte chunks. A store of
       // one chunk per lane would touch 16 rows (32 separate lines) per instruction, and the
       // load/store unit would spend more time on the epilogue than the arithmetic does. The
@@ -1480,7 +1526,7 @@ int launch_fna(const void* q, const void* k, const void* v, FnaParams& p, int D,
 #ifdef B200NA_TEST_HOOKS
   p.test_withhold = g_test_withhold;
 #endif
-  p.total_work = (long long)p.n_qtiles * p.Hq * p.Bp;
+  p.total_work = (long long)p.n_qtiles * p.Hq * p.Bp * (p.splits > 1 ? p.splits : 1);
   if (p.total_work == 0) return B200NA_OK;
   const long long slots = (long long)st->sms * ctas_per_sm(p.halves);
   const int grid = (int)(p.total_work < slots ? p.total_work : slots);
@@ -1846,10 +1892,74 @@ extern "C" B200NA_API int b200na_fna_forward(const void* q, const void* k, const
                                   scale, nullptr, nullptr, nullptr, nullptr, nullptr, 0, stream);
 }
 
-extern "C" B200NA_API int b200na_fmha_forward(const void* q, const void* k, const void* v, void* o, float* lse,
-                                   int B, int Nq, int Nk, int Hq, int Hkv, int D, int dtype,
-                                   float scale, int causal, b200na_stream_t stream) {
-  using namespace b200na;
+namespace b200na {
+namespace {
+constexpr int kSplitSms = 148;       // SMs the split is planned for
+constexpr int kMinSplitTiles = 4;    // key/value tiles a part has at least
+
+// Rows of the query tile: 256 (one CTA per SM) unless 128-row tiles (two CTAs per SM) waste less. They
+// do when the last 256-row tile would be mostly padding (a 128-row tile is charged 1.15 of half a
+// 256-row one, as in the tile plans), and when even they do not fill the SMs: a CTA alone on its SM
+// takes about as long for a tile of 128 rows as for 256, with half the rows to do.
+int dense_halves(int B, int Nq, int Hq) {
+  const long long t128 = (Nq + 127) / 128, t256 = (Nq + 255) / 256, heads = (long long)B * Hq;
+  return (t128 * heads <= kSplitSms || 1.15 * t128 < 2.0 * t256) ? 1 : 2;
+}
+// Parts the keys of dense attention are cut into. A few queries against many keys are a few items for
+// 148 SMs, each a serial walk over all the key/value tiles: cut so that the parts fill the SMs, at
+// least kMinSplitTiles tiles each, so that adding the parts up stays small beside them.
+int dense_splits(int B, int Nq, int Nk, int Hq, int D, int dtype, int causal) {
+  if (causal || elem_bytes_of(dtype) != 2 || kernel_head_dim(D, dtype) == 0) return 1;
+  if (B < 1 || Nq < 1 || Nk < 1 || Hq < 1) return 1;
+  const int halves = dense_halves(B, Nq, Hq), rows = kHalf * halves;
+  const long long items = (long long)((Nq + rows - 1) / rows) * B * Hq;
+  const int tiles = (Nk + kKVTile - 1) / kKVTile;
+  long long n = (long long)kSplitSms * ctas_per_sm(halves) / items;
+  if (n > tiles / kMinSplitTiles) n = tiles / kMinSplitTiles;
+  if (n < 2) return 1;
+  const int per = (tiles + (int)n - 1) / (int)n;
+  return (tiles + per - 1) / per;   // no empty part
+}
+
+// out = sum_s w_s part_s / sum_s w_s with w_s = e^(lse_s - max lse): a warp per row, four columns a lane.
+template <class T>
+__global__ void __launch_bounds__(256) add_parts_kernel(const float* __restrict__ part_o,
+                                                        const float* __restrict__ part_lse, T* o,
+                                                        float* lse, long long rows, int D, int splits) {
+  const long long row = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
+  const int lane = threadIdx.x & 31, col = lane * 4;
+  if (row >= rows) return;
+  float top = -INFINITY;
+  for (int s = lane; s < splits; s += 32) top = fmaxf(top, part_lse[s * rows + row]);
+#pragma unroll
+  for (int d = 16; d > 0; d >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, d));
+  const float base = top == -INFINITY ? 0.f : top;
+  float weight = 0.f;
+  float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+  for (int s = 0; s < splits; ++s) {
+    const float w = expf(part_lse[s * rows + row] - base);
+    weight += w;
+    if (col < D) {
+      const float4 x = *reinterpret_cast<const float4*>(part_o + (s * rows + row) * D + col);
+      acc.x += w * x.x; acc.y += w * x.y; acc.z += w * x.z; acc.w += w * x.w;
+    }
+  }
+  // a NaN anywhere stays one
+  const float inv = weight == 0.f ? 0.f : 1.f / weight;
+  if (col < D) {
+    constexpr int kType = std::is_same<T, __nv_bfloat16>::value ? kTyBf16 : kTyF16;
+    uint2 y;
+    y.x = pack2<kType>(acc.x * inv, acc.y * inv);
+    y.y = pack2<kType>(acc.z * inv, acc.w * inv);
+    *reinterpret_cast<uint2*>(o + row * D + col) = y;
+  }
+  if (lse != nullptr && lane == 0) lse[row] = top + logf(weight);
+}
+
+int fmha_impl(const void* q, const void* k, const void* v, void* o, float* lse, int B, int Nq, int Nk,
+              int Hq, int Hkv, int D, int dtype, float scale, int causal, int splits, float* scratch,
+              b200na_stream_t stream) {
   if (!q || !k || !v || !o) return B200NA_ERR_INVALID_ARGUMENT;
   if (B < 1 || Nq < 1 || Nk < 1 || Hq < 1 || Hkv < 1 || Hq % Hkv != 0)
     return B200NA_ERR_INVALID_ARGUMENT;
@@ -1872,14 +1982,14 @@ extern "C" B200NA_API int b200na_fmha_forward(const void* q, const void* k, cons
   p.X[0] = Nk;
   p.q_len[0] = Nq;
   p.causal[0] = causal ? 1 : 0;
-  p.Tq[0] = kQTile;
+  p.halves = dense_halves(B, Nq, Hq);
+  p.Tq[0] = kHalf * p.halves;
   p.Tkv[0] = kKVTile;
   p.tkv_shift[0] = 7;
-  p.n_qtiles = (Nq + kQTile - 1) / kQTile;
+  p.n_qtiles = (Nq + p.Tq[0] - 1) / p.Tq[0];
   p.Rq[0] = p.n_qtiles;
   p.Rkv[0] = (Nk + kKVTile - 1) / kKVTile;
   p.dense = 1;
-  p.halves = 2;
   p.q_rows = kHalf;
   p.kv_rows = kKVTile;
   p.Bp = B; p.Hq = Hq; p.Hkv = Hkv;
@@ -1888,8 +1998,50 @@ extern "C" B200NA_API int b200na_fmha_forward(const void* q, const void* k, cons
   p.scale_log2 = scale * 1.4426950408889634f;
   p.o = o;
   p.lse = lse;
-  return launch_fna(q, k, v, p, D, dtype, reinterpret_cast<cudaStream_t>(stream));
+  cudaStream_t cs = reinterpret_cast<cudaStream_t>(stream);
+  if (splits < 2) return launch_fna(q, k, v, p, D, dtype, cs);
+  const long long rows = (long long)B * Nq * Hq;
+  p.splits = splits;
+  p.split_tiles = (p.Rkv[0] + splits - 1) / splits;
+  p.part_o = scratch;
+  p.part_lse = scratch + (long long)splits * rows * D;
+  const int rc = launch_fna(q, k, v, p, D, dtype, cs);
+  if (rc != B200NA_OK) return rc;
+  const unsigned grid = (unsigned)((rows + 7) / 8);
+  if (dtype == B200NA_BF16)
+    add_parts_kernel<<<grid, 256, 0, cs>>>(p.part_o, p.part_lse, (__nv_bfloat16*)o, lse, rows, D, splits);
+  else
+    add_parts_kernel<<<grid, 256, 0, cs>>>(p.part_o, p.part_lse, (__half*)o, lse, rows, D, splits);
+  B200NA_CUDA_TRY(cudaGetLastError());
+  return B200NA_OK;
 }
+}  // namespace
+}  // namespace b200na
+
+extern "C" B200NA_API int b200na_fmha_forward(const void* q, const void* k, const void* v, void* o,
+                                              float* lse, int B, int Nq, int Nk, int Hq, int Hkv, int D,
+                                              int dtype, float scale, int causal,
+                                              b200na_stream_t stream) {
+  return b200na::fmha_impl(q, k, v, o, lse, B, Nq, Nk, Hq, Hkv, D, dtype, scale, causal, 1, nullptr,
+                           stream);
+}
+
+extern "C" B200NA_API int b200na_fmha_splits(int B, int Nq, int Nk, int Hq, int D, int dtype,
+                                             int causal) {
+  return b200na::dense_splits(B, Nq, Nk, Hq, D, dtype, causal);
+}
+
+extern "C" B200NA_API int b200na_fmha_forward_split(const void* q, const void* k, const void* v, void* o,
+                                                    float* lse, int B, int Nq, int Nk, int Hq, int Hkv,
+                                                    int D, int dtype, float scale, float* scratch,
+                                                    b200na_stream_t stream) {
+  const int splits = b200na::dense_splits(B, Nq, Nk, Hq, D, dtype, 0);
+  if (splits > 1 && (!scratch || reinterpret_cast<uintptr_t>(scratch) % 16 != 0))
+    return B200NA_ERR_INVALID_ARGUMENT;
+  return b200na::fmha_impl(q, k, v, o, lse, B, Nq, Nk, Hq, Hkv, D, dtype, scale, 0, splits, scratch,
+                           stream);
+}
+
 
 #ifdef B200NA_PROFILE
 // Instrumented builds only: device buffer of [grid][4][8] int64 cycle counters.

@@ -49,7 +49,8 @@ constexpr int kMaxDim = 3;
 
 // ---- the C library (the one the Python package loaded) -----------------------------------------
 #define B200NA_FUNCTIONS(X)                                                                  \
-  X(na_forward_view) X(na_forward_simt) X(fmha_forward) X(na_backward_view) X(na_backward_simt) \
+  X(na_forward_view) X(na_forward_simt) X(fmha_forward) X(fmha_splits) X(fmha_forward_split)  \
+  X(na_backward_view) X(na_backward_simt)                                                     \
   X(column_sum) X(column_sum_scratch) X(strerror)
 struct Lib {
 #define X(name) decltype(&b200na_##name) name = nullptr;
@@ -656,6 +657,17 @@ Forward forward_now(const Call& c, const Tensor& q, const Tensor& k, const Tenso
     const Tensor qc = q.contiguous(), kc = k.contiguous(), vc = v.contiguous();
     const int nq = (int)(q.numel() / (c.z.B * c.z.Hq * c.z.D)),
               nk = (int)(k.numel() / (c.z.B * c.z.Hkv * c.z.D));
+    const int splits =
+        c.scale > 0.f ? lib.fmha_splits(c.z.B, nq, nk, c.z.Hq, c.z.D, c.z.dt, c.p.causal[0]) : 1;
+    if (splits > 1) {
+      const Tensor scratch = at::empty({(int64_t)splits * c.z.B * nq * c.z.Hq * (c.z.D + 1)},
+                                       q.options().dtype(at::kFloat));
+      f.status = lib.fmha_forward_split(qc.data_ptr(), kc.data_ptr(), vc.data_ptr(), f.out.data_ptr(),
+                                        lse, c.z.B, nq, nk, c.z.Hq, c.z.Hkv, c.z.D, c.z.dt, c.scale,
+                                        scratch.data_ptr<float>(), stream);
+      launches += 2;
+      return f;
+    }
     f.status = lib.fmha_forward(qc.data_ptr(), kc.data_ptr(), vc.data_ptr(), f.out.data_ptr(), lse,
                                 c.z.B, nq, nk, c.z.Hq, c.z.Hkv, c.z.D, c.z.dt, c.scale,
                                 c.p.causal[0], stream);

@@ -155,6 +155,16 @@ def fmha_forward(query: Tensor, key: Tensor, value: Tensor, is_causal: bool,
     everything else on CUDA cores (the library picks the kernel)."""
     out, lse = _attn_fake(query)
     B, Nq, Hq, D = query.shape
+    splits = _lib.lib.b200na_fmha_splits(B, Nq, key.shape[1], Hq, D, DTYPE_CODE[query.dtype],
+                                         1 if is_causal else 0)
+    if splits > 1 and scale > 0:
+        scratch = torch.empty(splits * B * Nq * Hq * (D + 1), dtype=torch.float32, device=query.device)
+        with torch.cuda.device(query.device):
+            _lib.check(_lib.lib.b200na_fmha_forward_split(
+                _ptr(query), _ptr(key), _ptr(value), _ptr(out), _ptr(lse), B, Nq, key.shape[1], Hq,
+                key.shape[2], D, DTYPE_CODE[query.dtype], float(scale), _ptr(scratch),
+                _stream(query)), "b200na_fmha_forward_split", kernel_launches=2)
+        return out, lse
     with torch.cuda.device(query.device):
         _lib.check(_lib.lib.b200na_fmha_forward(
             _ptr(query), _ptr(key), _ptr(value), _ptr(out), _ptr(lse), B, Nq, key.shape[1], Hq,

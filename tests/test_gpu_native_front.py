@@ -166,3 +166,31 @@ def test_planned_tiles_8bit(shape, ks, st, di):
     assert L.device_status() == 0
     want, _ = oracle.na_forward(*[t.float().numpy() for t in (q, k, v)], ks, st, di, ca)
     assert np.abs(out.float().cpu().numpy() - want).max() <= 0.125 * max(1.0, np.abs(want).max())
+
+
+@pytest.mark.parametrize("B,nq,nk,hq,hkv,D", [
+    (1, 1, 1024, 1, 1, 64),       # two parts of four tiles, the fewest there are
+    (2, 3, 16384, 4, 2, 128),     # a decoding step: many parts, GQA
+    (1, 130, 5000, 2, 2, 40),     # two query tiles, a ragged last part and tile, a narrow head
+    (3, 300, 1537, 3, 1, 128),    # 128-row tiles
+    (1, 257, 511, 1, 1, 64),      # too few keys to cut
+])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_dense_attention_over_parts_of_the_keys(B, nq, nk, hq, hkv, D, dtype):
+    """Against attention in 64 bits: the result's rounding (2^-8 / 2^-11 of it) and that of the
+    probabilities, the same relative size; the registered operator gives the same bits."""
+    torch.manual_seed(61)
+    q = torch.randn(B, nq, hq, D, device="cuda").to(dtype)
+    k, v = (torch.randn(B, nk, hkv, D, device="cuda").to(dtype) for _ in range(2))
+    parts = L.lib.b200na_fmha_splits(B, nq, nk, hq, D, L.BF16, 0)
+    assert (parts > 1) == (nk >= 1024)
+    out, lse = nb.attention(q, k, v, return_lse=True)
+    assert L.device_status() == 0
+    kd, vd = (t.double().repeat_interleave(hq // hkv, 2) for t in (k, v))
+    s = torch.einsum("bqhd,bkhd->bqhk", q.double(), kd) * D ** -0.5
+    want = torch.einsum("bqhk,bkhd->bqhd", s.softmax(-1), vd)
+    bound = 2 ** (-7 if dtype == torch.bfloat16 else -10) * want.abs().max()
+    assert (out.double() - want).abs().max() <= bound
+    assert (lse.double() - s.logsumexp(-1)).abs().max() <= 1e-3
+    again, lse2 = torch.compile(lambda a, b, c: nb.attention(a, b, c, return_lse=True))(q, k, v)
+    assert torch.equal(again, out) and torch.equal(lse2, lse)
