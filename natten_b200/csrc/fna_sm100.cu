@@ -1907,7 +1907,9 @@ int dense_halves(int B, int Nq, int Hq) {
 }
 // Parts the keys of dense attention are cut into. A few queries against many keys are a few items for
 // 148 SMs, each a serial walk over all the key/value tiles: cut so that the parts fill the SMs, at
-// least kMinSplitTiles tiles each, so that adding the parts up stays small beside them.
+// least kMinSplitTiles tiles each, so that adding the parts up stays small beside them. Whole calls,
+// us: 1 query, 16384 keys, 8 heads of 128: 236 -> 44.5; 4 x 64, 4096, 12 of 64: 71 -> 39.5; 512, 8192, 4 of
+// 128: 129 -> 44.5; 2 x 200, 12000, 8 of 128: 178 -> 62.5.
 int dense_splits(int B, int Nq, int Nk, int Hq, int D, int dtype, int causal) {
   if (causal || elem_bytes_of(dtype) != 2 || kernel_head_dim(D, dtype) == 0) return 1;
   if (B < 1 || Nq < 1 || Nk < 1 || Hq < 1) return 1;
