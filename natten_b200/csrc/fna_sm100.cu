@@ -1204,21 +1204,53 @@ typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t,
                                   const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
                                   CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 
-int get_encode_fn(EncodeTiledFn* fn) {
-  static std::mutex mu;
-  static EncodeTiledFn cached = nullptr;
-  std::lock_guard<std::mutex> lk(mu);
-  if (!cached) {
-    void* sym = nullptr;
-    cudaDriverEntryPointQueryResult qres;
-    B200NA_CUDA_TRY(cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &sym, cudaEnableDefault, &qres));
-    if (!sym || qres != cudaDriverEntryPointSuccess) {
-      set_last_cuda_error(cudaErrorUnknown, "cudaGetDriverEntryPoint(cuTensorMapEncodeTiled)");
-      return B200NA_ERR_CUDA;
-    }
-    cached = reinterpret_cast<EncodeTiledFn>(sym);
+typedef CUresult (*CtxGetCurrentFn)(CUcontext*);
+
+// Looks up a driver function once per process (the library does not link libcuda).
+template <class Fn>
+int driver_function(const char* name, std::atomic<Fn>& cached, Fn* fn) {
+  *fn = cached.load(std::memory_order_acquire);
+  if (*fn) return B200NA_OK;
+  void* sym = nullptr;
+  cudaDriverEntryPointQueryResult qres;
+  B200NA_CUDA_TRY(cudaGetDriverEntryPoint(name, &sym, cudaEnableDefault, &qres));
+  if (!sym || qres != cudaDriverEntryPointSuccess) {
+    set_last_cuda_error(cudaErrorUnknown, name);
+    return B200NA_ERR_CUDA;
   }
-  *fn = cached;
+  *fn = reinterpret_cast<Fn>(sym);
+  cached.store(*fn, std::memory_order_release);
+  return B200NA_OK;
+}
+
+// cuTensorMapEncodeTiled, a driver function, for a 128-byte-swizzled tiled map. Driver functions use the
+// calling thread's current context, and a thread that has made no runtime call yet (autograd's, in a
+// backward that starts with one of these kernels) has none, although cudaGetDevice answers there:
+// cudaSetDevice binds the device's primary context.
+int encode_tiled(CUtensorMap* tm, CUtensorMapDataType type, int rank, const void* ptr,
+                 const cuuint64_t* dims, const cuuint64_t* strides, const cuuint32_t* box,
+                 const cuuint32_t* element_strides) {
+  static std::atomic<EncodeTiledFn> cached_encode{nullptr};
+  static std::atomic<CtxGetCurrentFn> cached_current{nullptr};
+  EncodeTiledFn encode;
+  CtxGetCurrentFn current;
+  int rc = driver_function("cuTensorMapEncodeTiled", cached_encode, &encode);
+  if (rc == B200NA_OK) rc = driver_function("cuCtxGetCurrent", cached_current, &current);
+  if (rc != B200NA_OK) return rc;
+  CUcontext context = nullptr;
+  if (current(&context) != CUDA_SUCCESS || !context) {
+    int dev = 0;
+    B200NA_CUDA_TRY(cudaGetDevice(&dev));
+    B200NA_CUDA_TRY(cudaSetDevice(dev));
+  }
+  const CUresult r = encode(tm, type, (cuuint32_t)rank, const_cast<void*>(ptr), dims, strides, box,
+                            element_strides, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                            CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) {
+    set_last_cuda_error(static_cast<cudaError_t>(r), "cuTensorMapEncodeTiled");   // same numbers
+    return B200NA_ERR_CUDA;
+  }
   return B200NA_OK;
 }
 
@@ -1235,23 +1267,13 @@ CUtensorMapDataType tma_type_of(int dtype) {
 // Tensor map over a heads-last [Bp, S, H, D] tensor; box = 128 bytes of the head dim (64 16-bit or
 // 128 8-bit elements) x 1 (h) x 128 (s) x 1.
 int make_tensor_map(CUtensorMap* tm, const void* ptr, int dtype, int Bp, int S, int H, int D) {
-  EncodeTiledFn enc = nullptr;
-  int rc = get_encode_fn(&enc);
-  if (rc != B200NA_OK) return rc;
   const cuuint64_t es = (cuuint64_t)elem_bytes_of(dtype);
   const cuuint64_t dims[4] = {(cuuint64_t)D, (cuuint64_t)H, (cuuint64_t)S, (cuuint64_t)Bp};
   const cuuint64_t strides[3] = {(cuuint64_t)D * es, (cuuint64_t)H * D * es,
                                  (cuuint64_t)S * H * D * es};
   const cuuint32_t box[4] = {(cuuint32_t)(128 / es), 1, (cuuint32_t)kKVTile, 1};
   const cuuint32_t estr[4] = {1, 1, 1, 1};
-  const CUresult r = enc(tm, tma_type_of(dtype), 4, const_cast<void*>(ptr), dims, strides, box,
-                         estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                         CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS) {
-    set_last_cuda_error(cudaErrorInvalidValue, "cuTensorMapEncodeTiled");
-    return B200NA_ERR_CUDA;
-  }
-  return B200NA_OK;
+  return encode_tiled(tm, tma_type_of(dtype), 4, ptr, dims, strides, box, estr);
 }
 
 // Tensor map over the caller's heads-last [B, X0, X1, X2, H, D] tensor, seen as the 5-D array
@@ -1264,9 +1286,6 @@ int make_tensor_map(CUtensorMap* tm, const void* ptr, int dtype, int Bp, int S, 
 int make_tensor_map_direct(CUtensorMap* tm, const void* ptr, int dtype, int B, const int* X,
                            int H, int D, const int* tile, const int* dil,
                            long long token_stride, int ndim_sep, const FoldedAxis* fold) {
-  EncodeTiledFn enc = nullptr;
-  int rc = get_encode_fn(&enc);
-  if (rc != B200NA_OK) return rc;
   const cuuint64_t es = (cuuint64_t)elem_bytes_of(dtype);
   if (fold) {
     const cuuint64_t row = (cuuint64_t)(token_stride > 0 ? token_stride : (long long)H * D) * es;
@@ -1283,16 +1302,8 @@ int make_tensor_map_direct(CUtensorMap* tm, const void* ptr, int dtype, int B, c
                                   (cuuint64_t)B};
     const cuuint64_t str_t[4] = {by_pos, row, by_batch, by_batch};
     const cuuint32_t box_t[5] = {ch, n, 1, 1, 1};
-    const CUresult r = enc(tm, tma_type_of(dtype), 5, const_cast<void*>(base),
-                           ndim_sep ? dims_h : dims_t, ndim_sep ? str_h : str_t,
-                           ndim_sep ? box_h : box_t, ones, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                           CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) {
-      set_last_cuda_error(cudaErrorInvalidValue, "cuTensorMapEncodeTiled");
-      return B200NA_ERR_CUDA;
-    }
-    return B200NA_OK;
+    return encode_tiled(tm, tma_type_of(dtype), 5, base, ndim_sep ? dims_h : dims_t,
+                        ndim_sep ? str_h : str_t, ndim_sep ? box_h : box_t, ones);
   }
   if (ndim_sep > 0) {
     // Head dim below the kernel's: the head becomes an axis of its own, (D, H, then the ndim_sep
@@ -1323,14 +1334,7 @@ int make_tensor_map_direct(CUtensorMap* tm, const void* ptr, int dtype, int B, c
       strides[1 + ndim_sep] = row * tokens;
     }
     for (int a = ndim_sep + 1; a < 3; ++a) strides[1 + a] = row * tokens * (cuuint64_t)B;  // extent 1
-    const CUresult r = enc(tm, tma_type_of(dtype), 5, const_cast<void*>(ptr), dims, strides, box,
-                           estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                           CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) {
-      set_last_cuda_error(cudaErrorInvalidValue, "cuTensorMapEncodeTiled");
-      return B200NA_ERR_CUDA;
-    }
-    return B200NA_OK;
+    return encode_tiled(tm, tma_type_of(dtype), 5, ptr, dims, strides, box, estr);
   }
   // bytes from one token to the next: H * D elements when the tensor is contiguous, more when it
   // is a view into a wider row (q, k or v inside a fused [.., 3, H, D] projection output)
@@ -1346,14 +1350,7 @@ int make_tensor_map_direct(CUtensorMap* tm, const void* ptr, int dtype, int B, c
     estr[1 + a] = (cuuint32_t)dil[a];
     if (box[1 + a] > 256 || estr[1 + a] > 8) return B200NA_ERR_UNSUPPORTED;
   }
-  const CUresult r = enc(tm, tma_type_of(dtype), 5, const_cast<void*>(ptr), dims, strides, box,
-                         estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                         CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS) {
-    set_last_cuda_error(cudaErrorInvalidValue, "cuTensorMapEncodeTiled");
-    return B200NA_ERR_CUDA;
-  }
-  return B200NA_OK;
+  return encode_tiled(tm, tma_type_of(dtype), 5, ptr, dims, strides, box, estr);
 }
 
 template <int D, int kType>

@@ -2,6 +2,10 @@
 1-D layouts folded into tensor-map axes, narrow head dims in the backward, layers as one autograd
 node, column sums. Against the oracle with the 16-bit tolerance of the other files (2e-2 of the
 largest entry), or against the Python front."""
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 import torch
@@ -194,3 +198,32 @@ def test_dense_attention_over_parts_of_the_keys(B, nq, nk, hq, hkv, D, dtype):
     assert (lse.double() - s.logsumexp(-1)).abs().max() <= 1e-3
     again, lse2 = torch.compile(lambda a, b, c: nb.attention(a, b, c, return_lse=True))(q, k, v)
     assert torch.equal(again, out) and torch.equal(lse2, lse)
+
+
+FIRST_CALL = """
+import sys, threading, torch, natten_b200 as nb
+q = torch.randn(1, 24, 40, 2, 128, device="cuda").bfloat16().requires_grad_()
+k, v, g = (torch.randn_like(q) for _ in range(3))
+pool = [torch.empty(n, device="cuda") for n in (10, 1000, 100000, 1 << 20) for _ in range(8)]
+del pool                      # cached memory: nothing below has to ask the driver for any
+out = nb.na2d(q, k, v, (7, 9))
+torch.cuda.synchronize()
+out.backward(g)               # the first GPU work of the engine's thread
+want, got = q.grad.clone(), []
+def work():                   # the first GPU work of this thread, its backward in the engine's
+    got.append(nb.na2d(q, k, v, (7, 9)))
+    got.extend(torch.autograd.grad(got[0], q, g))
+thread = threading.Thread(target=work)
+thread.start(); thread.join()
+assert torch.equal(got[0], out) and torch.equal(got[1], want)
+print("done")
+"""
+
+
+def test_first_gpu_work_of_a_thread():
+    """A thread that has not called the CUDA runtime has no current context, and encoding a tensor map
+    needs one."""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(nb.__file__)))
+    r = subprocess.run([sys.executable, "-c", FIRST_CALL], cwd=root, capture_output=True, text=True,
+                       timeout=300)
+    assert r.returncode == 0 and r.stdout.strip() == "done", r.stderr[-2000:]
