@@ -1687,6 +1687,8 @@ int fna_direct_impl(const void* q, const void* k, const void* v, void* o, float*
                     bool views = false) {
   if (!q || !k || !v || !o || !shape || !kernel || !q_tile || !kv_tile)
     return B200NA_ERR_INVALID_ARGUMENT;
+  for (int i = 0; token_strides && i < 3; ++i)   // as the backward: 0 = contiguous, nothing else below H D
+    if (token_strides[i] < 0) return B200NA_ERR_INVALID_ARGUMENT;
   // slabs: q / o / lse hold layout coordinates [q_origin, q_origin + q_extent), k / v hold
   // [kv_origin, kv_origin + kv_extent); window arithmetic stays in layout coordinates
   const bool sharded = q_origin || q_extent || kv_origin || kv_extent;

@@ -491,22 +491,24 @@ bool reads_natively(int dt, int D) {
 
 // Elements between consecutive tokens of a heads-last tensor whose tokens (batch entries included)
 // are evenly spaced and whose [H, D] block is contiguous; -1 when it is not of that form or not
-// aligned for a tensor map.
+// aligned for a tensor map. The stride of an axis of one entry means nothing and is not looked at:
+// [B, 1, N, D] transposed to [B, N, 1, D] has a head stride of N D.
 long long token_stride(const Tensor& t) {
   const int n = (int)t.dim();
   const int64_t H = t.size(n - 2), D = t.size(n - 1);
-  if (t.stride(n - 1) != 1 || t.stride(n - 2) != D) return -1;
-  const int64_t ts = t.stride(n - 3);
-  int64_t expected = ts;
+  if ((D != 1 && t.stride(n - 1) != 1) || (H != 1 && t.stride(n - 2) != D)) return -1;
+  int64_t ts = H * D, expected = -1;
   for (int i = n - 3; i >= 0; --i) {
-    if (t.size(i) != 1 && t.stride(i) != expected) return -1;
+    if (t.size(i) == 1) continue;
+    if (expected < 0) ts = expected = t.stride(i);   // innermost axis of more than one token
+    if (t.stride(i) != expected) return -1;
     expected *= t.size(i);
   }
   if (ts < H * D || (ts * t.element_size()) % 16 || reinterpret_cast<uintptr_t>(t.data_ptr()) % 16)
     return -1;
   return ts;
 }
-// a token-strided tensor (a copy when it is not one) and its stride
+// a token-strided tensor (a contiguous one when it is not) and its stride, 0 = contiguous
 struct View {
   Tensor t;
   long long ts;
@@ -514,8 +516,7 @@ struct View {
 View as_view(const Tensor& t) {
   const long long ts = token_stride(t);
   if (ts >= 0) return {t, ts};
-  Tensor c = t.contiguous();
-  return {c, token_stride(c)};
+  return {t.contiguous(), 0};
 }
 
 struct Sizes {

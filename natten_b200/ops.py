@@ -129,14 +129,18 @@ def token_stride(t: Tensor) -> int:
     """Elements between consecutive tokens of a heads-last ``[B, *X, H, D]`` tensor whose tokens
     (batch entries included) are evenly spaced and whose ``[H, D]`` block is contiguous - true for
     contiguous tensors and for q / k / v sliced out of a fused ``[B, *X, 3, H, D]`` projection.
-    -1 when the tensor is not of that form (or not aligned for a tensor map)."""
+    -1 when the tensor is not of that form (or not aligned for a tensor map). The stride of an axis
+    of one entry means nothing and is not looked at."""
     H, D = t.shape[-2], t.shape[-1]
-    if t.stride(-1) != 1 or t.stride(-2) != D:
+    if (D != 1 and t.stride(-1) != 1) or (H != 1 and t.stride(-2) != D):
         return -1
-    ts = t.stride(-3)
-    expected = ts
+    ts, expected = H * D, None
     for i in range(t.dim() - 3, -1, -1):
-        if t.shape[i] != 1 and t.stride(i) != expected:
+        if t.shape[i] == 1:
+            continue
+        if expected is None:                # innermost axis of more than one token
+            ts = expected = t.stride(i)
+        if t.stride(i) != expected:
             return -1
         expected *= t.shape[i]
     if ts < H * D or (ts * t.element_size()) % 16 != 0 or t.data_ptr() % 16 != 0:
@@ -196,7 +200,7 @@ def na_forward_direct(query: Tensor, key: Tensor, value: Tensor,
     if min(strides) < 0:
         query, key, value = (t if s >= 0 else t.contiguous()
                              for t, s in zip((query, key, value), strides))
-        strides = [token_stride(t) for t in (query, key, value)]
+        strides = [max(s, 0) for s in strides]     # 0: contiguous
     out, lse = _attn_fake(query)
     na_dim = query.dim() - 3
     n_extra = additional_keys.shape[1] if additional_keys is not None else 0

@@ -105,3 +105,18 @@ def test_merge_and_simt_reject_bad_arguments():
              L.F32, 1.0, None, None, 0, None) == L.ERR_UNSUPPORTED
     assert f(one, one, one, one, None, 1, L.ints([8]), L.ints([3]), None, None, None, 1, 1, 1, 8,
              L.F32, 1.0, None, None, 3, None) == L.ERR_INVALID_ARGUMENT  # extra KV without tensors
+
+
+def test_both_directions_agree_on_what_a_token_stride_is():
+    """0 is contiguous; a negative stride is refused by the forward and by the backward, before any
+    CUDA call."""
+    one = ctypes.c_void_p(1024)
+    geometry = [1] + [L.ints(x) for x in ([512], [64], [1], [1], [0], [128], [128])]
+    sizes = [1, 2, 1, 64, L.BF16, 0.125]
+    for i in range(3):
+        ts = [-1 if j == i else 0 for j in range(3)]
+        for f in (L.lib.b200na_na_forward_direct_strided, L.lib.b200na_na_forward_view):
+            assert f(one, one, one, None, None, 0, one, None, *geometry, *sizes, *ts,
+                     None) == L.ERR_INVALID_ARGUMENT
+        assert L.lib.b200na_na_backward_view(*[one] * 6, None, None, 0, one, one, one, None, None, one,
+                                             *geometry, *sizes, *ts, 0, 0, 0, None) == L.ERR_INVALID_ARGUMENT

@@ -227,3 +227,30 @@ def test_first_gpu_work_of_a_thread():
     r = subprocess.run([sys.executable, "-c", FIRST_CALL], cwd=root, capture_output=True, text=True,
                        timeout=300)
     assert r.returncode == 0 and r.stdout.strip() == "done", r.stderr[-2000:]
+
+
+def _fresh(t):
+    """The same values in standard strides (clone() would keep the odd ones)."""
+    return torch.empty(t.shape, dtype=t.dtype, device=t.device).copy_(t)
+
+
+@pytest.mark.parametrize("op,hq,hkv,D", [("na", 4, 1, 64), ("na", 1, 1, 128), ("na", 1, 1, 40),
+                                         ("attention", 4, 1, 64), ("attention", 1, 1, 128)])
+def test_one_head_in_heads_first_layout(op, hq, hkv, D):
+    """[B, 1, N, D].transpose(1, 2) counts as contiguous, with a head stride that is not D: the same
+    results as from standard strides, forward and backward."""
+    torch.manual_seed(67)
+    q = torch.randn(2, hq, 200, D, device="cuda").bfloat16().transpose(1, 2)
+    k, v = (torch.randn(2, hkv, 200, D, device="cuda").bfloat16().transpose(1, 2) for _ in range(2))
+    assert k.is_contiguous() and k.stride(2) != D
+    d_out = torch.randn(2, 200, hq, D, device="cuda").bfloat16()
+    fn = (lambda *a: nb.na1d(*a, 33)) if op == "na" else nb.attention
+    results = []
+    for leaves in ([q, k, v], [_fresh(t) for t in (q, k, v)]):
+        leaves = [t.detach().requires_grad_() for t in leaves]
+        out = fn(*leaves)
+        assert "NaFunction" in out.grad_fn.name()
+        results.append([out.detach(), *torch.autograd.grad(out, leaves, d_out)])
+    assert L.device_status() == 0
+    for a, b in zip(*results):
+        assert torch.equal(a, b)

@@ -131,3 +131,13 @@ def test_operators_trace_into_one_graph_without_breaks(monkeypatch, dynamic):
         return nb.token_unpermute_operation(p, layout, (8, 8), (2, 1))
     assert _traced_ops(permute_roundtrip, q, dynamic=False) == [
         "natten_b200::token_permute", "natten_b200::token_unpermute"]
+
+
+def test_token_stride_of_axes_with_one_entry():
+    one_head = torch.empty(2, 1, 30, 64, dtype=torch.bfloat16).transpose(1, 2)
+    assert one_head.is_contiguous() and one_head.stride(2) != 64
+    assert ops.token_stride(one_head) == 64
+    assert ops.token_stride(torch.empty(1, 30, 3, 1, 64, dtype=torch.bfloat16)[:, :, 0]) == 192
+    assert ops.token_stride(torch.empty(2, 2, 30, 64, dtype=torch.bfloat16).transpose(1, 2)) == -1
+    assert ops.token_stride(torch.empty(2, 30, 2, 64, dtype=torch.bfloat16)[:, ::2, :, :]) == 256
+    assert ops.token_stride(torch.empty(2, 31, 2, 64, dtype=torch.bfloat16)[:, :30]) == -1
