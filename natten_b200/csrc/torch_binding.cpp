@@ -519,6 +519,14 @@ View as_view(const Tensor& t) {
   return {t.contiguous(), 0};
 }
 
+// A contiguous tensor on a 16-byte boundary, as the tensor-core backward and the column sums read an
+// output gradient. A piece of a flat buffer (split, cat's backward) is contiguous wherever it starts.
+Tensor aligned(const Tensor& t) {
+  Tensor c = t.contiguous();
+  if (reinterpret_cast<uintptr_t>(c.data_ptr()) % 16 != 0) c = c.clone(at::MemoryFormat::Contiguous);
+  return c;
+}
+
 struct Sizes {
   int B, Hq, Hkv, D, dt;
 };
@@ -747,7 +755,7 @@ struct NaFunction : torch::autograd::Function<NaFunction> {
     } else {
       qv = {q.contiguous(), 0}; kv = {k.contiguous(), 0}; vv = {v.contiguous(), 0};
     }
-    const Tensor d_out = d_out_.contiguous();
+    const Tensor d_out = tc ? aligned(d_out_) : d_out_.contiguous();
     const Tensor dq = at::empty(q.sizes(), q.options()), dk = at::empty(k.sizes(), q.options()),
                  dv = at::empty(k.sizes(), q.options());
     Tensor akc, avc, dak, dav;
@@ -842,7 +850,7 @@ struct LayerFunction : torch::autograd::Function<LayerFunction> {
       c10::impl::ExcludeDispatchKeyGuard no_autocast(c10::DispatchKey::AutocastCUDA);
       c10::cuda::CUDAGuard guard(x.device());
       const int64_t E = x.size(-1), T = x.numel() / E;
-      const Tensor dy = grads[0].contiguous().view({T, E});
+      const Tensor dy = aligned(grads[0]).view({T, E});
       if (need_w2) g[2] = at::mm(dy.t(), attn.view({T, E}));
       if (need_b2) g[b2_at] = column_sum(dy, c.z.dt);
       if (need_x || need_w1 || need_b1) {

@@ -325,6 +325,8 @@ def na_backward_direct(query: Tensor, key: Tensor, value: Tensor, out: Tensor, d
                        ) -> Tuple[Tensor, Tensor, Tensor, Tensor, Tensor]:
     """dQ, dK, dV and the extra tokens' gradients (empty tensors when there are none) on tensor
     cores (fp16/bf16, head dim 64/128), caller's layout."""
+    if d_out.data_ptr() % 16:     # contiguous, but a piece of a flat buffer: tensor maps need 16 bytes
+        d_out = d_out.clone()
     dq, dk, dv, dak, dav = _na_backward_direct_fake(
         query, key, value, out, d_out, lse, additional_keys, additional_values, kernel_size,
         stride, dilation, is_causal, scale, q_tile_shape, kv_tile_shape)

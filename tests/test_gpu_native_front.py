@@ -254,3 +254,43 @@ def test_one_head_in_heads_first_layout(op, hq, hkv, D):
     assert L.device_status() == 0
     for a, b in zip(*results):
         assert torch.equal(a, b)
+
+
+
+def _off_16_bytes(t):
+    """The same values one element behind a 16-byte boundary, contiguous."""
+    u = torch.empty(t.numel() + 1, dtype=t.dtype, device=t.device)[1:].view(t.shape).copy_(t)
+    assert u.is_contiguous() and u.data_ptr() % 16
+    return u
+
+
+@pytest.mark.parametrize("case", ["attention", "attention-narrow", "narrow", "folded", "layer"])
+def test_output_gradient_off_16_bytes(case):
+    """A piece of a flat buffer: autograd passes it on as it is."""
+    torch.manual_seed(71)
+    if case == "layer":
+        layer = nb.NeighborhoodAttention2D(96, 3, 5).cuda().bfloat16()
+        x = torch.randn(2, 14, 17, 96, device="cuda").bfloat16().requires_grad_()
+        wrt, fn = [x, *layer.parameters()], lambda: layer(x)
+    else:
+        D = 24 if case in ("narrow", "attention-narrow") else 64
+        tokens = (12, 13) if case == "narrow" else (150,)
+        wrt = [torch.randn(2, *tokens, 2, D, device="cuda").bfloat16().requires_grad_() for _ in range(3)]
+        fn = {"narrow": lambda: nb.na2d(*wrt, 5), "folded": lambda: nb.na1d(*wrt, 9, dilation=5)}.get(
+            case, lambda: nb.attention(*wrt))
+    d_out = torch.randn_like(fn())
+    want = torch.autograd.grad(fn(), wrt, d_out)
+    got = torch.autograd.grad(fn(), wrt, _off_16_bytes(d_out))
+    assert L.device_status() == 0
+    for a, b in zip(got, want):
+        assert torch.equal(a, b)
+
+
+def test_compiled_backward_with_an_output_gradient_off_16_bytes():
+    torch.manual_seed(71)
+    wrt = [torch.randn(2, 150, 2, 64, device="cuda").bfloat16().requires_grad_() for _ in range(3)]
+    out = torch.compile(nb.attention)(*wrt)
+    d_out = torch.randn_like(out)
+    want = torch.autograd.grad(out, wrt, d_out, retain_graph=True)
+    for a, b in zip(torch.autograd.grad(out, wrt, _off_16_bytes(d_out)), want):
+        assert torch.equal(a, b)
