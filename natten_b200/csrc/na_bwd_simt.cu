@@ -40,111 +40,137 @@ struct BwdSmem {
 };
 
 // out0 = dQ or dK, out1 = dV.
-template <class T, int DM, bool kVec, bool kKeyRows>
-__global__ void __launch_bounds__(kThreads) na_bwd_kernel(
-    const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v,
-    const T* __restrict__ o, const T* __restrict__ d_out, const float* __restrict__ lse,
-    float* __restrict__ delta, const T* __restrict__ add_k, const T* __restrict__ add_v,
-    T* __restrict__ out0, T* __restrict__ out1, const Params p) {
-  extern __shared__ __align__(16) uint8_t smem_raw[];
-  using SM = BwdSmem<DM, kKeyRows>;
-  SM& sm = *reinterpret_cast<SM*>(smem_raw);
+template <class T>
+struct BwdTensors {
+  const T *q, *k, *v, *o, *d_out;
+  const float* lse;
+  float* delta;
+  const T *add_k, *add_v;
+  T *out0, *out1;
+};
+
+// One item: the block's 32 rows, decoded in sm.rows, against their columns. False if the sums are not
+// finite and nothing was stored; kAgain: stored in any case (see simt_tile.cuh).
+template <class T, int DM, bool kVec, bool kKeyRows, bool kAgain>
+__device__ __forceinline__ bool gradients(BwdSmem<DM, kKeyRows>& sm, const BwdTensors<T>& x,
+                                          const Params& p) {
   const int tid = threadIdx.x;
   const int rg = tid >> 4, cl = tid & 15;
   const int nd = p.ax.ndim;
   const int dp = (p.D + 3) & ~3;
-
-  for (int64_t item = blockIdx.x; item < p.n_items; item += gridDim.x) {
-    __syncthreads();                 // the previous item's readers are done
-    if (tid < kRows) decode_rows<kKeyRows>(p, item, sm.rows);
+  int64_t n_tok = (int64_t)sm.rows.box_len[0] * sm.rows.box_len[1] * sm.rows.box_len[2];
+  int64_t n_all = n_tok;
+  if (kKeyRows) n_all = n_tok = n_tok * (p.Hq / p.Hkv);
+  else if (n_tok > 0) n_all += p.n_extra;
+  if (tid < kCols) decode_col<kKeyRows>(p, sm.rows, n_tok, n_all, tid, sm.cols[0], tid);
+  float row_lse[4], row_delta[4];
+  if (kKeyRows) {
+    load_rows<T, DM, kVec, kRows>(sm.r1, p.extra_rows ? x.add_k : x.k, sm.rows.row, p.D);
+    load_rows<T, DM, kVec, kRows>(sm.r2, p.extra_rows ? x.add_v : x.v, sm.rows.row, p.D);
+  } else {
+    load_rows<T, DM, kVec, kRows>(sm.r1, x.q, sm.rows.row, p.D);
+    load_rows<T, DM, kVec, kRows>(sm.r2, x.d_out, sm.rows.row, p.D);
+    load_rows<T, DM, kVec, kRows>(sm.c1, x.o, sm.rows.row, p.D);
     __syncthreads();
-    int64_t n_tok = (int64_t)sm.rows.box_len[0] * sm.rows.box_len[1] * sm.rows.box_len[2];
-    int64_t n_all = n_tok;
-    if (kKeyRows) n_all = n_tok = n_tok * (p.Hq / p.Hkv);
-    else if (n_tok > 0) n_all += p.n_extra;
-    if (tid < kCols) decode_col<kKeyRows>(p, sm.rows, n_tok, n_all, tid, sm.cols[0], tid);
-    float row_lse[4], row_delta[4];
-    if (kKeyRows) {
-      load_rows<T, DM, kVec, kRows>(sm.r1, p.extra_rows ? add_k : k, sm.rows.row, p.D);
-      load_rows<T, DM, kVec, kRows>(sm.r2, p.extra_rows ? add_v : v, sm.rows.row, p.D);
-    } else {
-      load_rows<T, DM, kVec, kRows>(sm.r1, q, sm.rows.row, p.D);
-      load_rows<T, DM, kVec, kRows>(sm.r2, d_out, sm.rows.row, p.D);
-      load_rows<T, DM, kVec, kRows>(sm.c1, o, sm.rows.row, p.D);
-      __syncthreads();
-#pragma unroll
-      for (int r = 0; r < 4; ++r) {
-        const int64_t row = sm.rows.row[rg * 4 + r];
-        float part = 0.f;
-        for (int d = cl; d < p.D; d += 16)
-          part = fmaf(sm.r2[(rg * 4 + r) * (DM + 4) + d], sm.c1[(rg * 4 + r) * (DM + 4) + d], part);
-        row_delta[r] = row_sum(part);
-        row_lse[r] = row >= 0 ? lse[row] : 0.f;
-        if (row >= 0 && cl == 0) delta[row] = row_delta[r];
-      }
-    }
-
-    float acc0[4][OutCols<DM>::kPer], acc1[kKeyRows ? 4 : 1][OutCols<DM>::kPer];
-#pragma unroll
-    for (int r = 0; r < 4; ++r)
-#pragma unroll
-      for (int t = 0; t < OutCols<DM>::kPer; ++t) {
-        acc0[r][t] = 0.f;
-        if (kKeyRows) acc1[kKeyRows ? r : 0][t] = 0.f;
-      }
-    int buf = 0;
-    for (int64_t j0 = 0; j0 < n_all; j0 += kCols, buf ^= 1) {
-      __syncthreads();               // this step's column table is written, the last tiles are read
-      const Cols& cols = sm.cols[buf];
-      if (kKeyRows) {
-        load_rows<T, DM, kVec, kCols>(sm.c1, q, cols.row, p.D);
-        load_rows<T, DM, kVec, kCols>(sm.c2, d_out, cols.row, p.D);
-        if (tid < kCols) {
-          const int64_t row = cols.row[tid];
-          sm.lse[tid] = row >= 0 ? lse[row] : 0.f;
-          sm.delta[tid] = row >= 0 ? delta[row] : 0.f;
-        }
-      } else {
-        load_key_values<T, DM, kVec>(p, sm.rows, cols, j0, n_tok, n_all, sm.c1, sm.c2, k, v, add_k,
-                                     add_v);
-      }
-      if (tid < kCols && j0 + kCols < n_all)
-        decode_col<kKeyRows>(p, sm.rows, n_tok, n_all, j0 + kCols + tid, sm.cols[buf ^ 1], tid);
-      __syncthreads();
-
-      float s[4][4], dpv[4][4];
-#pragma unroll
-      for (int r = 0; r < 4; ++r)
-#pragma unroll
-        for (int i = 0; i < 4; ++i) s[r][i] = dpv[r][i] = 0.f;
-      dot_tile<DM>(sm.r1, sm.c1, rg, cl, dp, s);
-      dot_tile<DM>(sm.r2, sm.c2, rg, cl, dp, dpv);
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int4 cc = cols.c[cl + 16 * i];
-        const float cl_lse = kKeyRows ? sm.lse[cl + 16 * i] : 0.f;
-        const float cl_delta = kKeyRows ? sm.delta[cl + 16 * i] : 0.f;
-#pragma unroll
-        for (int r = 0; r < 4; ++r) {
-          const bool on = pair_on(sm.rows, rg * 4 + r, cc, nd);
-          const float pj = on ? expf(s[r][i] * p.scale - (kKeyRows ? cl_lse : row_lse[r])) : 0.f;
-          const int at = (rg * 4 + r) * kPStride + cl + 16 * i;
-          sm.ds[at] = p.scale * pj * (dpv[r][i] - (kKeyRows ? cl_delta : row_delta[r]));
-          if (kKeyRows) sm.pr[at] = pj;
-        }
-      }
-      __syncwarp();                  // these rows are read by the warp that wrote them
-      const int n4 = (int)min((int64_t)kCols, (n_all - j0 + 3) & ~(int64_t)3);
-      accumulate_tile<DM>(sm.ds, sm.c1, rg, cl, n4, acc0);
-      if constexpr (kKeyRows) accumulate_tile<DM>(sm.pr, sm.c2, rg, cl, n4, acc1);
-    }
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
       const int64_t row = sm.rows.row[rg * 4 + r];
-      if (row < 0) continue;
-      store_row<T, DM>(out0 + row * p.D, acc0[r], 1.f, cl, p.D);
-      if constexpr (kKeyRows) store_row<T, DM>(out1 + row * p.D, acc1[r], 1.f, cl, p.D);
+      float part = 0.f;
+      for (int d = cl; d < p.D; d += 16)
+        part = fmaf(sm.r2[(rg * 4 + r) * (DM + 4) + d], sm.c1[(rg * 4 + r) * (DM + 4) + d], part);
+      row_delta[r] = row_sum(part);
+      row_lse[r] = row >= 0 ? x.lse[row] : 0.f;
+      if (row >= 0 && cl == 0) x.delta[row] = row_delta[r];
     }
+  }
+
+  float acc0[4][OutCols<DM>::kPer], acc1[4][kKeyRows ? OutCols<DM>::kPer : 1];
+#pragma unroll
+  for (int r = 0; r < 4; ++r)
+#pragma unroll
+    for (int t = 0; t < OutCols<DM>::kPer; ++t) {
+      acc0[r][t] = 0.f;
+      acc1[r][kKeyRows ? t : 0] = 0.f;
+    }
+  int buf = 0;
+  for (int64_t j0 = 0; j0 < n_all; j0 += kCols, buf ^= 1) {
+    __syncthreads();               // this step's column table is written, the last tiles are read
+    const Cols& cols = sm.cols[buf];
+    if (kKeyRows) {
+      load_rows<T, DM, kVec, kCols>(sm.c1, x.q, cols.row, p.D);
+      load_rows<T, DM, kVec, kCols>(sm.c2, x.d_out, cols.row, p.D);
+      if (tid < kCols) {
+        const int64_t row = cols.row[tid];
+        sm.lse[tid] = row >= 0 ? x.lse[row] : 0.f;
+        sm.delta[tid] = row >= 0 ? x.delta[row] : 0.f;
+      }
+    } else {
+      load_key_values<T, DM, kVec>(p, sm.rows, cols, j0, n_tok, n_all, sm.c1, sm.c2, x.k, x.v,
+                                   x.add_k, x.add_v);
+    }
+    if (tid < kCols && j0 + kCols < n_all)
+      decode_col<kKeyRows>(p, sm.rows, n_tok, n_all, j0 + kCols + tid, sm.cols[buf ^ 1], tid);
+    __syncthreads();
+
+    float s[4][4], dpv[4][4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) s[r][i] = dpv[r][i] = 0.f;
+    dot_tile<DM>(sm.r1, sm.c1, rg, cl, dp, s);
+    dot_tile<DM>(sm.r2, sm.c2, rg, cl, dp, dpv);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int4 cc = cols.c[cl + 16 * i];
+      const float cl_lse = kKeyRows ? sm.lse[cl + 16 * i] : 0.f;
+      const float cl_delta = kKeyRows ? sm.delta[cl + 16 * i] : 0.f;
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        const bool on = pair_on(sm.rows, rg * 4 + r, cc, nd);
+        const float pj = on ? expf(s[r][i] * p.scale - (kKeyRows ? cl_lse : row_lse[r])) : 0.f;
+        const float ds = p.scale * pj * (dpv[r][i] - (kKeyRows ? cl_delta : row_delta[r]));
+        const int at = (rg * 4 + r) * kPStride + cl + 16 * i;
+        sm.ds[at] = kAgain ? weight_if(on, ds) : ds;
+        if (kKeyRows) sm.pr[at] = kAgain ? weight_if(on, pj) : pj;
+      }
+    }
+    __syncwarp();                  // these rows are read by the warp that wrote them
+    const int n4 = (int)min((int64_t)kCols, (n_all - j0 + 3) & ~(int64_t)3);
+    if constexpr (kAgain) {
+      accumulate_interacting<DM>(sm.ds, sm.c1, rg, cl, n4, acc0);
+      if constexpr (kKeyRows) accumulate_interacting<DM>(sm.pr, sm.c2, rg, cl, n4, acc1);
+    } else {
+      accumulate_tile<DM>(sm.ds, sm.c1, rg, cl, n4, acc0);
+      if constexpr (kKeyRows) accumulate_tile<DM>(sm.pr, sm.c2, rg, cl, n4, acc1);
+    }
+  }
+  if (!kAgain && __syncthreads_or(any_non_finite(acc0) || any_non_finite(acc1))) return false;
+#pragma unroll
+  for (int r = 0; r < 4; ++r) {
+    const int64_t row = sm.rows.row[rg * 4 + r];
+    if (row < 0) continue;
+    store_row<T, DM>(x.out0 + row * p.D, acc0[r], 1.f, cl, p.D);
+    if constexpr (kKeyRows) store_row<T, DM>(x.out1 + row * p.D, acc1[r], 1.f, cl, p.D);
+  }
+  return true;
+}
+template <class T, int DM, bool kVec, bool kKeyRows>
+__device__ __noinline__ void gradients_again(BwdSmem<DM, kKeyRows>& sm, const BwdTensors<T>& x,
+                                             const Params& p) {
+  gradients<T, DM, kVec, kKeyRows, true>(sm, x, p);
+}
+
+template <class T, int DM, bool kVec, bool kKeyRows>
+__global__ void __launch_bounds__(kThreads, bwd_blocks(DM)) na_bwd_kernel(
+    const __grid_constant__ BwdTensors<T> x, const __grid_constant__ Params p) {
+  extern __shared__ __align__(16) uint8_t smem_raw[];
+  using SM = BwdSmem<DM, kKeyRows>;
+  SM& sm = *reinterpret_cast<SM*>(smem_raw);
+  for (int64_t item = blockIdx.x; item < p.n_items; item += gridDim.x) {
+    __syncthreads();                 // the previous item's readers are done
+    if (threadIdx.x < kRows) decode_rows<kKeyRows>(p, item, sm.rows);
+    __syncthreads();
+    if (!gradients<T, DM, kVec, kKeyRows, false>(sm, x, p)) gradients_again<T, DM, kVec, kKeyRows>(sm, x, p);
   }
 }
 
@@ -177,11 +203,11 @@ int launch_bwd_dm(BwdPointers& a, const Params& base, cudaStream_t stream) {
       for (int x = 0; x < B200NA_MAX_DIM; ++x) p.ax.dilation[x] = 1;
     }
     plan_rows(p);
-    void* out0 = pass == 0 ? a.dq : (pass == 1 ? a.dk : a.d_add_k);
-    void* out1 = pass == 0 ? nullptr : (pass == 1 ? a.dv : a.d_add_v);
-    void* args[] = {(void*)&a.q, (void*)&a.k, (void*)&a.v, (void*)&a.o, (void*)&a.d_out,
-                    (void*)&a.lse, (void*)&a.delta, (void*)&a.add_k, (void*)&a.add_v, (void*)&out0,
-                    (void*)&out1, (void*)&p};
+    BwdTensors<T> x = {(const T*)a.q, (const T*)a.k, (const T*)a.v, (const T*)a.o,
+                       (const T*)a.d_out, a.lse, a.delta, (const T*)a.add_k, (const T*)a.add_v,
+                       (T*)(pass == 0 ? a.dq : (pass == 1 ? a.dk : a.d_add_k)),
+                       (T*)(pass == 0 ? nullptr : (pass == 1 ? a.dv : a.d_add_v))};
+    void* args[] = {(void*)&x, (void*)&p};
     const int rc = simt::launch(pass == 0 ? fn_q : fn_k, p.n_items,
                                 (int)(pass == 0 ? sizeof(BwdSmem<DM, false>)
                                                 : sizeof(BwdSmem<DM, true>)), args, stream);

@@ -37,89 +37,109 @@ struct FwdSmem {
   Rows rows;
 };
 
-template <class T, int DM, bool kVec>
-__global__ void __launch_bounds__(kThreads) na_simt_kernel(
-    const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v, T* __restrict__ o,
-    float* __restrict__ lse, const T* __restrict__ add_k, const T* __restrict__ add_v,
-    const Params p) {
-  extern __shared__ __align__(16) uint8_t smem_raw[];
-  FwdSmem<DM>& sm = *reinterpret_cast<FwdSmem<DM>*>(smem_raw);
+template <class T>
+struct FwdTensors {
+  const T *q, *k, *v;
+  T* o;
+  float* lse;
+  const T *add_k, *add_v;
+};
+
+// One item: the block's 32 queries, decoded in sm.rows and loaded in sm.q, against their keys. False if
+// the sums are not finite and nothing was stored; kAgain: stored in any case (see simt_tile.cuh).
+template <class T, int DM, bool kVec, bool kAgain>
+__device__ __forceinline__ bool attend(FwdSmem<DM>& sm, const FwdTensors<T>& x, const Params& p) {
   const int tid = threadIdx.x;
   const int rg = tid >> 4, cl = tid & 15;
   const int nd = p.ax.ndim;
   const int dp = (p.D + 3) & ~3;
+  const int64_t n_tok = (int64_t)sm.rows.box_len[0] * sm.rows.box_len[1] * sm.rows.box_len[2];
+  const int64_t n_all = n_tok > 0 ? n_tok + p.n_extra : 0;   // no columns: padding rows only
+  if (tid < kCols) decode_col<false>(p, sm.rows, n_tok, n_all, tid, sm.cols[0], tid);
+  if (!kAgain) load_rows<T, DM, kVec, kRows>(sm.q, x.q, sm.rows.row, p.D);
 
+  float m[4], sum[4], acc[4][OutCols<DM>::kPer];
+#pragma unroll
+  for (int r = 0; r < 4; ++r) {
+    m[r] = -INFINITY;
+    sum[r] = 0.f;
+#pragma unroll
+    for (int t = 0; t < OutCols<DM>::kPer; ++t) acc[r][t] = 0.f;
+  }
+  int buf = 0;
+  for (int64_t j0 = 0; j0 < n_all; j0 += kCols, buf ^= 1) {
+    __syncthreads();               // this step's column table is written, the last tiles are read
+    const Cols& cols = sm.cols[buf];
+    load_key_values<T, DM, kVec>(p, sm.rows, cols, j0, n_tok, n_all, sm.k, sm.v, x.k, x.v, x.add_k,
+                                 x.add_v);
+    if (tid < kCols && j0 + kCols < n_all)
+      decode_col<false>(p, sm.rows, n_tok, n_all, j0 + kCols + tid, sm.cols[buf ^ 1], tid);
+    __syncthreads();
+
+    float s[4][4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) s[r][i] = 0.f;
+    dot_tile<DM>(sm.q, sm.k, rg, cl, dp, s);
+    int4 cc[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) cc[i] = cols.c[cl + 16 * i];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      float mx = -INFINITY;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        s[r][i] = pair_on(sm.rows, rg * 4 + r, cc[i], nd) ? s[r][i] * p.scale : -INFINITY;
+        mx = fmaxf(mx, s[r][i]);
+      }
+      const float m_new = fmaxf(m[r], row_max(mx));
+      // a row without a key so far keeps -inf; its exponents must not become NaN
+      const float ref = m_new == -INFINITY ? 0.f : m_new;
+      const float corr = expf(m[r] - ref);      // exp(-inf) = 0 on the first keys
+      float part = 0.f;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float pj = expf(s[r][i] - ref);
+        part += pj;
+        sm.w[(rg * 4 + r) * kPStride + cl + 16 * i] =
+            kAgain ? weight_if(pair_on(sm.rows, rg * 4 + r, cc[i], nd), pj) : pj;
+      }
+      sum[r] = sum[r] * corr + row_sum(part);
+      m[r] = m_new;
+#pragma unroll
+      for (int t = 0; t < OutCols<DM>::kPer; ++t) acc[r][t] *= corr;
+    }
+    __syncwarp();                  // P rows are read by the warp that wrote them
+    const int n4 = (int)min((int64_t)kCols, (n_all - j0 + 3) & ~(int64_t)3);
+    if constexpr (kAgain) accumulate_interacting<DM>(sm.w, sm.v, rg, cl, n4, acc);
+    else accumulate_tile<DM>(sm.w, sm.v, rg, cl, n4, acc);
+  }
+  if (!kAgain && __syncthreads_or(any_non_finite(acc))) return false;
+#pragma unroll
+  for (int r = 0; r < 4; ++r) {
+    const int64_t row = sm.rows.row[rg * 4 + r];
+    if (row < 0) continue;
+    store_row<T, DM>(x.o + row * p.D, acc[r], 1.f / sum[r], cl, p.D);
+    if (x.lse && cl == 0) x.lse[row] = logf(sum[r]) + m[r];
+  }
+  return true;
+}
+template <class T, int DM, bool kVec>
+__device__ __noinline__ void attend_again(FwdSmem<DM>& sm, const FwdTensors<T>& x, const Params& p) {
+  attend<T, DM, kVec, true>(sm, x, p);
+}
+
+template <class T, int DM, bool kVec>
+__global__ void __launch_bounds__(kThreads, fwd_blocks(DM)) na_simt_kernel(
+    const __grid_constant__ FwdTensors<T> x, const __grid_constant__ Params p) {
+  extern __shared__ __align__(16) uint8_t smem_raw[];
+  FwdSmem<DM>& sm = *reinterpret_cast<FwdSmem<DM>*>(smem_raw);
   for (int64_t item = blockIdx.x; item < p.n_items; item += gridDim.x) {
     __syncthreads();                 // the previous item's readers are done
-    if (tid < kRows) decode_rows<false>(p, item, sm.rows);
+    if (threadIdx.x < kRows) decode_rows<false>(p, item, sm.rows);
     __syncthreads();
-    const int64_t n_tok = (int64_t)sm.rows.box_len[0] * sm.rows.box_len[1] * sm.rows.box_len[2];
-    const int64_t n_all = n_tok > 0 ? n_tok + p.n_extra : 0;   // no columns: padding rows only
-    if (tid < kCols) decode_col<false>(p, sm.rows, n_tok, n_all, tid, sm.cols[0], tid);
-    load_rows<T, DM, kVec, kRows>(sm.q, q, sm.rows.row, p.D);
-
-    float m[4], sum[4], acc[4][OutCols<DM>::kPer];
-#pragma unroll
-    for (int r = 0; r < 4; ++r) {
-      m[r] = -INFINITY;
-      sum[r] = 0.f;
-#pragma unroll
-      for (int t = 0; t < OutCols<DM>::kPer; ++t) acc[r][t] = 0.f;
-    }
-    int buf = 0;
-    for (int64_t j0 = 0; j0 < n_all; j0 += kCols, buf ^= 1) {
-      __syncthreads();               // this step's column table is written, the last tiles are read
-      const Cols& cols = sm.cols[buf];
-      load_key_values<T, DM, kVec>(p, sm.rows, cols, j0, n_tok, n_all, sm.k, sm.v, k, v, add_k,
-                                   add_v);
-      if (tid < kCols && j0 + kCols < n_all)
-        decode_col<false>(p, sm.rows, n_tok, n_all, j0 + kCols + tid, sm.cols[buf ^ 1], tid);
-      __syncthreads();
-
-      float s[4][4];
-#pragma unroll
-      for (int r = 0; r < 4; ++r)
-#pragma unroll
-        for (int i = 0; i < 4; ++i) s[r][i] = 0.f;
-      dot_tile<DM>(sm.q, sm.k, rg, cl, dp, s);
-      int4 cc[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) cc[i] = cols.c[cl + 16 * i];
-#pragma unroll
-      for (int r = 0; r < 4; ++r) {
-        float mx = -INFINITY;
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          s[r][i] = pair_on(sm.rows, rg * 4 + r, cc[i], nd) ? s[r][i] * p.scale : -INFINITY;
-          mx = fmaxf(mx, s[r][i]);
-        }
-        const float m_new = fmaxf(m[r], row_max(mx));
-        // a row without a key so far keeps -inf; its exponents must not become NaN
-        const float ref = m_new == -INFINITY ? 0.f : m_new;
-        const float corr = expf(m[r] - ref);      // exp(-inf) = 0 on the first keys
-        float part = 0.f;
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const float pj = expf(s[r][i] - ref);
-          part += pj;
-          sm.w[(rg * 4 + r) * kPStride + cl + 16 * i] = pj;
-        }
-        sum[r] = sum[r] * corr + row_sum(part);
-        m[r] = m_new;
-#pragma unroll
-        for (int t = 0; t < OutCols<DM>::kPer; ++t) acc[r][t] *= corr;
-      }
-      __syncwarp();                  // P rows are read by the warp that wrote them
-      const int n4 = (int)min((int64_t)kCols, (n_all - j0 + 3) & ~(int64_t)3);
-      accumulate_tile<DM>(sm.w, sm.v, rg, cl, n4, acc);
-    }
-#pragma unroll
-    for (int r = 0; r < 4; ++r) {
-      const int64_t row = sm.rows.row[rg * 4 + r];
-      if (row < 0) continue;
-      store_row<T, DM>(o + row * p.D, acc[r], 1.f / sum[r], cl, p.D);
-      if (lse && cl == 0) lse[row] = logf(sum[r]) + m[r];
-    }
+    if (!attend<T, DM, kVec, false>(sm, x, p)) attend_again<T, DM, kVec>(sm, x, p);
   }
 }
 
@@ -130,8 +150,8 @@ int launch_dm(const void* q, const void* k, const void* v, void* o, float* lse, 
                               reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v));
   const void* fn = vec ? (const void*)na_simt_kernel<T, DM, true>
                        : (const void*)na_simt_kernel<T, DM, false>;
-  void* args[] = {(void*)&q, (void*)&k, (void*)&v, (void*)&o, (void*)&lse, (void*)&ak, (void*)&av,
-                  (void*)&p};
+  FwdTensors<T> x = {(const T*)q, (const T*)k, (const T*)v, (T*)o, lse, (const T*)ak, (const T*)av};
+  void* args[] = {(void*)&x, (void*)&p};
   return simt::launch(fn, p.n_items, (int)sizeof(FwdSmem<DM>), args, stream);
 }
 template <class T>

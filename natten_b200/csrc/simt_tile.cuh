@@ -26,6 +26,11 @@ constexpr int kCols = 64;      // columns per step
 constexpr int kThreads = 128;
 constexpr int kPStride = kCols + 4;
 constexpr int kMaxD = 256;
+// Blocks per SM of the kernels for head dims up to DM, the registers' share: as many as the shared memory
+// lets in where that is few, so that the function for non-finite columns (accumulate_interacting), which
+// is rarely called, does not raise the registers of all.
+constexpr int fwd_blocks(int DM) { return DM <= 32 ? 5 : (DM <= 64 ? 4 : (DM <= 128 ? 2 : 1)); }
+constexpr int bwd_blocks(int DM) { return DM <= 32 ? 4 : (DM <= 64 ? 3 : 1); }
 
 template <class T> __device__ __forceinline__ float ldf(const T* p);
 template <> __device__ __forceinline__ float ldf<float>(const float* p) { return *p; }
@@ -352,6 +357,43 @@ __device__ __forceinline__ void accumulate_tile(const float* w, const float* col
       }
     }
   }
+}
+// Non-finite columns. A column of the union box is multiplied with every row of the block, by zero where
+// the pair does not interact, and 0 x NaN is NaN: a row would take over the NaN or infinity of a token
+// outside its window. All that can reach a row that way makes its sums non-finite, so a block looks at
+// its finished sums (one multiply-add each) and, if one is not finite, does the item again in a function
+// that is not inlined (kAgain; a 32 x 32 map of 4 heads takes 22.5 us that way, as without the check, and
+// 24.6 us with the second accumulation as a branch inside the loop). There the weights of pairs that do not interact are kNoWeight, which
+// no interacting pair has, and are skipped.
+constexpr unsigned kNoWeight = 0x80000000u;   // -0
+__device__ __forceinline__ float weight_if(bool on, float w) {
+  return on ? w + 0.f : __uint_as_float(kNoWeight);   // -0 + 0 = +0
+}
+template <int DM>
+__device__ __forceinline__ void accumulate_interacting(const float* w, const float* cols, int rg, int cl,
+                                                       int n4, float (&acc)[4][OutCols<DM>::kPer]) {
+  using OC = OutCols<DM>;
+#pragma unroll 1
+  for (int j = 0; j < n4; ++j) {
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      const float f = w[(rg * 4 + r) * kPStride + j];
+      if (__float_as_uint(f) == kNoWeight) continue;
+#pragma unroll
+      for (int t = 0; t < OC::kPer; ++t)
+        acc[r][t] = fmaf(f, cols[j * (DM + 4) + (t / OC::kW) * 16 * OC::kW + cl * OC::kW + t % OC::kW],
+                         acc[r][t]);
+    }
+  }
+}
+template <int kN>
+__device__ __forceinline__ bool any_non_finite(const float (&acc)[4][kN]) {
+  float t = 0.f;
+#pragma unroll
+  for (int r = 0; r < 4; ++r)
+#pragma unroll
+    for (int i = 0; i < kN; ++i) t = fmaf(acc[r][i], 0.f, t);
+  return t != 0.f;   // NaN
 }
 template <class T, int DM>
 __device__ __forceinline__ void store_row(T* dst, const float (&acc)[OutCols<DM>::kPer], float mul,

@@ -294,3 +294,35 @@ def test_compiled_backward_with_an_output_gradient_off_16_bytes():
     want = torch.autograd.grad(out, wrt, d_out, retain_graph=True)
     for a, b in zip(torch.autograd.grad(out, wrt, _off_16_bytes(d_out)), want):
         assert torch.equal(a, b)
+
+
+
+@pytest.mark.parametrize("shape,ks,st,di,ca,hq,hkv,D,n_extra", [
+    ((150,), (40,), (1,), (1,), (True,), 2, 1, 32, 0), ((150,), (33,), (4,), (3,), (False,), 2, 2, 20, 7),
+    ((13, 21), (5, 7), (1, 2), (1, 2), (False, True), 4, 2, 64, 0), ((64,), (64,), (1,), (1,), (True,), 1, 1, 130, 0)])
+@pytest.mark.parametrize("value", [float("nan"), float("inf")])
+def test_fp32_non_finite_tokens_stay_inside_their_windows(shape, ks, st, di, ca, hq, hkv, D, n_extra, value):
+    """One token of q, k, v or the output gradient is NaN or infinite: the rows that attend it (that it
+    attends) are what the oracle makes of them, all others are what they are without it."""
+    torch.manual_seed(73)
+    fn = {1: nb.na1d, 2: nb.na2d}[len(shape)]
+    ops = [torch.randn(1, *shape, h, D) for h in (hq, hkv, hkv, hq)]
+    extras = [torch.randn(1, n_extra, hkv, D) for _ in range(2)] if n_extra else []
+    for which in range(4):
+        for token in (0, 37, 63):
+            poisoned = [t.clone() for t in ops]
+            poisoned[which].view(-1, ops[which].shape[-2], D)[token, -1, 3] = value
+            leaves = [t.cuda().requires_grad_() for t in poisoned[:3]]
+            add = dict(zip(("additional_keys", "additional_values"), [t.cuda() for t in extras]))
+            out = fn(*leaves, ks, st, di, ca, **add)
+            got = [out.detach(), *torch.autograd.grad(out, leaves, poisoned[3].cuda())]
+            f = [t.numpy() for t in poisoned]
+            ex = dict(add_k=extras[0].numpy(), add_v=extras[1].numpy()) if n_extra else {}
+            with np.errstate(invalid="ignore"):
+                want = [oracle.na_forward(*f[:3], ks, st, di, ca, **ex)[0],
+                        *oracle.na_backward(*f, ks, st, di, ca, **ex)[:3]]
+            for g, w in zip(got, want):
+                g, on = g.cpu().numpy(), np.isfinite(w)
+                assert np.array_equal(np.isfinite(g), on)
+                if on.any():    # not where a causal window over everything starts with the token
+                    assert np.abs(g[on] - w[on]).max() <= 2e-4 * max(1.0, np.abs(w[on]).max())
