@@ -386,6 +386,9 @@ B200NA_API int b200na_na_backward_direct(
  *   - any 1-D dilation (see b200na_na_forward_view; two launches per pass when it does not divide
  *     the length);
  *   - tiles of up to 128 tokens (kv_tile: exactly 128 with extra tokens).
+ * With a 1-D window over the whole layout (no extra tokens) and with 1-D dilation above 2 the
+ * probabilities and dS are held in two 16-bit parts instead of being rounded to the operand type, here
+ * and in b200na_na_backward_direct.
  */
 B200NA_API int b200na_na_backward_view(
     const void* q, const void* k, const void* v, const void* o, const void* d_out, const float* lse,

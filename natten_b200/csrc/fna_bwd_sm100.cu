@@ -7,8 +7,10 @@
 // csrc/include/natten/cuda/reference/fna_reference_backward.hpp:62-385): with
 // P = exp(scale q.k - LSE), dP = dO.v, delta = dO.O:  dS = P (dP - delta),
 //   dQ = scale dS K,   dK = scale dS^T Q,   dV = P^T dO,
-// P and dS rounded to the operand type before the second products. The design is this library's:
-// ONE kernel template serves both passes, because they are mirror images of each other.
+// P and dS rounded to the operand type before the second products - or, kExact, split into two parts of
+// that type each (16 or 22 significant bits) whose products with the same operand add up in the fp32
+// accumulator. The design is this library's: ONE kernel template serves both passes, because they are
+// mirror images of each other.
 //   * A CTA owns a stationary 128-token ROW tile and streams 128-token COLUMN tiles past it:
 //       pass dQ   : rows = queries (R1 = Q, R2 = dO), columns = keys    (C1 = K, C2 = V)
 //       pass dKdV : rows = keys    (R1 = K, R2 = V),  columns = queries (C1 = Q, C2 = dO)
@@ -25,6 +27,11 @@
 //     them in registers, and the next tile's S and dP are computed while this tile's dS is. The
 //     C1 (K) and C2 (V) column tiles have rings of their own there: a C2 stage is free after dP,
 //     a C1 stage only after the dQ product.
+//   * kExact: both parts of P take the place of S, both parts of dS that of dP (pass dQ: one buffer in
+//     [384,512) instead of two), so no region changes its role between tiles. S of the next tile still
+//     goes out right after the product with P, while the threads work on dS. fp16 has five exponent bits:
+//     P is scaled by 2^15 and dS by a power of two from the largest norms of a dO and a V row, which a
+//     kernel ahead finds; both through the exponential's argument, undone in the epilogue.
 //   * Row statistics (LSE, delta) are per thread in pass dQ; in pass dKdV they belong to the
 //     columns and a warp of their own stages them through shared memory, up to four tiles ahead.
 //   * Warp roles: 16 softmax warps (four threads per row, 32 columns each: the P / dS arithmetic
@@ -105,6 +112,7 @@ struct BwdTcParams {
   float scale_log2;         // scale * log2(e)
   const float* lse;         // [B, *X, Hq]
   const float* delta;       // [B, *X, Hq]
+  const float* norms;       // fp16 with kExact: see ds_exponent
   void* out0;               // dQ (pass dQ) or dK (pass dKdV)
   void* out1;               // dV (pass dKdV)
   int* status;
@@ -304,6 +312,24 @@ struct Bars {
 
 constexpr int kTileInterior = 1, kTileBoundary = 2, kTileRagged = 3;
 
+// What rounding a and b to the 16-bit pair `packed` left over, as a pair of its own.
+template <int kType>
+__device__ __forceinline__ uint32_t pack2_rest(uint32_t packed, float a, float b) {
+  if (kType == kTyBf16)
+    return pack2<kType>(a - __uint_as_float(packed << 16), b - __uint_as_float(packed & 0xffff0000u));
+  const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&packed));
+  return pack2<kType>(a - f.x, b - f.y);
+}
+
+// fp16, kExact: P is held as 2^kPExponent P and dS as 2^ds_exponent dS. |dS_ij| = P_ij |dO_i . (V_j - O_i)|
+// is at most 2 |dO_i| max |V| (O_i is a mean of V rows; 1 % for its rounding), so that the scaled one stays
+// below 2^15 and values 2^-22 of that keep 11 bits in two parts. `norms`: the largest squared norms.
+constexpr int kPExponent = 15;
+__device__ __forceinline__ int ds_exponent(const float* norms) {
+  const float bound = 2.02f * sqrtf(norms[0]) * sqrtf(norms[1]);
+  return bound > 0.f && bound < INFINITY ? 14 - ilogbf(bound) : 0;
+}
+
 // Per-item constants of the column-tile walk and classification, held in registers by the load
 // thread (all its instructions are dependent, so shared-memory reads per tile would add latency).
 struct TileWalk {
@@ -339,7 +365,7 @@ struct TileWalk {
   }
 };
 
-template <int D, int kType, int NDIM, bool kKeyRows>
+template <int D, int kType, int NDIM, bool kKeyRows, bool kExact>
 __global__ void __launch_bounds__(kThreads, 1)
 fna_bwd_kernel(const __grid_constant__ CUtensorMap tm_r1, const __grid_constant__ CUtensorMap tm_r2,
                const __grid_constant__ CUtensorMap tm_c1, const __grid_constant__ CUtensorMap tm_c2,
@@ -462,7 +488,11 @@ fna_bwd_kernel(const __grid_constant__ CUtensorMap tm_r1, const __grid_constant_
   // dS (64 columns each). With dS written there instead of over dP, the logit / dP columns are
   // free again as soon as the softmax threads have read them, and the MMA thread computes the next
   // column tile's S and dP while the threads turn this tile's values into dS.
-  constexpr uint32_t kDsCol = 384, kDsBufCols = 64;
+  // With both parts of dS (kExact) there is room for one buffer.
+  constexpr uint32_t kDsCol = 384, kDsBufCols = 64, kDsBufs = kExact ? 1 : 2;
+  // packed columns between a thread's 16 of one 32-column part and the next thread's
+  constexpr uint32_t kDsPart = kExact ? 32 : 16;
+  constexpr bool kScaled = kExact && kType == kTyF16;
 
   if (warp < kSoftmaxWarps) {
     // ============ P / dS computation and the epilogue (four threads per row) ====================
@@ -473,6 +503,7 @@ fna_bwd_kernel(const __grid_constant__ CUtensorMap tm_r1, const __grid_constant_
     const uint32_t my_dp = lane_addr + kDpCol + part * 32;
     const float c = p.scale_log2;
     constexpr float kLog2e = 1.4426950408889634f;
+    const int ds_exp = kScaled ? ds_exponent(p.norms) : 0;
     uint32_t ph_sdp = 0, ph_dp = 0, ph_acc = 0, tseq = 0, dseq = 0;
     BTRACE_DECL(4 * 40)
     // in-tile coordinates of this thread's row
@@ -518,8 +549,9 @@ fna_bwd_kernel(const __grid_constant__ CUtensorMap tm_r1, const __grid_constant_
         row_l = p.lse[row_tok * p.Hq + it.h] * kLog2e;
         row_d = p.delta[row_tok * p.Hq + it.h];
       }
-      const uint64_t c2 = ptx::f32x2(c, c), nl2 = ptx::f32x2(-row_l, -row_l),
-                     nd2 = ptx::f32x2(-row_d, -row_d);
+      // pass dQ needs P only as a factor of dS: its exponent takes the whole scale
+      const float nl = (float)ds_exp - row_l;
+      const uint64_t c2 = ptx::f32x2(c, c), nl2 = ptx::f32x2(nl, nl), nd2 = ptx::f32x2(-row_d, -row_d);
       bool alive = true;
       for (int iter = 0; iter < n_tiles; ++iter) {
         if (!__all_sync(0xffffffffu,
@@ -573,7 +605,7 @@ fna_bwd_kernel(const __grid_constant__ CUtensorMap tm_r1, const __grid_constant_
           if (lane == 0) ptx::mbar_arrive(bars.sdp_free);
           if (lane == 0 && (warp == 0 || warp == 15)) BTRACE(warp == 0 ? 2 : 3, 9);
           // packed (two-wide) arithmetic: half the instructions of the scalar forms
-          uint32_t dk[16];
+          uint32_t dk[16], dl[kExact ? 16 : 1];
 #pragma unroll
           for (int j = 0; j < 32; j += 2) {
             float x0, x1, d0, d1;
@@ -587,18 +619,20 @@ fna_bwd_kernel(const __grid_constant__ CUtensorMap tm_r1, const __grid_constant_
                                             ptx::add_f32x2(ptx::f32x2(dr[j], dr[j + 1]), nd2)),
                              d0, d1);
             dk[j >> 1] = pack2<kType>(d0, d1);
+            if constexpr (kExact) dl[j >> 1] = pack2_rest<kType>(dk[j >> 1], d0, d1);
           }
           if (lane == 0 && (warp == 0 || warp == 15)) BTRACE(warp == 0 ? 2 : 3, 10);
-          // the dS buffer of two tiles ago must have been consumed by its dQ product
-          const uint32_t buf = dseq & 1;
-          if (!__all_sync(0xffffffffu, wait_bar(bars.ds_free + buf, ((dseq >> 1) & 1) ^ 1,
+          // the buffer's last dS must have been consumed by its dQ product
+          const uint32_t buf = dseq % kDsBufs;
+          if (!__all_sync(0xffffffffu, wait_bar(bars.ds_free + buf, ((dseq / kDsBufs) & 1) ^ 1,
                                                 abort_flag, p.status, (5 << 8) | kStDsFree))) {
             alive = false;
             break;
           }
           ++dseq;
           ptx::tc_fence_after_sync();
-          ptx::tmem_st16(lane_addr + kDsCol + buf * kDsBufCols + part * 16, dk);
+          ptx::tmem_st16(lane_addr + kDsCol + buf * kDsBufCols + part * kDsPart, dk);
+          if constexpr (kExact) ptx::tmem_st16(lane_addr + kDsCol + part * kDsPart + 16, dl);
           ptx::tmem_st_wait();
           ptx::tc_fence_before_sync();
           __syncwarp();
@@ -611,7 +645,9 @@ fna_bwd_kernel(const __grid_constant__ CUtensorMap tm_r1, const __grid_constant_
           // dP product still runs; dS = P (dP - delta) follows once dP is there and goes over
           // the second half. As soon as dP is in registers its region is handed back, and the
           // next tile's S is computed there during this tile's dS arithmetic and products.
-          const uint32_t reg = dseq & 1;
+          // kExact: S always arrives in the first region, where both parts of P replace it, dP in the
+          // second, where both parts of dS do.
+          const uint32_t reg = kExact ? 0 : dseq & 1;
           ++dseq;
           const uint32_t my_r = lane_addr + (reg ? kDpCol : kSCol) + part * 32;
           const uint32_t my_o = lane_addr + (reg ? kSCol : kDpCol) + part * 32;
@@ -621,7 +657,7 @@ fna_bwd_kernel(const __grid_constant__ CUtensorMap tm_r1, const __grid_constant_
             ptx::tmem_ld32(my_r, sr);
             ptx::tmem_ld_wait();
             if (lane == 0 && (warp == 0 || warp == 15)) BTRACE(warp == 0 ? 2 : 3, 9);
-            uint32_t pk[16];
+            uint32_t pk[16], pl[kExact ? 16 : 1];
 #pragma unroll
             for (int j = 0; j < 32; j += 2) {
               const uint64_t nl = *reinterpret_cast<const uint64_t*>(stat + part * 32 + j);
@@ -635,8 +671,10 @@ fna_bwd_kernel(const __grid_constant__ CUtensorMap tm_r1, const __grid_constant_
               pf[j] = p0;
               pf[j + 1] = p1;
               pk[j >> 1] = pack2<kType>(p0, p1);
+              if constexpr (kExact) pl[j >> 1] = pack2_rest<kType>(pk[j >> 1], p0, p1);
             }
             ptx::tmem_st16(my_r, pk);
+            if constexpr (kExact) ptx::tmem_st16(my_r + 16, pl);
           }
           if (lane == 0 && (warp == 0 || warp == 15)) BTRACE(warp == 0 ? 2 : 3, 10);
           // P is complete: its product with C2 can start while dS is still being computed
@@ -661,17 +699,28 @@ fna_bwd_kernel(const __grid_constant__ CUtensorMap tm_r1, const __grid_constant_
             __syncwarp();
             if (lane == 0) ptx::mbar_arrive(bars.sdp_free);
             if (lane == 0 && (warp == 0 || warp == 15)) BTRACE(warp == 0 ? 2 : 3, 13);
-            uint32_t dk[16];
+            uint32_t dk[16], dl[kExact ? 16 : 1];
+            // kScaled: 2^kPExponent P (dP - delta) 2^(ds_exp - kPExponent), delta scaled already
+            const float rest = kScaled ? exp2f((float)(ds_exp - kPExponent)) : 1.f;
+            const uint64_t rest2 = ptx::f32x2(rest, rest);
 #pragma unroll
             for (int j = 0; j < 32; j += 2) {
               const uint64_t nd = *reinterpret_cast<const uint64_t*>(stat + kTile + part * 32 + j);
+              const uint64_t dp2 = ptx::f32x2(dr[j], dr[j + 1]);
               float d0, d1;
               ptx::f32x2_split(ptx::mul_f32x2(ptx::f32x2(pf[j], pf[j + 1]),
-                                              ptx::add_f32x2(ptx::f32x2(dr[j], dr[j + 1]), nd)),
+                                              kScaled ? ptx::fma_f32x2(dp2, rest2, nd)
+                                                      : ptx::add_f32x2(dp2, nd)),
                                d0, d1);
               dk[j >> 1] = pack2<kType>(d0, d1);
+              if constexpr (kExact) dl[j >> 1] = pack2_rest<kType>(dk[j >> 1], d0, d1);
             }
-            ptx::tmem_st16(my_r + 16, dk);
+            if constexpr (kExact) {
+              ptx::tmem_st16(my_o, dk);
+              ptx::tmem_st16(my_o + 16, dl);
+            } else {
+              ptx::tmem_st16(my_r + 16, dk);
+            }
           }
           ptx::tmem_st_wait();
           ptx::tc_fence_before_sync();
@@ -695,7 +744,8 @@ fna_bwd_kernel(const __grid_constant__ CUtensorMap tm_r1, const __grid_constant_
         constexpr int kCols = D / kParts;  // output columns per thread: 32 or 16
         T* orow = reinterpret_cast<T*>(acc ? p.out1 : p.out0) +
                   row_tok * (acc ? p.out1_stride : p.out0_stride) + it.h * p.d_real + part * kCols;
-        const float mul = acc ? 1.f : p.scale;
+        float mul = acc ? 1.f : p.scale;
+        if (kScaled) mul *= exp2f((float)-(acc ? kPExponent : ds_exp));
         const uint32_t src = lane_addr + (acc ? kAcc1Col : kAcc0Col) + part * kCols;
         uint32_t orr[kCols];
         if (kCols == 32) ptx::tmem_ld32(src, reinterpret_cast<uint32_t(&)[32]>(orr));
@@ -823,10 +873,10 @@ fna_bwd_kernel(const __grid_constant__ CUtensorMap tm_r1, const __grid_constant_
         } else if (kPipe) {
           // ---- pass dQ, second issuer: dQ += dS C1 of each column tile when its dS is stored
           for (int t = 0; t < n; ++t) {
-            const uint32_t buf = gt & 1;
+            const uint32_t buf = gt % kDsBufs;
             // the C1 wait cannot block (S of this tile was computed from the same stage); it
             // orders this thread's reads after the tile's arrival
-            if (!wait_all(bars.ds_full + buf, (gt >> 1) & 1, abort_flag, p.status,
+            if (!wait_all(bars.ds_full + buf, (gt / kDsBufs) & 1, abort_flag, p.status,
                           (role << 8) | kStDsFull) ||
                 !wait_all(bars.c_full + slot, ph_c, abort_flag, p.status,
                           (role << 8) | kStCFull)) {
@@ -843,8 +893,10 @@ fna_bwd_kernel(const __grid_constant__ CUtensorMap tm_r1, const __grid_constant_
             }
             if (lane == 0) BTRACE(4, 4);
             ptx::tc_fence_after_sync();
-            issue_acc(acc0_tm, tmem_base + kDsCol + buf * kDsBufCols, 16,
+            issue_acc(acc0_tm, tmem_base + kDsCol + buf * kDsBufCols, kDsPart,
                       col_base + slot * kTileBytes, t == 0);
+            if constexpr (kExact)
+              issue_acc(acc0_tm, tmem_base + kDsCol + 16, kDsPart, col_base + slot * kTileBytes, false);
             ptx::tc_commit_if(issue, bars.c_empty + slot);
             ptx::tc_commit_if(issue, bars.ds_free + buf);
             if (t == n - 1) ptx::tc_commit_if(issue, bars.acc_full);
@@ -861,7 +913,9 @@ fna_bwd_kernel(const __grid_constant__ CUtensorMap tm_r1, const __grid_constant_
           // behind their readers in issue order).
           if (!wait_all(bars.r_full, ph_r, abort_flag, p.status, (role << 8) | kStRFull)) break;
           ph_r ^= 1;
-          const uint32_t reg_tm[2] = {s_tm, dp_tm};
+          // regions of the products of tile number k
+          auto s_reg = [&](uint32_t k) { return kExact || !(k & 1) ? s_tm : dp_tm; };
+          auto dp_reg = [&](uint32_t k) { return kExact || !(k & 1) ? dp_tm : s_tm; };
           // first tile of the item: S, then dP (the other region's last readers, the previous
           // item's accumulations, were issued before)
           if (!wait_all(bars.c_full + slot, ph_c, abort_flag, p.status, (role << 8) | kStCFull) ||
@@ -870,9 +924,9 @@ fna_bwd_kernel(const __grid_constant__ CUtensorMap tm_r1, const __grid_constant_
             break;
           uint32_t c_cur = col_base + slot * 2 * kTileBytes, c_next = 0;
           ptx::tc_fence_after_sync();
-          issue_rc(reg_tm[gt & 1], r1_lo, c_cur);
+          issue_rc(s_reg(gt), r1_lo, c_cur);
           ptx::tc_commit_if(issue, bars.sdp_full);
-          issue_rc(reg_tm[(gt & 1) ^ 1], r2_lo, c_cur + kTileBytes);
+          issue_rc(dp_reg(gt), r2_lo, c_cur + kTileBytes);
           ptx::tc_commit_if(issue, bars.dp_full);
           if (n == 1) ptx::tc_commit_if(issue, bars.r_empty);
           ++gt;
@@ -891,17 +945,20 @@ fna_bwd_kernel(const __grid_constant__ CUtensorMap tm_r1, const __grid_constant_
               ph_ae ^= 1;
             }
             // Of a thread's columns [32 q, 32 q + 32) of the tile's region, [32 q, 32 q + 16)
-            // hold its packed P and [32 q + 16, 32 q + 32) its dS.
+            // hold its packed P and [32 q + 16, 32 q + 32) its dS (kExact: the second part of P;
+            // dS likewise in the other region).
             // acc1 += P C2 as soon as P is stored, while the threads still work on dS
             if (!wait_all(bars.p_full, k & 1, abort_flag, p.status, (role << 8) | kStPFull)) {
               alive = false; break;
             }
             if (lane == 0) BTRACE(0, 1);
             ptx::tc_fence_after_sync();
-            issue_acc(acc1_tm, reg_tm[k & 1], 32, c_cur + kTileBytes, t == 0);
+            issue_acc(acc1_tm, s_reg(k), 32, c_cur + kTileBytes, t == 0);
+            if constexpr (kExact) issue_acc(acc1_tm, s_reg(k) + 16, 32, c_cur + kTileBytes, false);
             if (lane == 0) BTRACE(0, 2);
             if (t + 1 < n) {
-              // S of the next tile, into the region dP of this tile has been taken out of
+              // S of the next tile, into the region dP of this tile has been taken out of (kExact:
+              // over P, behind its readers in issue order)
               if (!wait_all(bars.c_full + slot, ph_c, abort_flag, p.status,
                             (role << 8) | kStCFull) ||
                   !wait_all(bars.sdp_free, (gt & 1) ^ 1, abort_flag, p.status,
@@ -911,7 +968,7 @@ fna_bwd_kernel(const __grid_constant__ CUtensorMap tm_r1, const __grid_constant_
               c_next = col_base + slot * 2 * kTileBytes;
               if (lane == 0) BTRACE(0, 3);
               ptx::tc_fence_after_sync();
-              issue_rc(reg_tm[gt & 1], r1_lo, c_next);
+              issue_rc(s_reg(gt), r1_lo, c_next);
               ptx::tc_commit_if(issue, bars.sdp_full);
               if (lane == 0) BTRACE(0, 4);
               ++gt;
@@ -926,14 +983,15 @@ fna_bwd_kernel(const __grid_constant__ CUtensorMap tm_r1, const __grid_constant_
             }
             if (lane == 0) BTRACE(0, 5);
             ptx::tc_fence_after_sync();
-            issue_acc(acc0_tm, reg_tm[k & 1] + 16, 32, c_cur, t == 0);
+            issue_acc(acc0_tm, kExact ? dp_reg(k) : s_reg(k) + 16, 32, c_cur, t == 0);
+            if constexpr (kExact) issue_acc(acc0_tm, dp_reg(k) + 16, 32, c_cur, false);
             ptx::tc_commit_if(issue, bars.c_empty + slot_d);
             if (lane == 0) BTRACE(0, 6);
             if (t == n - 1) ptx::tc_commit_if(issue, bars.acc_full);
             if (++slot_d == kStages) slot_d = 0;
             if (t + 1 < n) {
               // dP of the next tile over this tile's P / dS, behind their readers in issue order
-              issue_rc(reg_tm[k & 1], r2_lo, c_next + kTileBytes);
+              issue_rc(dp_reg(k + 1), r2_lo, c_next + kTileBytes);
               ptx::tc_commit_if(issue, bars.dp_full);
               if (lane == 0) BTRACE(0, 7);
               // the row tiles are read by the S / dP products only
@@ -960,6 +1018,8 @@ fna_bwd_kernel(const __grid_constant__ CUtensorMap tm_r1, const __grid_constant_
       }
     }
     constexpr float kLog2e = 1.4426950408889634f;
+    constexpr float p_exp = kScaled ? (float)kPExponent : 0.f;
+    const float d_mul = kScaled ? -exp2f((float)(ds_exponent(p.norms) - kPExponent)) : -1.f;
     uint32_t tseq = 0;
     bool alive = true;
     for (uint32_t seq = 0; alive; ++seq) {
@@ -1001,8 +1061,8 @@ fna_bwd_kernel(const __grid_constant__ CUtensorMap tm_r1, const __grid_constant_
                   p.fold_g0 + it.g[1];
           // stored negated, so that the packed additions take them as they are; a column past the
           // extent gets -LSE = -inf, i.e. P = 0
-          l[q] = ok ? -p.lse[tok * p.Hq + hq] * kLog2e : -INFINITY;
-          d[q] = ok ? -p.delta[tok * p.Hq + hq] : 0.f;
+          l[q] = ok ? -p.lse[tok * p.Hq + hq] * kLog2e + p_exp : -INFINITY;
+          d[q] = ok ? p.delta[tok * p.Hq + hq] * d_mul : 0.f;
         }
         const uint32_t sbuf = tseq % kStatBufs;
         if (!__all_sync(0xffffffffu,
@@ -1214,11 +1274,20 @@ int g_bwd_trace_pass = 0;
 template <int D, bool kBf16, bool kKeyRows>
 const void* bwd_kernel_for_ndim(int ndim) {
   constexpr int kType = kBf16 ? kTyBf16 : kTyF16;
-  if (ndim == 1) return (const void*)fna_bwd_kernel<D, kType, 1, kKeyRows>;
-  if (ndim == 2) return (const void*)fna_bwd_kernel<D, kType, 2, kKeyRows>;
-  return (const void*)fna_bwd_kernel<D, kType, 3, kKeyRows>;
+  if (ndim == 1) return (const void*)fna_bwd_kernel<D, kType, 1, kKeyRows, false>;
+  if (ndim == 2) return (const void*)fna_bwd_kernel<D, kType, 2, kKeyRows, false>;
+  return (const void*)fna_bwd_kernel<D, kType, 3, kKeyRows, false>;
 }
-const void* bwd_kernel_variant(int D, bool bf16, int ndim, bool key_rows) {
+template <int D, int kType>
+const void* bwd_kernel_exact(bool key_rows) {
+  return key_rows ? (const void*)fna_bwd_kernel<D, kType, 1, true, true>
+                  : (const void*)fna_bwd_kernel<D, kType, 1, false, true>;
+}
+const void* bwd_kernel_variant(int D, bool bf16, int ndim, bool key_rows, bool exact) {
+  if (exact) {   // one axis
+    if (D == 128) return bf16 ? bwd_kernel_exact<128, kTyBf16>(key_rows) : bwd_kernel_exact<128, kTyF16>(key_rows);
+    return bf16 ? bwd_kernel_exact<64, kTyBf16>(key_rows) : bwd_kernel_exact<64, kTyF16>(key_rows);
+  }
   if (D == 128) {
     if (bf16) return key_rows ? bwd_kernel_for_ndim<128, true, true>(ndim)
                               : bwd_kernel_for_ndim<128, true, false>(ndim);
@@ -1234,12 +1303,13 @@ const void* bwd_kernel_variant(int D, bool bf16, int ndim, bool key_rows) {
 // Opt-in shared memory per kernel variant and device, set once.
 int ensure_smem_attribute(const void* fn, int smem_bytes) {
   static std::mutex mu;
-  static const void* done[64][24];
+  constexpr int kVariants = 32;
+  static const void* done[64][kVariants];
   int dev = 0;
   B200NA_CUDA_TRY(cudaGetDevice(&dev));
   if (dev < 0 || dev >= 64) return B200NA_ERR_DEVICE;
   std::lock_guard<std::mutex> lk(mu);
-  for (int i = 0; i < 24; ++i) {
+  for (int i = 0; i < kVariants; ++i) {
     if (done[dev][i] == fn) return B200NA_OK;
     if (done[dev][i] == nullptr) {
       B200NA_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1269,9 +1339,9 @@ struct BwdCall {
 };
 
 // One pass over one part of the layout (all of it, or the dilation groups of a folded 1-D part).
-int launch_pass(const BwdTcParams& p, int D, int dtype, int kernel_ndim, bool key_rows, void** args,
-                int sms, cudaStream_t stream) {
-  const void* fn = bwd_kernel_variant(D, dtype == B200NA_BF16, kernel_ndim, key_rows);
+int launch_pass(const BwdTcParams& p, int D, int dtype, int kernel_ndim, bool key_rows, bool exact,
+                void** args, int sms, cudaStream_t stream) {
+  const void* fn = bwd_kernel_variant(D, dtype == B200NA_BF16, kernel_ndim, key_rows, exact);
   const int smem_bytes = key_rows ? (D == 128 ? Smem<128, false>::kBytes : Smem<64, false>::kBytes)
                                   : (D == 128 ? Smem<128, true>::kBytes : Smem<64, true>::kBytes);
   const int rc = ensure_smem_attribute(fn, smem_bytes);
@@ -1364,9 +1434,22 @@ int backward_impl(const BwdCall& c, int ndim, const int* shape, const int* kerne
     if ((rc = fna_make_tensor_map_direct(&mdof, c.d_out, dtype, B, x_flat, Hq, D, flat_tile, ones, 0, sep1)) != B200NA_OK) return rc;
   }
 
+  // Dense attention and 1-D dilation above 2 had their gradients from the CUDA cores first, with P and dS in
+  // fp32; here two parts keep that precision. 2-norm errors of dQ, dK, dV against 64 bits, in 1e-3: B2 N1370
+  // H12 D64 bf16 1.690 1.662 1.660, the CUDA cores the same; N4096 D64 bf16 1.682 1.660 1.651 (CUDA cores
+  // 1.683 1.660 1.651; with P and dS rounded to bf16 2.390 2.342 2.263); N65536 1.690 1.665 1.663 (1.683
+  // 1.658 1.656), where the tensor cores' accumulators, which round towards zero, begin to show. fp16:
+  // N4096 0.2114 0.2076 0.2074 (0.2111 0.2073 0.2072), N65536 0.260 0.258 0.256 (0.211 0.207 0.207): the
+  // front sends sums of more than 4096 terms to the CUDA cores. B2 N1370 H12 D64 bf16, forward and
+  // backward: 118 us with rounded P and dS, 141 us.
+  const bool exact =
+      ndim == 1 && (base.dil[0] > 2 || (n_extra == 0 && base.kernel[0] == base.X[0]));
   FoldedPart parts[2] = {{0, 0, 0}, {0, 0, 0}};
   const int n_fold = c.views ? fna_fold_parts(ndim, base.X[0], base.dil[0], parts) : 0;
   bool delta_done = false;
+  static std::mutex norms_mu;
+  std::unique_lock<std::mutex> norms_lock;
+  float* norms = nullptr;
   for (int part = 0; part < (n_fold ? n_fold : 1); ++part) {
     BwdTcParams view = base;
     FoldedAxis folded = {base.dil[0], parts[part].g0, parts[part].groups, base.X[0]};
@@ -1385,6 +1468,15 @@ int backward_impl(const BwdCall& c, int ndim, const int* shape, const int* kerne
     if ((rc = fna_make_tensor_map_direct(&mk, c.k, dtype, B, view.X, Hkv, D, tkv, view.dil, k_ts, sep, fold)) != B200NA_OK) return rc;
     if ((rc = fna_make_tensor_map_direct(&mv, c.v, dtype, B, view.X, Hkv, D, tkv, view.dil, v_ts, sep, fold)) != B200NA_OK) return rc;
     if (n_extra == 0) { mek = mk; mev = mv; }
+    if (!delta_done && exact && dtype == B200NA_F16) {
+      // norms of another call on this stream must not come between these launches
+      norms_lock = std::unique_lock<std::mutex>(norms_mu);
+      if ((rc = fna_call_norms(&norms, stream)) != B200NA_OK) return rc;
+      const NormRows in[3] = {{c.d_out, tokens * B, Hq, wq, 0}, {c.v, tokens * B, Hkv, v_ts, 1},
+                              {c.add_v, (int64_t)n_extra * B, Hkv, wkv, 1}};
+      if ((rc = launch_max_norms(in, n_extra > 0 ? 3 : 2, D, norms, stream)) != B200NA_OK) return rc;
+      base.norms = view.norms = norms;
+    }
     if (!delta_done) {   // after every check of the first part
       if ((rc = launch_delta(c.o, c.d_out, c.delta, tokens * B * Hq, D, dtype, stream)) != B200NA_OK)
         return rc;
@@ -1421,8 +1513,8 @@ int backward_impl(const BwdCall& c, int ndim, const int* shape, const int* kerne
       p.trace = pass == g_bwd_trace_pass ? g_bwd_trace : nullptr;
       void* args_q[] = {(void*)&mq, (void*)&mdo, (void*)&mk, (void*)&mv, (void*)&mek, (void*)&mev, (void*)&p};
       void* args_k[] = {(void*)&mk, (void*)&mv, (void*)&mq, (void*)&mdo, (void*)&mek, (void*)&mev, (void*)&p};
-      if ((rc = launch_pass(p, Dk, dtype, ndim, key_rows, key_rows ? args_k : args_q, sms, stream)) !=
-          B200NA_OK)
+      if ((rc = launch_pass(p, Dk, dtype, ndim, key_rows, exact, key_rows ? args_k : args_q, sms,
+                            stream)) != B200NA_OK)
         return rc;
     }
   }
@@ -1450,7 +1542,7 @@ int backward_impl(const BwdCall& c, int ndim, const int* shape, const int* kerne
   if ((rc = fna_work_counters(&p.work, stream)) != B200NA_OK) return rc;
   p.trace = g_bwd_trace_pass == 2 ? g_bwd_trace : nullptr;
   void* args[] = {(void*)&mek, (void*)&mev, (void*)&mqf, (void*)&mdof, (void*)&mek, (void*)&mev, (void*)&p};
-  return launch_pass(p, Dk, dtype, 1, true, args, sms, stream);
+  return launch_pass(p, Dk, dtype, 1, true, exact, args, sms, stream);
 }
 }  // namespace
 }  // namespace b200na

@@ -40,6 +40,21 @@ int fna_device_info(int* sms, int** status_ptr);
 // under stream capture gets a pair of its own from a pool of 3072 that is handed out in turn.
 int fna_work_counters(unsigned long long** pair, cudaStream_t stream);
 
+// Two zeroed-by-the-user floats of device memory for one call on `stream`, from slots of their own that are
+// handed out like the counter pairs.
+int fna_call_norms(float** norms, cudaStream_t stream);
+
+// norms[slot] = the largest squared 2-norm of the rows of D fp16 elements (a multiple of 8, at most 128,
+// 16-byte aligned) of the inputs with that slot; both are set to 0 first. NaN where an input holds one.
+struct NormRows {
+  const void* rows;
+  int64_t tokens;
+  int heads;
+  int64_t token_stride;   // elements
+  int slot;
+};
+int launch_max_norms(const NormRows* in, int n_inputs, int D, float* norms, cudaStream_t stream);
+
 // delta[row] = sum_d o[row, d] * d_out[row, d] (fp32), rows of D 16-bit elements (a multiple of
 // 8, at most 128).
 int launch_delta(const void* o, const void* d_out, float* delta, int64_t rows, int D, int dtype,

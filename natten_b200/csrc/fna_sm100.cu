@@ -69,6 +69,8 @@ __device__ int g_status_word;
 constexpr int kStreamSlots = 1024;
 constexpr int kCounterSlots = 4096;
 __device__ unsigned long long g_work_counters[kCounterSlots][2];
+// Two floats per slot for a call that hands a reduction from one launch to the next (fna_call_norms).
+__device__ float g_call_norms[kCounterSlots][2];
 
 struct FnaParams {
   int ndim;
@@ -1418,6 +1420,7 @@ struct DeviceState {
   int sms = 0;
   int* status_ptr = nullptr;
   unsigned long long* counters = nullptr;  // g_work_counters on this device
+  float* norms = nullptr;                  // g_call_norms
   std::mutex slot_mu;
   std::unordered_map<cudaStream_t, int> stream_slot;   // counter pair of each stream seen so far
   unsigned next_graph_slot = 0;                        // captured launches take theirs in turn
@@ -1459,6 +1462,8 @@ int device_state(DeviceState** out) {
     B200NA_CUDA_TRY(cudaGetSymbolAddress(&sp, g_work_counters));
     st.counters = reinterpret_cast<unsigned long long*>(sp);
     B200NA_CUDA_TRY(cudaMemset(st.counters, 0, sizeof(unsigned long long) * kCounterSlots * 2));
+    B200NA_CUDA_TRY(cudaGetSymbolAddress(&sp, g_call_norms));
+    st.norms = reinterpret_cast<float*>(sp);
     st.ready = true;
   }
   *out = &st;
@@ -1553,18 +1558,18 @@ int fna_fold_parts(int ndim, int len, int d, FoldedPart (&parts)[2]) {
   parts[n++] = {rest, d - rest, len / d};
   return n;
 }
-int fna_work_counters(unsigned long long** pair, cudaStream_t stream) {
-  DeviceState* st = nullptr;
-  const int rc = device_state(&st);
+// Slot of device memory for a launch on `stream` (see g_work_counters).
+static int call_slot(int* slot, DeviceState** state, cudaStream_t stream) {
+  const int rc = device_state(state);
   if (rc != B200NA_OK) return rc;
+  DeviceState* const st = *state;
   cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
   B200NA_CUDA_TRY(cudaStreamIsCapturing(stream, &capturing));
   std::lock_guard<std::mutex> lk(st->slot_mu);
-  int slot;
   if (capturing != cudaStreamCaptureStatusNone) {
     // a graph node keeps its pair for every replay; nodes get distinct pairs until the pool of
     // kCounterSlots - kStreamSlots has gone round once
-    slot = kStreamSlots + (int)(st->next_graph_slot++ % (unsigned)(kCounterSlots - kStreamSlots));
+    *slot = kStreamSlots + (int)(st->next_graph_slot++ % (unsigned)(kCounterSlots - kStreamSlots));
   } else {
     auto it = st->stream_slot.find(stream);
     if (it == st->stream_slot.end()) {
@@ -1572,10 +1577,23 @@ int fna_work_counters(unsigned long long** pair, cudaStream_t stream) {
       const int fresh = (int)(st->stream_slot.size() % (size_t)kStreamSlots);
       it = st->stream_slot.emplace(stream, fresh).first;
     }
-    slot = it->second;
+    *slot = it->second;
   }
-  *pair = st->counters + 2 * slot;
   return B200NA_OK;
+}
+int fna_work_counters(unsigned long long** pair, cudaStream_t stream) {
+  DeviceState* st = nullptr;
+  int slot = 0;
+  const int rc = call_slot(&slot, &st, stream);
+  if (rc == B200NA_OK) *pair = st->counters + 2 * slot;
+  return rc;
+}
+int fna_call_norms(float** norms, cudaStream_t stream) {
+  DeviceState* st = nullptr;
+  int slot = 0;
+  const int rc = call_slot(&slot, &st, stream);
+  if (rc == B200NA_OK) *norms = st->norms + 2 * slot;
+  return rc;
 }
 int fna_device_info(int* sms, int** status_ptr) {
   DeviceState* st = nullptr;

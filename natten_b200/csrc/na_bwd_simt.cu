@@ -278,7 +278,53 @@ int launch_delta_typed(const void* o, const void* d_out, float* delta, int64_t r
   return B200NA_OK;
 }
 
+// A lane per 16 bytes, kLanes per row, a block's largest row in one atomic. Squared norms are not negative,
+// so that their bits order like they do, with NaN above all.
+template <int kLanes>
+__global__ void __launch_bounds__(kDeltaThreads) max_norms_kernel(NormRows a, NormRows b, NormRows c,
+                                                                  int chunks, unsigned* norms) {
+  const NormRows in = blockIdx.y == 0 ? a : (blockIdx.y == 1 ? b : c);
+  const int ch = threadIdx.x % kLanes;
+  const int64_t rows = in.tokens * in.heads, step = (int64_t)gridDim.x * (kDeltaThreads / kLanes);
+  unsigned most = 0;
+  for (int64_t r0 = (int64_t)blockIdx.x * (kDeltaThreads / kLanes); r0 < rows; r0 += step) {
+    const int64_t row = r0 + threadIdx.x / kLanes;
+    float sum = 0.f;
+    if (row < rows && ch < chunks) {
+      const __half* p = static_cast<const __half*>(in.rows) + (row / in.heads) * in.token_stride +
+                        (row % in.heads) * chunks * 8 + ch * 8;
+      const uint4 x = *reinterpret_cast<const uint4*>(p);
+      const __half* v = reinterpret_cast<const __half*>(&x);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) sum = fmaf(ldf(v + e), ldf(v + e), sum);
+    }
+#pragma unroll
+    for (int off = kLanes / 2; off > 0; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
+    most = max(most, __float_as_uint(sum) & 0x7fffffffu);
+  }
+  most = __reduce_max_sync(0xffffffffu, most);
+  __shared__ unsigned part[kDeltaThreads / 32];
+  if (threadIdx.x % 32 == 0) part[threadIdx.x / 32] = most;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < kDeltaThreads / 32; ++w) most = max(most, part[w]);
+    atomicMax(norms + in.slot, most);
+  }
+}
+
 }  // namespace
+
+int launch_max_norms(const NormRows* in, int n_inputs, int D, float* norms, cudaStream_t stream) {
+  if (n_inputs < 2 || n_inputs > 3 || D % 8 != 0 || D < 8 || D > 128) return B200NA_ERR_INVALID_ARGUMENT;
+  B200NA_CUDA_TRY(cudaMemsetAsync(norms, 0, 2 * sizeof(float), stream));
+  const dim3 grid(148, n_inputs);
+  const NormRows& last = in[n_inputs - 1];
+  unsigned* out = reinterpret_cast<unsigned*>(norms);
+  if (D <= 64) max_norms_kernel<8><<<grid, kDeltaThreads, 0, stream>>>(in[0], in[1], last, D / 8, out);
+  else max_norms_kernel<16><<<grid, kDeltaThreads, 0, stream>>>(in[0], in[1], last, D / 8, out);
+  B200NA_CUDA_TRY(cudaGetLastError());
+  return B200NA_OK;
+}
 
 int launch_delta(const void* o, const void* d_out, float* delta, int64_t rows, int D, int dtype,
                  cudaStream_t stream) {

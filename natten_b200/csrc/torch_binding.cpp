@@ -588,8 +588,19 @@ struct GradPointers {
   long long dq_ts, dk_ts, dv_ts;   // tensor-core path only; the CUDA-core path needs 0 (contiguous)
   void *dak, *dav;
 };
+// Gradients whose P and dS keep more bits than the operands have: dense attention (a window over all of
+// one axis) and 1-D dilation above 2.
+bool exact_gradients(const Problem& p, bool extra) {
+  return p.nd == 1 && (p.dilation[0] > 2 || (!extra && p.kernel[0] == p.shape[0]));
+}
+// Sums of more terms than this have an error of their own beside fp16's results on the tensor cores, whose
+// accumulators round towards zero: 2 % of it at 16384 terms, 25 to 45 % at 65536.
+constexpr int kMostExactTermsF16 = 4096;
 bool backward_on_tensor_cores(const Problem& p, const Sizes& z, bool extra, Tiles* t) {
   if (!is_16bit(z.dt) || !reads_natively(z.dt, z.D)) return false;
+  if (z.dt == B200NA_F16 && exact_gradients(p, extra) &&
+      (extra ? p.shape[0] : p.kernel[0]) > kMostExactTermsF16)
+    return false;
   if (p.nd == 3 && z.B > 1 && z.D != 64 && z.D != 128) return false;
   *t = plan(p, true, extra);
   return p.nd == 1 || (box_fits(t->q, p) && box_fits(t->kv, p));
@@ -604,7 +615,8 @@ void run_backward(const Problem& p, const Sizes& z, float scale, bool tensor_cor
                                t.kv.data(), z.B, z.Hq, z.Hkv, z.D, z.dt, scale, a.q_ts, a.k_ts, a.v_ts,
                                g.dq_ts, g.dk_ts, g.dv_ts, stream),
           "b200na_na_backward_view");
-    launches += 1 + 2 * parts_of(p) + (a.n_extra ? 1 : 0);
+    launches += 1 + 2 * parts_of(p) + (a.n_extra ? 1 : 0) +
+                (exact_gradients(p, a.n_extra) && z.dt == B200NA_F16 ? 1 : 0);
   } else {
     check(lib.na_backward_simt(a.q, a.k, a.v, out, d_out, lse, a.ak, a.av, a.n_extra, g.dq, g.dk, g.dv,
                                g.dak, g.dav, delta, p.nd, p.shape.data(), p.kernel.data(),

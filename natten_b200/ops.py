@@ -366,10 +366,10 @@ def _fmha_backward(ctx, d_out, d_lse):
     n = query.shape[1]
     args = (query, key, value, out, d_out.contiguous(), lse, None, None, [n], [1], [1],
             [bool(ctx.is_causal)], ctx.scale)
-    # Same operands as neighborhood attention takes to the tensor cores; a window needs two tokens.
-    # The CUDA-core kernels read every key / value row once per query (no reuse between queries):
-    # forward + backward of B2 N1370 H12 D64 bf16 took 47.8 ms that way and takes 0.27 ms now.
-    if (query.dtype in (torch.float16, torch.bfloat16) and query.shape[-1] in (64, 128) and n >= 2):
+    # 16 bits on tensor cores, with P and dS in two 16-bit parts each; fp16 sums of more than 4096 terms,
+    # where the accumulators' rounding shows, on the CUDA cores. A window needs two tokens.
+    if query.shape[-1] in (64, 128) and n >= 2 and (query.dtype == torch.bfloat16 or (
+            query.dtype == torch.float16 and n <= 4096)):
         dq, dk, dv, _, _ = na_backward_direct(*args, [128], [128])
     else:
         dq, dk, dv, _, _ = na_backward_simt(*args)

@@ -326,3 +326,38 @@ def test_fp32_non_finite_tokens_stay_inside_their_windows(shape, ks, st, di, ca,
                 assert np.array_equal(np.isfinite(g), on)
                 if on.any():    # not where a causal window over everything starts with the token
                     assert np.abs(g[on] - w[on]).max() <= 2e-4 * max(1.0, np.abs(w[on]).max())
+
+
+@pytest.mark.parametrize("n,win,dil,causal,hq,hkv,D,n_extra", [
+    (129, 0, 1, False, 2, 1, 64, 0), (700, 0, 1, True, 3, 3, 128, 0), (1000, 0, 1, False, 2, 2, 40, 0),
+    (128, 0, 1, True, 1, 1, 64, 0), (1201, 65, 3, True, 2, 2, 64, 20), (1500, 129, 8, False, 4, 2, 128, 0),
+    (4097, 0, 1, True, 1, 1, 64, 0), (4100, 9, 3, True, 2, 2, 64, 40)])
+@pytest.mark.parametrize("dtype,size", [(torch.bfloat16, 1.0), (torch.float16, 1.0), (torch.float16, 2.0 ** -10),
+                                        (torch.float16, 2.0 ** 10)])
+def test_gradients_with_more_bits_than_the_operands(n, win, dil, causal, hq, hkv, D, n_extra, dtype, size):
+    """Dense attention and 1-D dilation above 2: P and dS are not rounded to the operands' type. Against
+    the CUDA-core kernels, which hold them in fp32: the same up to the results' own rounding. A relative
+    difference of 2^-16 (fp16: 2^-20, the sums' order) flips it for 2^-16 / 2^-8 (2^-20 / 2^-11) of the
+    entries by 2^-8 (2^-11), 2^-12 (2^-15.5) of the norm where there are thousands of them; with rounded P
+    and dS it was 2^-8.6 (2^-11.6)."""
+    torch.manual_seed(79)
+    q, d_out = (torch.randn(2, n, hq, D, device="cuda").to(dtype) for _ in range(2))
+    k, v = (torch.randn(2, n, hkv, D, device="cuda").to(dtype) for _ in range(2))
+    d_out = d_out * size
+    extras = [torch.randn(2, n_extra, hkv, D, device="cuda").to(dtype) for _ in range(2)] if n_extra else []
+    leaves = [t.requires_grad_() for t in [q, k, v] + extras]
+    if win:
+        add = dict(additional_keys=leaves[3], additional_values=leaves[4]) if n_extra else {}
+        out, lse = nb.na1d(*leaves[:3], win, 1, dil, causal, return_lse=True, **add)
+    else:
+        out, lse = nb.attention(*leaves, is_causal=causal, return_lse=True)
+    got = torch.autograd.grad(out, leaves, d_out)
+    assert L.device_status() == 0
+    with torch.no_grad():
+        want = nb.ops.na_backward_simt(q, k, v, out, d_out, lse, *(extras or (None, None)), [win or n], [1],
+                                       [dil], [causal], D ** -0.5)
+    tol = 2.0 ** -11.5 if dtype == torch.bfloat16 else 2.0 ** -14
+    if dtype == torch.float16 and (n if n_extra else win or n) > 4096:
+        tol = 0.0                                   # these are the CUDA-core kernels
+    for a, b in zip(got, want):
+        assert (a.float() - b.float()).norm() <= tol * b.float().norm()
