@@ -527,6 +527,13 @@ Tensor aligned(const Tensor& t) {
   return c;
 }
 
+// tokens of a batch entry of a heads-last tensor (its sizes' product may need 64 bits: callers check it)
+int64_t token_count(const Tensor& t) {
+  int64_t n = 1;
+  for (int64_t i = 1; i < t.dim() - 2; ++i) n *= t.size(i);
+  return n;
+}
+
 struct Sizes {
   int B, Hq, Hkv, D, dt;
 };
@@ -676,8 +683,7 @@ Forward forward_now(const Call& c, const Tensor& q, const Tensor& k, const Tenso
   b200na_stream_t stream = stream_of(q);
   if (c.dense) {
     const Tensor qc = q.contiguous(), kc = k.contiguous(), vc = v.contiguous();
-    const int nq = (int)(q.numel() / (c.z.B * c.z.Hq * c.z.D)),
-              nk = (int)(k.numel() / (c.z.B * c.z.Hkv * c.z.D));
+    const int nq = (int)token_count(q), nk = (int)token_count(k);
     const int splits =
         c.scale > 0.f ? lib.fmha_splits(c.z.B, nq, nk, c.z.Hq, c.z.D, c.z.dt, c.p.causal[0]) : 1;
     if (splits > 1) {
@@ -754,7 +760,7 @@ struct NaFunction : torch::autograd::Function<NaFunction> {
     Problem p = c.p;
     if (c.dense) {
       p.nd = 1;
-      p.shape = {(int)(q.numel() / (c.z.B * c.z.Hq * c.z.D)), 1, 1};
+      p.shape = {(int)token_count(q), 1, 1};
       p.kernel = {p.shape[0], 1, 1};
       p.stride = p.dilation = {1, 1, 1};
       p.causal = {c.p.causal[0], 0, 0};

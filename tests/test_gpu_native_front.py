@@ -361,3 +361,14 @@ def test_gradients_with_more_bits_than_the_operands(n, win, dil, causal, hq, hkv
         tol = 0.0                                   # these are the CUDA-core kernels
     for a, b in zip(got, want):
         assert (a.float() - b.float()).norm() <= tol * b.float().norm()
+
+
+def test_batches_of_more_than_2_to_31_elements():
+    """2^20 entries of one query and one key, 32 heads of 128: 2^32 elements. With one key the result is
+    its value."""
+    B, Hq, D = 1 << 20, 32, 128
+    q = torch.zeros(B, 1, Hq, D, device="cuda", dtype=torch.bfloat16)
+    v = torch.randn(B, 1, 1, D, device="cuda").bfloat16()
+    out = nb.attention(q, v, v)
+    for a in range(0, B, B // 8):
+        assert torch.equal(out[a:a + B // 8], v[a:a + B // 8].expand(-1, -1, Hq, -1))
