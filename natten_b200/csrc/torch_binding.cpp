@@ -753,7 +753,9 @@ struct NaFunction : torch::autograd::Function<NaFunction> {
     return seal(std::move(g));
   }
   static variable_list gradients(const Call& c, const variable_list& s, const Tensor& d_out_) {
-    const Tensor &out = s[0], &lse = s[1], &q = s[2], &k = s[3], &v = s[4];
+    // (saved-tensor hooks may have put them into other strides)
+    const Tensor out = s[0].contiguous(), lse = s[1].contiguous();
+    const Tensor &q = s[2], &k = s[3], &v = s[4];
     const bool extra = s.size() == 7;
     const Tensor ak = extra ? s[5] : Tensor(), av = extra ? s[6] : Tensor();
     c10::cuda::CUDAGuard guard(q.device());
@@ -857,7 +859,9 @@ struct LayerFunction : torch::autograd::Function<LayerFunction> {
     const auto call = c10::static_intrusive_pointer_cast<SharedCall>(
         ctx->saved_data["call"].toCapsule());
     const Call& c = call->c;
-    const Tensor &x = s[0], &w1 = s[1], &w2 = s[2], &qkv = s[3], &attn = s[4], &lse = s[5];
+    const Tensor &x = s[0], &w1 = s[1], &w2 = s[2];
+    // (saved-tensor hooks may have put them into other strides)
+    const Tensor qkv = s[3].contiguous(), attn = s[4].contiguous(), lse = s[5].contiguous();
     const int64_t b1_at = ctx->saved_data["b1"].toInt(), b2_at = ctx->saved_data["b2"].toInt();
     const bool need_x = ctx->needs_input_grad(0), need_w1 = ctx->needs_input_grad(1),
                need_w2 = ctx->needs_input_grad(2), need_b1 = b1_at && ctx->needs_input_grad(b1_at),

@@ -562,7 +562,8 @@ def _na_backward(ctx, d_out, d_lse):
     ignored, as in the reference's backward (src/natten/backends/blackwell_fna.py:185-318)."""
     query, key, value, out, lse = ctx.saved_tensors[:5]
     query, key, value = query.contiguous(), key.contiguous(), value.contiguous()
-    ak, av = ctx.saved_tensors[5:] if ctx.has_extra else (None, None)
+    out, lse = out.contiguous(), lse.contiguous()   # saved-tensor hooks may return other strides
+    ak, av = (t.contiguous() for t in ctx.saved_tensors[5:]) if ctx.has_extra else (None, None)
     kernel_size, stride, dilation, is_causal, scale = ctx.na_args
     na_dim = query.dim() - 3
     tensor_core = (query.dtype in (torch.float16, torch.bfloat16)

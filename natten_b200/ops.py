@@ -364,7 +364,8 @@ def _fmha_backward(ctx, d_out, d_lse):
         raise NotImplementedError("natten_b200: backward of attention() needs equal query and "
                                   "key/value lengths.")
     n = query.shape[1]
-    args = (query, key, value, out, d_out.contiguous(), lse, None, None, [n], [1], [1],
+    # (saved-tensor hooks may return other strides)
+    args = (*(t.contiguous() for t in (query, key, value, out, d_out, lse)), None, None, [n], [1], [1],
             [bool(ctx.is_causal)], ctx.scale)
     # 16 bits on tensor cores, with P and dS in two 16-bit parts each; fp16 sums of more than 4096 terms,
     # where the accumulators' rounding shows, on the CUDA cores. A window needs two tokens.

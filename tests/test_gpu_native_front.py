@@ -372,3 +372,35 @@ def test_batches_of_more_than_2_to_31_elements():
     out = nb.attention(q, v, v)
     for a in range(0, B, B // 8):
         assert torch.equal(out[a:a + B // 8], v[a:a + B // 8].expand(-1, -1, Hq, -1))
+
+
+def _strided(t):
+    """The same values with the axes' strides reversed."""
+    return t.permute(*reversed(range(t.dim()))).contiguous().permute(*reversed(range(t.dim())))
+
+
+@pytest.mark.parametrize("case", ["attention", "na", "na-fp32", "layer", "compiled-attention", "compiled-na"])
+def test_saved_tensor_hooks_that_return_other_strides(case):
+    torch.manual_seed(83)
+    dtype = torch.float32 if case == "na-fp32" else torch.bfloat16
+    if case == "layer":
+        layer = nb.NeighborhoodAttention2D(96, 3, 5).cuda().bfloat16()
+        x = torch.randn(2, 14, 17, 96, device="cuda").bfloat16().requires_grad_()
+        wrt, fn = [x, *layer.parameters()], lambda: layer(x)
+    else:
+        wrt = [torch.randn(2, 12, 13, 2, 64, device="cuda").to(dtype).requires_grad_() for _ in range(3)]
+        if "attention" in case:
+            wrt = [t.detach().flatten(1, 2).requires_grad_() for t in wrt]
+        fn = (lambda: nb.attention(*wrt)) if "attention" in case else (lambda: nb.na2d(*wrt, 5))
+        if "compiled" in case:   # the registered operators, as compiled code calls them
+            op = nb.functional.ops.fmha_forward if "attention" in case else nb.functional.na_forward_op
+            args = (False, 0.125) if "attention" in case else (None, None, [5, 5], [1, 1], [1, 1],
+                                                               [False, False], 0.125, [], [], False, [], [])
+            fn = lambda: op(*wrt, *args)[0]
+    out = fn()
+    d_out = torch.randn_like(out)
+    want = torch.autograd.grad(out, wrt, d_out)
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: t, _strided):
+        out = fn()
+    for a, b in zip(torch.autograd.grad(out, wrt, d_out), want):
+        assert torch.equal(a, b)
