@@ -578,12 +578,12 @@ int run_forward(const Problem& p, const Sizes& z, float scale, Path path, const 
                              p.kernel.data(), p.stride.data(), p.dilation.data(), p.causal.data(),
                              t.q.data(), t.kv.data(), z.B, z.Hq, z.Hkv, z.D, z.dt, scale, a.q_ts,
                              a.k_ts, a.v_ts, stream);
-    launches += parts_of(p);
+    if (rc == B200NA_OK) launches += parts_of(p);
   } else {
     rc = lib.na_forward_simt(a.q, a.k, a.v, out, lse, p.nd, p.shape.data(), p.kernel.data(),
                              p.stride.data(), p.dilation.data(), p.causal.data(), z.B, z.Hq, z.Hkv,
                              z.D, z.dt, scale, a.ak, a.av, a.n_extra, stream);
-    ++launches;
+    if (rc == B200NA_OK) ++launches;
   }
   return rc;
 }
@@ -692,13 +692,13 @@ Forward forward_now(const Call& c, const Tensor& q, const Tensor& k, const Tenso
       f.status = lib.fmha_forward_split(qc.data_ptr(), kc.data_ptr(), vc.data_ptr(), f.out.data_ptr(),
                                         lse, c.z.B, nq, nk, c.z.Hq, c.z.Hkv, c.z.D, c.z.dt, c.scale,
                                         scratch.data_ptr<float>(), stream);
-      launches += 2;
+      if (f.status == B200NA_OK) launches += 2;
       return f;
     }
     f.status = lib.fmha_forward(qc.data_ptr(), kc.data_ptr(), vc.data_ptr(), f.out.data_ptr(), lse,
                                 c.z.B, nq, nk, c.z.Hq, c.z.Hkv, c.z.D, c.z.dt, c.scale,
                                 c.p.causal[0], stream);
-    ++launches;
+    if (f.status == B200NA_OK) ++launches;
     return f;
   }
   View qv, kv, vv;
@@ -824,7 +824,8 @@ LayerForward layer_now(const Call& c, const Tensor& x, const Tensor& w1, const T
   }
   f.status = run_forward(c.p, c.z, c.scale, c.path, c.tiles, slices_of(f.qkv, c.z.Hq, c.z.D),
                          f.attn.data_ptr(), want_lse ? f.lse.data_ptr<float>() : nullptr, stream_of(x));
-  f.y = at::linear(f.attn, w2, opt(b2));
+  // not run: the layer goes through its modules then, and what an autograd node returns is dropped
+  f.y = f.status == B200NA_OK ? at::linear(f.attn, w2, opt(b2)) : at::empty_like(x);
   return f;
 }
 // Bias gradient: column sums of the output gradient.

@@ -404,3 +404,12 @@ def test_saved_tensor_hooks_that_return_other_strides(case):
         out = fn()
     for a, b in zip(torch.autograd.grad(out, wrt, d_out), want):
         assert torch.equal(a, b)
+
+
+def test_refused_calls_count_no_launches():
+    q = _off_16_bytes(torch.randn(1, 12, 12, 2, 64, device="cuda").bfloat16())
+    for leaf in (q, q.detach().requires_grad_()):
+        before = L.launches
+        with pytest.raises(L.NattenB200Error):   # refused by the native front, then by the Python one
+            nb.na2d(leaf, q, q, 3)
+        assert L.launches == before
