@@ -388,7 +388,8 @@ B200NA_API int b200na_na_backward_direct(
  *   - tiles of up to 128 tokens (kv_tile: exactly 128 with extra tokens).
  * With a 1-D window over the whole layout (no extra tokens) and with 1-D dilation above 2 the
  * probabilities and dS are held in two 16-bit parts instead of being rounded to the operand type, here
- * and in b200na_na_backward_direct.
+ * and in b200na_na_backward_direct; with contiguous operands, a NaN or an infinity then also stays with
+ * the rows that interact with it (elsewhere it spreads inside 128-token tiles).
  */
 B200NA_API int b200na_na_backward_view(
     const void* q, const void* k, const void* v, const void* o, const void* d_out, const float* lse,

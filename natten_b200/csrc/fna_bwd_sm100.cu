@@ -113,6 +113,7 @@ struct BwdTcParams {
   const float* lse;         // [B, *X, Hq]
   const float* delta;       // [B, *X, Hq]
   const float* norms;       // fp16 with kExact: see ds_exponent
+  unsigned* redo;           // kExact, may be null: set to 1 where a gradient is not finite
   void* out0;               // dQ (pass dQ) or dK (pass dKdV)
   void* out1;               // dV (pass dKdV)
   int* status;
@@ -751,6 +752,12 @@ fna_bwd_kernel(const __grid_constant__ CUtensorMap tm_r1, const __grid_constant_
         if (kCols == 32) ptx::tmem_ld32(src, reinterpret_cast<uint32_t(&)[32]>(orr));
         else ptx::tmem_ld16(src, reinterpret_cast<uint32_t(&)[16]>(orr));
         ptx::tmem_ld_wait();
+        if (kExact && p.redo && row_valid) {
+          float t = 0.f;
+#pragma unroll
+          for (int j = 0; j < kCols; ++j) t = fmaf(__uint_as_float(orr[j]) * mul, 0.f, t);
+          if (t != 0.f) *p.redo = 1;   // NaN
+        }
         if (row_valid) {
 #pragma unroll
           for (int v4 = 0; v4 < kCols / 8; ++v4) {
@@ -1447,9 +1454,14 @@ int backward_impl(const BwdCall& c, int ndim, const int* shape, const int* kerne
   FoldedPart parts[2] = {{0, 0, 0}, {0, 0, 0}};
   const int n_fold = c.views ? fna_fold_parts(ndim, base.X[0], base.dil[0], parts) : 0;
   bool delta_done = false;
-  static std::mutex norms_mu;
-  std::unique_lock<std::mutex> norms_lock;
-  float* norms = nullptr;
+  // A tensor-core product takes all 128 columns of a tile, with weights of zero where a pair does not
+  // interact, and 0 x NaN is NaN. Where the CUDA cores were exact about that they still are: a pass that
+  // writes a gradient that is not finite says so, and such rows are done again there.
+  const bool contiguous = q_ts == wq && k_ts == wkv && v_ts == wkv && dq_ts == wq && dk_ts == wkv && dv_ts == wkv;
+  const bool redo = exact && contiguous && (base.dil[0] > 2 || base.causal[0]);
+  static std::mutex scratch_mu;
+  std::unique_lock<std::mutex> scratch_lock;
+  CallScratch* scratch = nullptr;
   for (int part = 0; part < (n_fold ? n_fold : 1); ++part) {
     BwdTcParams view = base;
     FoldedAxis folded = {base.dil[0], parts[part].g0, parts[part].groups, base.X[0]};
@@ -1468,14 +1480,17 @@ int backward_impl(const BwdCall& c, int ndim, const int* shape, const int* kerne
     if ((rc = fna_make_tensor_map_direct(&mk, c.k, dtype, B, view.X, Hkv, D, tkv, view.dil, k_ts, sep, fold)) != B200NA_OK) return rc;
     if ((rc = fna_make_tensor_map_direct(&mv, c.v, dtype, B, view.X, Hkv, D, tkv, view.dil, v_ts, sep, fold)) != B200NA_OK) return rc;
     if (n_extra == 0) { mek = mk; mev = mv; }
+    if (!delta_done && (redo || (exact && dtype == B200NA_F16))) {
+      scratch_lock = std::unique_lock<std::mutex>(scratch_mu);
+      if ((rc = fna_call_scratch(&scratch, stream)) != B200NA_OK) return rc;
+      base.norms = view.norms = scratch->norms;
+      view.redo = redo ? &scratch->redo : nullptr;
+      base.redo = view.redo;
+    }
     if (!delta_done && exact && dtype == B200NA_F16) {
-      // norms of another call on this stream must not come between these launches
-      norms_lock = std::unique_lock<std::mutex>(norms_mu);
-      if ((rc = fna_call_norms(&norms, stream)) != B200NA_OK) return rc;
       const NormRows in[3] = {{c.d_out, tokens * B, Hq, wq, 0}, {c.v, tokens * B, Hkv, v_ts, 1},
                               {c.add_v, (int64_t)n_extra * B, Hkv, wkv, 1}};
-      if ((rc = launch_max_norms(in, n_extra > 0 ? 3 : 2, D, norms, stream)) != B200NA_OK) return rc;
-      base.norms = view.norms = norms;
+      if ((rc = launch_max_norms(in, n_extra > 0 ? 3 : 2, D, scratch->norms, stream)) != B200NA_OK) return rc;
     }
     if (!delta_done) {   // after every check of the first part
       if ((rc = launch_delta(c.o, c.d_out, c.delta, tokens * B * Hq, D, dtype, stream)) != B200NA_OK)
@@ -1518,6 +1533,11 @@ int backward_impl(const BwdCall& c, int ndim, const int* shape, const int* kerne
         return rc;
     }
   }
+  if (redo &&
+      (rc = simt_backward(c.q, c.k, c.v, c.o, c.d_out, c.lse, c.add_k, c.add_v, n_extra, c.dq, c.dk, c.dv,
+                          c.d_add_k, c.d_add_v, c.delta, ndim, shape, kernel, stride, dilation, causal, B,
+                          Hq, Hkv, D, dtype, scale, &scratch->redo, stream)) != B200NA_OK)
+    return rc;
   if (n_extra == 0) return B200NA_OK;
   // gradients of the extra tokens: rows = the extra tokens, columns = all queries of the batch
   // entry, flat
@@ -1525,6 +1545,7 @@ int backward_impl(const BwdCall& c, int ndim, const int* shape, const int* kerne
   p.ndim = 1;
   p.G = 1;
   p.dense_rows = 1;
+  p.redo = nullptr;   // every pair interacts
   p.r_rows = p.c_rows = kTile;
   p.row_extent = n_extra;
   for (int a = 0; a < B200NA_MAX_DIM; ++a) {

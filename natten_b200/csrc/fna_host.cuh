@@ -40,12 +40,18 @@ int fna_device_info(int* sms, int** status_ptr);
 // under stream capture gets a pair of its own from a pool of 3072 that is handed out in turn.
 int fna_work_counters(unsigned long long** pair, cudaStream_t stream);
 
-// Two zeroed-by-the-user floats of device memory for one call on `stream`, from slots of their own that are
-// handed out like the counter pairs.
-int fna_call_norms(float** norms, cudaStream_t stream);
+// Device memory that a call on `stream` hands from one of its launches to the next, from slots that are
+// handed out like the counter pairs; set to 0 on the stream. Another thread's call on the same stream must
+// not come between: the caller holds a lock from here to its last launch.
+struct CallScratch {
+  float norms[2];
+  unsigned redo;
+  unsigned unused;
+};
+int fna_call_scratch(CallScratch** scratch, cudaStream_t stream);
 
 // norms[slot] = the largest squared 2-norm of the rows of D fp16 elements (a multiple of 8, at most 128,
-// 16-byte aligned) of the inputs with that slot; both are set to 0 first. NaN where an input holds one.
+// 16-byte aligned) of the inputs with that slot, or what was there. NaN where an input holds one.
 struct NormRows {
   const void* rows;
   int64_t tokens;
@@ -59,5 +65,14 @@ int launch_max_norms(const NormRows* in, int n_inputs, int D, float* norms, cuda
 // 8, at most 128).
 int launch_delta(const void* o, const void* d_out, float* delta, int64_t rows, int D, int dtype,
                  cudaStream_t stream);
+
+// b200na_na_backward_simt; redo not null: dq, dk and dv are there already, and if *redo (device memory) is not
+// 0, the 32-row blocks of them that hold a NaN or an infinity are done again (16-bit types, D a multiple of 8).
+int simt_backward(
+    const void* q, const void* k, const void* v, const void* o, const void* d_out, const float* lse,
+    const void* add_k, const void* add_v, int n_extra, void* dq, void* dk, void* dv, void* d_add_k,
+    void* d_add_v, float* delta_scratch, int ndim, const int* shape, const int* kernel,
+    const int* stride, const int* dilation, const int* causal, int B, int Hq, int Hkv, int D,
+    int dtype, float scale, const unsigned* redo, cudaStream_t stream);
 
 }  // namespace b200na

@@ -69,8 +69,7 @@ __device__ int g_status_word;
 constexpr int kStreamSlots = 1024;
 constexpr int kCounterSlots = 4096;
 __device__ unsigned long long g_work_counters[kCounterSlots][2];
-// Two floats per slot for a call that hands a reduction from one launch to the next (fna_call_norms).
-__device__ float g_call_norms[kCounterSlots][2];
+__device__ CallScratch g_call_scratch[kCounterSlots];   // see fna_call_scratch
 
 struct FnaParams {
   int ndim;
@@ -1420,7 +1419,7 @@ struct DeviceState {
   int sms = 0;
   int* status_ptr = nullptr;
   unsigned long long* counters = nullptr;  // g_work_counters on this device
-  float* norms = nullptr;                  // g_call_norms
+  CallScratch* scratch = nullptr;          // g_call_scratch
   std::mutex slot_mu;
   std::unordered_map<cudaStream_t, int> stream_slot;   // counter pair of each stream seen so far
   unsigned next_graph_slot = 0;                        // captured launches take theirs in turn
@@ -1462,8 +1461,8 @@ int device_state(DeviceState** out) {
     B200NA_CUDA_TRY(cudaGetSymbolAddress(&sp, g_work_counters));
     st.counters = reinterpret_cast<unsigned long long*>(sp);
     B200NA_CUDA_TRY(cudaMemset(st.counters, 0, sizeof(unsigned long long) * kCounterSlots * 2));
-    B200NA_CUDA_TRY(cudaGetSymbolAddress(&sp, g_call_norms));
-    st.norms = reinterpret_cast<float*>(sp);
+    B200NA_CUDA_TRY(cudaGetSymbolAddress(&sp, g_call_scratch));
+    st.scratch = reinterpret_cast<CallScratch*>(sp);
     st.ready = true;
   }
   *out = &st;
@@ -1588,12 +1587,14 @@ int fna_work_counters(unsigned long long** pair, cudaStream_t stream) {
   if (rc == B200NA_OK) *pair = st->counters + 2 * slot;
   return rc;
 }
-int fna_call_norms(float** norms, cudaStream_t stream) {
+int fna_call_scratch(CallScratch** scratch, cudaStream_t stream) {
   DeviceState* st = nullptr;
   int slot = 0;
   const int rc = call_slot(&slot, &st, stream);
-  if (rc == B200NA_OK) *norms = st->norms + 2 * slot;
-  return rc;
+  if (rc != B200NA_OK) return rc;
+  *scratch = st->scratch + slot;
+  B200NA_CUDA_TRY(cudaMemsetAsync(*scratch, 0, sizeof(CallScratch), stream));
+  return B200NA_OK;
 }
 int fna_device_info(int* sms, int** status_ptr) {
   DeviceState* st = nullptr;

@@ -160,16 +160,40 @@ __device__ __noinline__ void gradients_again(BwdSmem<DM, kKeyRows>& sm, const Bw
   gradients<T, DM, kVec, kKeyRows, true>(sm, x, p);
 }
 
+// Whether a thread's share of the block's results, as another kernel left them, holds a NaN or an infinity
+// (16-bit types, D a multiple of 8, 16-byte aligned).
+template <class T, bool kKeyRows>
+__device__ __forceinline__ bool non_finite_results(const BwdTensors<T>& x, const Rows& s, int D) {
+  float t = 0.f;
+  if constexpr (sizeof(T) == 2) {
+    const int chunks = D / 8;
+    for (int i = threadIdx.x; i < kRows * chunks; i += kThreads) {
+      const int64_t row = s.row[i / chunks];
+      if (row < 0) continue;
+#pragma unroll
+      for (int o = 0; o < (kKeyRows ? 2 : 1); ++o) {
+        const uint4 v = *reinterpret_cast<const uint4*>((o ? x.out1 : x.out0) + row * D + i % chunks * 8);
+        const T* e = reinterpret_cast<const T*>(&v);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) t = fmaf(ldf(e + k), 0.f, t);
+      }
+    }
+  }
+  return t != 0.f;   // NaN
+}
+
 template <class T, int DM, bool kVec, bool kKeyRows>
 __global__ void __launch_bounds__(kThreads, bwd_blocks(DM)) na_bwd_kernel(
     const __grid_constant__ BwdTensors<T> x, const __grid_constant__ Params p) {
   extern __shared__ __align__(16) uint8_t smem_raw[];
   using SM = BwdSmem<DM, kKeyRows>;
   SM& sm = *reinterpret_cast<SM*>(smem_raw);
+  if (p.redo && *p.redo == 0) return;
   for (int64_t item = blockIdx.x; item < p.n_items; item += gridDim.x) {
     __syncthreads();                 // the previous item's readers are done
     if (threadIdx.x < kRows) decode_rows<kKeyRows>(p, item, sm.rows);
     __syncthreads();
+    if (p.redo && !__syncthreads_or(non_finite_results<T, kKeyRows>(x, sm.rows, p.D))) continue;
     if (!gradients<T, DM, kVec, kKeyRows, false>(sm, x, p)) gradients_again<T, DM, kVec, kKeyRows>(sm, x, p);
   }
 }
@@ -194,7 +218,8 @@ int launch_bwd_dm(BwdPointers& a, const Params& base, cudaStream_t stream) {
                          : (const void*)na_bwd_kernel<T, DM, false, false>;
   const void* fn_k = vec ? (const void*)na_bwd_kernel<T, DM, true, true>
                          : (const void*)na_bwd_kernel<T, DM, false, true>;
-  for (int pass = 0; pass < (base.n_extra > 0 ? 3 : 2); ++pass) {
+  // every query interacts with every extra token: nothing reaches their sums that does not belong there
+  for (int pass = 0; pass < (base.n_extra > 0 && !base.redo ? 3 : 2); ++pass) {
     Params p = base;
     p.row_heads = pass == 0 ? p.Hq : p.Hkv;
     if (pass == 2) {   // extra tokens: every query is a column, dilation groups do not matter
@@ -208,7 +233,9 @@ int launch_bwd_dm(BwdPointers& a, const Params& base, cudaStream_t stream) {
                        (T*)(pass == 0 ? a.dq : (pass == 1 ? a.dk : a.d_add_k)),
                        (T*)(pass == 0 ? nullptr : (pass == 1 ? a.dv : a.d_add_v))};
     void* args[] = {(void*)&x, (void*)&p};
-    const int rc = simt::launch(pass == 0 ? fn_q : fn_k, p.n_items,
+    // a look at *redo is all there is to do nearly always: as many blocks as are resident at once
+    const int64_t blocks = p.redo ? min(p.n_items, (int64_t)148 * bwd_blocks(DM)) : p.n_items;
+    const int rc = simt::launch(pass == 0 ? fn_q : fn_k, blocks,
                                 (int)(pass == 0 ? sizeof(BwdSmem<DM, false>)
                                                 : sizeof(BwdSmem<DM, true>)), args, stream);
     if (rc != B200NA_OK) return rc;
@@ -316,7 +343,6 @@ __global__ void __launch_bounds__(kDeltaThreads) max_norms_kernel(NormRows a, No
 
 int launch_max_norms(const NormRows* in, int n_inputs, int D, float* norms, cudaStream_t stream) {
   if (n_inputs < 2 || n_inputs > 3 || D % 8 != 0 || D < 8 || D > 128) return B200NA_ERR_INVALID_ARGUMENT;
-  B200NA_CUDA_TRY(cudaMemsetAsync(norms, 0, 2 * sizeof(float), stream));
   const dim3 grid(148, n_inputs);
   const NormRows& last = in[n_inputs - 1];
   unsigned* out = reinterpret_cast<unsigned*>(norms);
@@ -333,15 +359,13 @@ int launch_delta(const void* o, const void* d_out, float* delta, int64_t rows, i
   if (dtype == B200NA_BF16) return launch_delta_typed<__nv_bfloat16>(o, d_out, delta, rows, D, stream);
   return B200NA_ERR_INVALID_ARGUMENT;
 }
-}  // namespace b200na
 
-extern "C" B200NA_API int b200na_na_backward_simt(
+int simt_backward(
     const void* q, const void* k, const void* v, const void* o, const void* d_out, const float* lse,
     const void* add_k, const void* add_v, int n_extra, void* dq, void* dk, void* dv, void* d_add_k,
     void* d_add_v, float* delta_scratch, int ndim, const int* shape, const int* kernel,
     const int* stride, const int* dilation, const int* causal, int B, int Hq, int Hkv, int D,
-    int dtype, float scale, b200na_stream_t stream) {
-  using namespace b200na;
+    int dtype, float scale, const unsigned* redo, cudaStream_t stream) {
   if (!q || !k || !v || !o || !d_out || !lse || !dq || !dk || !dv || !delta_scratch)
     return B200NA_ERR_INVALID_ARGUMENT;
   if (n_extra < 0 || (n_extra > 0 && (!add_k || !add_v || !d_add_k || !d_add_v)))
@@ -365,12 +389,24 @@ extern "C" B200NA_API int b200na_na_backward_simt(
   p.B = B; p.Hq = Hq; p.Hkv = Hkv; p.D = D;
   p.n_extra = n_extra;
   p.scale = scale;
+  p.redo = redo;
   BwdPointers a = {q, k, v, o, d_out, lse, add_k, add_v, dq, dk, dv, d_add_k, d_add_v, delta_scratch};
-  cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   switch (dtype) {
-    case B200NA_F32: return launch_bwd<float>(a, p, s);
-    case B200NA_F16: return launch_bwd<__half>(a, p, s);
-    case B200NA_BF16: return launch_bwd<__nv_bfloat16>(a, p, s);
+    case B200NA_F32: return launch_bwd<float>(a, p, stream);
+    case B200NA_F16: return launch_bwd<__half>(a, p, stream);
+    case B200NA_BF16: return launch_bwd<__nv_bfloat16>(a, p, stream);
     default: return B200NA_ERR_INVALID_ARGUMENT;
   }
+}
+}  // namespace b200na
+
+extern "C" B200NA_API int b200na_na_backward_simt(
+    const void* q, const void* k, const void* v, const void* o, const void* d_out, const float* lse,
+    const void* add_k, const void* add_v, int n_extra, void* dq, void* dk, void* dv, void* d_add_k,
+    void* d_add_v, float* delta_scratch, int ndim, const int* shape, const int* kernel,
+    const int* stride, const int* dilation, const int* causal, int B, int Hq, int Hkv, int D,
+    int dtype, float scale, b200na_stream_t stream) {
+  return b200na::simt_backward(q, k, v, o, d_out, lse, add_k, add_v, n_extra, dq, dk, dv, d_add_k, d_add_v,
+                               delta_scratch, ndim, shape, kernel, stride, dilation, causal, B, Hq, Hkv, D,
+                               dtype, scale, nullptr, reinterpret_cast<cudaStream_t>(stream));
 }

@@ -67,6 +67,8 @@ struct Params {
   int64_t Nq;         // query tokens per batch entry (== N except for dense cross attention)
   int dense;          // dense attention: every query sees keys [0, N) (causal: [0, i + 1))
   int extra_rows;     // backward: the rows are the n_extra tokens, the columns all queries
+  const unsigned* redo;   // backward, not null: the results are there; if *redo is not 0, items with a
+                          // result that is not finite are done again
   int G;              // dilation groups
   int T[B200NA_MAX_DIM];   // row tile shape, product kRows
   int R[B200NA_MAX_DIM];   // row tiles per axis of the largest dilation group

@@ -622,8 +622,9 @@ void run_backward(const Problem& p, const Sizes& z, float scale, bool tensor_cor
                                t.kv.data(), z.B, z.Hq, z.Hkv, z.D, z.dt, scale, a.q_ts, a.k_ts, a.v_ts,
                                g.dq_ts, g.dk_ts, g.dv_ts, stream),
           "b200na_na_backward_view");
-    launches += 1 + 2 * parts_of(p) + (a.n_extra ? 1 : 0) +
-                (exact_gradients(p, a.n_extra) && z.dt == B200NA_F16 ? 1 : 0);
+    launches += 1 + 2 * parts_of(p) + (a.n_extra ? 1 : 0);
+    if (exact_gradients(p, a.n_extra))   // row norms; a look for non-finite rows where there are masks
+      launches += (z.dt == B200NA_F16 ? 1 : 0) + (p.dilation[0] > 2 || p.causal[0] ? 2 : 0);
   } else {
     check(lib.na_backward_simt(a.q, a.k, a.v, out, d_out, lse, a.ak, a.av, a.n_extra, g.dq, g.dk, g.dv,
                                g.dak, g.dav, delta, p.nd, p.shape.data(), p.kernel.data(),
@@ -770,9 +771,9 @@ struct NaFunction : torch::autograd::Function<NaFunction> {
     Tiles t;
     const bool tc = backward_on_tensor_cores(p, c.z, extra, &t) && p.kernel[0] >= 2;
     View qv, kv, vv;
-    if (tc) {
+    if (tc && !exact_gradients(p, extra)) {
       qv = as_view(q); kv = as_view(k); vv = as_view(v);
-    } else {
+    } else {   // also exact ones: rows may be done again on the CUDA cores, which read no views
       qv = {q.contiguous(), 0}; kv = {k.contiguous(), 0}; vv = {v.contiguous(), 0};
     }
     const Tensor d_out = tc ? aligned(d_out_) : d_out_.contiguous();
@@ -1152,7 +1153,8 @@ PyObject* py_layer(PyObject*, PyObject* const* a, Py_ssize_t n) {
   Tensor y;
   if (any_requires_grad({&x, &w1, &b1, &w2, &b2})) {
     Tiles t;
-    if (!backward_on_tensor_cores(c.p, c.z, false, &t)) Py_RETURN_NONE;
+    // exact gradients need contiguous operands: the layer in parts copies them
+    if (!backward_on_tensor_cores(c.p, c.z, false, &t) || exact_gradients(c.p, false)) Py_RETURN_NONE;
     auto call = c10::make_intrusive<SharedCall>();
     call->c = c;
     {

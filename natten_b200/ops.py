@@ -333,6 +333,9 @@ def na_backward_direct(query: Tensor, key: Tensor, value: Tensor, out: Tensor, d
     na_dim = query.dim() - 3
     n_extra = additional_keys.shape[1] if additional_keys is not None else 0
     delta = torch.empty(query.shape[:-1], dtype=torch.float32, device=query.device)
+    launches = 4 if n_extra else 3
+    if na_dim == 1 and not n_extra and kernel_size[0] == query.shape[1]:    # exact gradients
+        launches += (query.dtype == torch.float16) + 2 * bool(is_causal[0])
     with torch.cuda.device(query.device):
         full = full_tiles(q_tile_shape, kv_tile_shape)
         entry = _lib.lib.b200na_na_backward_direct if full else _lib.lib.b200na_na_backward_view
@@ -344,7 +347,7 @@ def na_backward_direct(query: Tensor, key: Tensor, value: Tensor, out: Tensor, d
             _lib.ints(dilation), _lib.ints(_flags(is_causal)), _lib.ints(q_tile_shape),
             _lib.ints(kv_tile_shape), query.shape[0], query.shape[-2], key.shape[-2],
             query.shape[-1], DTYPE_CODE[query.dtype], float(scale), *(() if full else (0,) * 6),
-            _stream(query)), "b200na_na_backward_direct", kernel_launches=4 if n_extra else 3)
+            _stream(query)), "b200na_na_backward_direct", kernel_launches=launches)
     return dq, dk, dv, dak, dav
 
 

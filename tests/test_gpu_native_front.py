@@ -413,3 +413,34 @@ def test_refused_calls_count_no_launches():
         with pytest.raises(L.NattenB200Error):   # refused by the native front, then by the Python one
             nb.na2d(leaf, q, q, 3)
         assert L.launches == before
+
+
+@pytest.mark.parametrize("n,win,dil,causal,hq,hkv,D,n_extra", [
+    (300, 0, 1, True, 2, 1, 64, 0), (260, 0, 1, True, 2, 2, 40, 0), (700, 33, 3, True, 2, 2, 128, 20),
+    (701, 40, 5, False, 4, 2, 64, 0)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_16bit_non_finite_tokens_stay_with_the_rows_that_interact(n, win, dil, causal, hq, hkv, D, n_extra, dtype):
+    """Gradients that the CUDA cores computed first: a NaN or an infinity in a key or an output gradient
+    reaches the rows that it reached there, and no others."""
+    torch.manual_seed(97)
+    ops = [torch.randn(2, n, h, D, device="cuda").to(dtype) for h in (hq, hkv, hkv, hq)]
+    extras = [torch.randn(2, n_extra, hkv, D, device="cuda").to(dtype) for _ in range(2)] if n_extra else []
+    add = dict(zip(("additional_keys", "additional_values"), extras))
+    for which, value, token in ((1, float("nan"), 131), (1, float("inf"), 40), (3, float("nan"), 200),
+                                (3, float("-inf"), 5), (0, float("nan"), 129)):
+        poisoned = [t.clone() for t in ops]
+        poisoned[which][1, token, -1, 3] = value
+        leaves = [t.requires_grad_() for t in poisoned[:3]]
+        if win:
+            out, lse = nb.na1d(*leaves, win, 1, dil, causal, return_lse=True, **add)
+        else:
+            out, lse = nb.attention(*leaves, is_causal=causal, return_lse=True)
+        got = torch.autograd.grad(out, leaves, poisoned[3])
+        assert L.device_status() == 0
+        with torch.no_grad():
+            want = nb.ops.na_backward_simt(*poisoned[:3], out, poisoned[3], lse, *(extras or (None, None)),
+                                           [win or n], [1], [dil], [causal], D ** -0.5)[:3]
+        for a, b in zip(got, want):
+            on = b.isfinite()
+            assert not on.all() and torch.equal(a.isfinite(), on)
+            assert (a[on].float() - b[on].float()).norm() <= 2.0 ** -11.5 * b[on].float().norm()
