@@ -18,7 +18,7 @@
 //     No atomics, no partial sums in memory: every gradient row is owned by exactly one CTA.
 //   * The columns a row tile needs form a box of tiles in both passes: a query's keys are its
 //     window, and a key's queries are the inverse window - an interval per axis, because window
-//     start and end never decrease with the query coordinate (found by bisection).
+//     start and end never decrease with the query coordinate (a closed form at unit stride, else bisection).
 //   * TMEM: S [0,128) dP [128,256) acc0 [256,256+D) acc1 [384,384+D). Pass dKdV: P and dS (16-bit)
 //     overwrite S and dP in place, privately per thread, and feed the second MMAs from TMEM; the
 //     four regions fill TMEM, so a column tile's products and its P / dS arithmetic alternate.

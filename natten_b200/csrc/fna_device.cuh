@@ -39,10 +39,6 @@ __device__ __forceinline__ bool wait_bar(uint64_t* bar, uint32_t parity, volatil
   return true;
 }
 
-__device__ __forceinline__ void named_bar_sync(int id, int threads) {
-  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
-}
-
 // Two fp32 values -> two 16-bit floats in one word, `lo` in the low half.
 template <int kType>
 __device__ __forceinline__ uint32_t pack2(float lo, float hi) {

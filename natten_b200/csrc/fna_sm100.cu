@@ -662,12 +662,12 @@ fna_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         // stored after that is known: the logits it overwrites are still there to start again).
         // A row without keys so far (its window starts in a later tile) has no maximum yet. The
         // one-half shape, chosen for small windows, meets boundary tiles nearly always; masks and
-        // packed P together spill there: 128 x 128, 13 x 13 windows, dilation 2 took 1052 us in one
-        // pass everywhere, 983 us with one pass for the other tiles, 935 us in two passes. The windows
-        // of 3-D layouts do hold whole tiles: 15 x 30 x 52, 7 x 15 x 15, forward 682 us in two
-        // passes, 655 us this way.
-        // 15 x 44 x 80 video in 8 bits: 2051 -> 1859 us; long causal sequences: the same time (the
-        // softmax gets 5 % shorter, the wait for the next logits longer).
+        // packed P together spill there: 8 x 16 heads of 128, 128 x 128 maps, 13 x 13 windows, dilation 2
+        // take 1060 us in one pass everywhere, 1009 us with one pass for interior tiles, 964 us in two
+        // passes (7 x 7 undilated 688, 638, 616). The windows of 3-D layouts do hold whole tiles, which
+        // take one pass: 15 x 30 x 52, 7 x 15 x 15, forward 682 us in two passes, 655 us this way. 15 x 44 x
+        // 80 video in 8 bits: 2097 -> 1859 us; long causal sequences: the same time (the softmax gets
+        // 5 % shorter, the wait for the next logits longer).
         bool again = iter == 0 || (kH == 1 && (NDIM != 3 || !interior)) ||
                      __any_sync(0xffffffffu, m == -INFINITY);
         if (!again) {
